@@ -157,7 +157,7 @@ __device__ __forceinline__ void bb_rx_partials_dense(const BBData &D, const T *R
 
 // Low-rank part, step 1: partials of R v.  Block b owns the b-th chunk of
 // every row of R; warp w of the block folds rows w, w + WARPS, ...
-__device__ void bb_rx_partials(const BBData &D, const double *v)
+static __device__ void bb_rx_partials(const BBData &D, const double *v)
 {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nb = gridDim.x;
     if (D.r_width) {
@@ -185,7 +185,7 @@ __device__ void bb_rx_partials(const BBData &D, const double *v)
 }
 
 // step 2: block r folds row r's partials in block order
-__device__ void bb_rx_fold(const BBData &D)
+static __device__ void bb_rx_fold(const BBData &D)
 {
     const int nb = gridDim.x;
     for (int r = blockIdx.x; r < D.k; r += nb) {
@@ -209,7 +209,7 @@ __device__ void bb_rx_fold(const BBData &D)
 // step 3: D (R v) into shared memory (every block, k <= BB_MAX_RANK)
 constexpr int BB_MAX_RANK = 512;
 
-__device__ void bb_drx_smem(const BBData &D, double *drx)
+static __device__ void bb_drx_smem(const BBData &D, double *drx)
 {
     for (int r = threadIdx.x; r < D.k; r += TPB) {
         double v;
@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(TPB) bb_kernel(BBData D, BBParams P)
 // refresh_inner_precond_kernel, src/kernels/pdhcg_kernels.cu:482-495, and
 // the tol_scale of src/pdhg_core_op.cu:511-523): m = diag_h + 1/tau (1 when
 // <= 0), partials of sum |m|.
-__global__ void __launch_bounds__(TPB) bb_precond_kernel(int n, const double *diag_h, double inv_tau, double *m_diag,
+static __global__ void __launch_bounds__(TPB) bb_precond_kernel(int n, const double *diag_h, double inv_tau, double *m_diag,
                                                          double *m_inv, double *partials)
 {
     const int ops[1] = {RSUM};
@@ -608,14 +608,14 @@ __global__ void __launch_bounds__(TPB) bb_precond_kernel(int n, const double *di
     block_reduce_store<1>(acc, ops, partials);
 }
 
-__global__ void bb_tol_scale_kernel(const double *sum, int n, double *tol_scale)
+static __global__ void bb_tol_scale_kernel(const double *sum, int n, double *tol_scale)
 {
     *tol_scale = n > 0 ? sqrt(*sum / (double)n) : 1.0;
 }
 
 // inner tolerance schedule after a fixed-point error (reference
 // compute_fixed_point_error, src/pdhg_core_op.cu:1029-1034)
-__global__ void bb_tol_update_kernel(const double *fpe_sums, double step, double omega, double min_tol, double *tol)
+static __global__ void bb_tol_update_kernel(const double *fpe_sums, double step, double omega, double min_tol, double *tol)
 {
     double pn = sqrt(fpe_sums[0]);
     *tol = fmin(*tol, fmax(0.0005 * pn / step * omega, min_tol));
@@ -624,7 +624,7 @@ __global__ void bb_tol_update_kernel(const double *fpe_sums, double step, double
 // diag(Q) + diag(R^T D R) for the preconditioner (reference
 // initialize_inner_solver, src/solver_state.cu:321-367)
 // R_dense: R row-major k x width over columns 0..width-1 (then R^T is not used)
-__global__ void bb_diag_h_kernel(int n, int sparse, const int *Q_rp, const int *Q_ci, const double *Q_v, int k,
+static __global__ void bb_diag_h_kernel(int n, int sparse, const int *Q_rp, const int *Q_ci, const double *Q_v, int k,
                                  const int *Rt_rp, const int *Rt_ci, const double *Rt_v, const double *R_dense,
                                  int width, int dkind, const double *Ddiag, const double *Ddense, double *diag_h)
 {
@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(TPB) q_apply_kernel(BBData D, const double *v,
 // its smallest (reference estimate_maximum_eigenvalue /
 // estimate_minimum_eigenvalue, src/pdhg_core_op.cu:1498-1671), one
 // cooperative launch each.  out = {lambda, iterations}.
-__global__ void __launch_bounds__(TPB) power_eig_kernel(int n, const int *Q_rp, const int *Q_ci, const double *Q_v,
+static __global__ void __launch_bounds__(TPB) power_eig_kernel(int n, const int *Q_rp, const int *Q_ci, const double *Q_v,
                                                         double *v, double *av, double *part, int max_iter,
                                                         double tol, int shifted, double lmax, double *out)
 {

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(256) long_partials_kernel(LongRows L, const in
 }
 
 // number of rows longer than LONG_ROW entries
-__global__ void long_count_kernel(int rows, const int *rp, int *count)
+static __global__ void long_count_kernel(int rows, const int *rp, int *count)
 {
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x)
         if (rp[r + 1] - rp[r] > LONG_ROW)
@@ -1090,7 +1090,7 @@ __host__ __device__ inline long long psd_scratch_doubles(int order, bool is_long
     return 2LL * order * order + (is_long ? 3 * L : 0);
 }
 
-__device__ void warp_project_psd_mem(const double *in, double *out, int L, int lane, double *work)
+static __device__ void warp_project_psd_mem(const double *in, double *out, int L, int lane, double *work)
 {
     const int n = psd_order(L);
     if (n == 1) {

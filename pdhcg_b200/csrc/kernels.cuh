@@ -461,7 +461,7 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[NS], const int (&
 }
 
 // out[s] = fold over blocks of partials[b*NS+s]; one block of TPB threads.
-__global__ void fold_partials_kernel(const double *partials, int nblocks, int ns, const int *ops, double *out)
+static __global__ void fold_partials_kernel(const double *partials, int nblocks, int ns, const int *ops, double *out)
 {
     __shared__ double sh[TPB];
     for (int s = 0; s < ns; ++s) {
@@ -487,7 +487,7 @@ __global__ void fold_partials_kernel(const double *partials, int nblocks, int ns
 
 // y = M x, one warp per tile of 32 rows (stream-mode products); lr: M's
 // long rows with the segment pass over this x done (or none)
-__global__ void __launch_bounds__(TPB) spmv_kernel(int rows, const int *rp, const int *ci, const double *v,
+static __global__ void __launch_bounds__(TPB) spmv_kernel(int rows, const int *rp, const int *ci, const double *v,
                                                    const double *x, double *y, LongRows lr)
 {
     __shared__ double stage_all[WARPS][STREAM_CHUNK];
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(TPB) spmv_kernel(int rows, const int *rp, cons
     }
 }
 
-__global__ void cone_len_kernel(int nc, const int *vdim, const int *type, int *len)
+static __global__ void cone_len_kernel(int nc, const int *vdim, const int *type, int *len)
 {
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nc; b += gridDim.x * blockDim.x) {
         int t = type[b], v = vdim[b];

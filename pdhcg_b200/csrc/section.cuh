@@ -514,7 +514,7 @@ __device__ __forceinline__ double sec_exp_obj(int kind, double y, double p0, dou
 
 // golden-section minimum over y in [lo, hi] after doubling hi while the
 // objective falls (reference src/kernels/pdhcg_exp_cone_kernels.cu:422-456)
-__device__ double sec_exp_golden(int kind, double lo, double hi, double p0, double ia, double ib, double wa, double wb)
+static __device__ double sec_exp_golden(int kind, double lo, double hi, double p0, double ia, double ib, double wa, double wb)
 {
     double prev = sec_exp_obj(kind, 0.5 * hi, p0, ia, ib, wa, wb);
     double cur = sec_exp_obj(kind, hi, p0, ia, ib, wa, wb);
@@ -546,7 +546,7 @@ __device__ double sec_exp_golden(int kind, double lo, double hi, double p0, doub
 
 // (x, z) with y > 0 fixed: safeguarded Newton in u (reference
 // project_2d_exp_persp, src/kernels/pdhcg_exp_cone_kernels.cu:134-231)
-__device__ void sec_exp_fixed_y(double rz0, double ry, double rt0, double d_r, double d_y, double d_t, double *warm,
+static __device__ void sec_exp_fixed_y(double rz0, double ry, double rt0, double d_r, double d_y, double d_t, double *warm,
                                 double &rzo, double &rto)
 {
     rzo = rz0;
@@ -614,7 +614,7 @@ __device__ void sec_exp_fixed_y(double rz0, double ry, double rt0, double d_r, d
 // exponential section in actual coordinates i (weights w); fixed slots keep
 // their inputs (reference project_exp_cone_section,
 // src/kernels/pdhcg_exp_cone_kernels.cu:285-524)
-__device__ __noinline__ void sec_exp_point(const double *i3, const double *w3, const bool *f3, double *warm,
+static __device__ __noinline__ void sec_exp_point(const double *i3, const double *w3, const bool *f3, double *warm,
                                            double *o3)
 {
     const double ix = i3[0], iy = i3[1], iz = i3[2];
@@ -734,7 +734,7 @@ __device__ __forceinline__ double sec_pow_xy_log_boundary(double lam, double rx,
 
 // (x, y) with z fixed (reference project_power_xy_fixed_z[_normalized],
 // src/kernels/pdhcg_power_cone_kernels.cu:146-234)
-__device__ void sec_pow_xy_fixed_z(double rx, double ry, double fz, double wx, double wy, double a, double &xo,
+static __device__ void sec_pow_xy_fixed_z(double rx, double ry, double fz, double wx, double wy, double a, double &xo,
                                    double &yo)
 {
     double scale = fmax(fabs(rx), fmax(fabs(ry), fabs(fz)));
@@ -823,7 +823,7 @@ __device__ __forceinline__ double sec_pow_derivative(double o, double ro, double
 // one axis fixed at f: (other, z) onto |z| <= f^fexp other^oexp
 // (reference project_power_section_fixed_axis[_normalized],
 // src/kernels/pdhcg_power_cone_kernels.cu:263-365)
-__device__ void sec_pow_fixed_axis(double f, double ro, double rz, double wo, double wz, double fexp, double oexp,
+static __device__ void sec_pow_fixed_axis(double f, double ro, double rz, double wo, double wz, double fexp, double oexp,
                                    double &oo, double &zo)
 {
     double scale = fmax(f, fmax(fabs(ro), fabs(rz)));
@@ -883,7 +883,7 @@ __device__ void sec_pow_fixed_axis(double f, double ro, double rz, double wo, do
 // power section in actual coordinates (reference
 // project_power_cone_point_with_fixed, src/kernels/pdhcg_power_cone_kernels.cu:367-433;
 // at least one slot is fixed here)
-__device__ __noinline__ void sec_pow_point(const double *i3, const double *w3, const bool *f3, double a, double *o3)
+static __device__ __noinline__ void sec_pow_point(const double *i3, const double *w3, const bool *f3, double a, double *o3)
 {
     const double rx = i3[0], ry = i3[1], rz = i3[2], om = 1.0 - a;
     double xo = rx, yo = ry, zo = rz;

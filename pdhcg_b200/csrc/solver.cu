@@ -28,25 +28,12 @@
 #include <vector>
 
 #include "internal.h"
-#include "bb.cuh"
-#include "residual.cuh"
+#include "launch.cuh"
 #include "setup.cuh"
 
 using namespace pdhcg;
 
 namespace {
-
-struct CudaError : std::runtime_error {
-    using std::runtime_error::runtime_error;
-};
-
-#define CK(call)                                                                                                       \
-    do {                                                                                                               \
-        cudaError_t e_ = (call);                                                                                       \
-        if (e_ != cudaSuccess)                                                                                         \
-            throw CudaError(std::string(#call) + ": " + cudaGetErrorString(e_) + " at " + __FILE__ + ":" +            \
-                            std::to_string(__LINE__));                                                                 \
-    } while (0)
 
 thread_local pdhcg_b200_stats_t g_last_stats;
 
@@ -223,37 +210,6 @@ struct Arena {
     }
 };
 
-int grid_for(long long work, int per_block, int cap = 148 * 16)
-{
-    long long g = (work + per_block - 1) / per_block;
-    if (g < 1)
-        g = 1;
-    if (g > cap)
-        g = cap;
-    return (int)g;
-}
-
-// Blocks of `kernel` (TPB threads, static shared memory) resident at once
-// on the current device; cached per kernel and device.
-int resident_blocks(const void *kernel)
-{
-    static std::mutex mu;
-    static std::unordered_map<const void *, int> cache[64];
-    int dev = 0;
-    CK(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lock(mu);
-    auto &c = cache[dev & 63];
-    auto it = c.find(kernel);
-    if (it != c.end())
-        return it->second;
-    int nsm = 0, per_sm = 0;
-    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, TPB, 0));
-    const int r = std::max(1, nsm * std::max(per_sm, 1));
-    c.emplace(kernel, r);
-    return r;
-}
-
 int print_frequency(int iter)
 {
     int step = 10;
@@ -279,58 +235,6 @@ std::vector<int2> row_tiles(const std::vector<int> &rows)
     }
     return t;
 }
-
-// The primal step launches the SOC / RSOC blocks and the 3-slot blocks
-// (exponential, power) separately: the 3-slot projections would otherwise
-// sit in the wide kernels' register allocation.  A list pointer stays null
-// when its launch covers every block (all of one kind).
-struct ConeSplit {
-    std::vector<int> wide, three, psd, sect;
-    int *wide_d = nullptr, *three_d = nullptr, *psd_d = nullptr, *sect_d = nullptr;
-    int n_wide = 0, n_three = 0, n_psd = 0, n_sect = 0;
-
-    // fixed (may be empty): per block, does it hold slots fixed by
-    // set_cone_fixed?  Those blocks take the section projectors.
-    void build(const std::vector<int> &types, const std::vector<char> &fixed = {})
-    {
-        wide.clear();
-        three.clear();
-        psd.clear();
-        sect.clear();
-        for (int b = 0; b < (int)types.size(); ++b) {
-            if (!fixed.empty() && fixed[b])
-                sect.push_back(b);
-            else if (types[b] == CONE_EXPONENTIAL || types[b] == CONE_POWER)
-                three.push_back(b);
-            else if (types[b] == CONE_PSD)
-                psd.push_back(b);
-            else
-                wide.push_back(b);
-        }
-        n_wide = (int)wide.size();
-        n_three = (int)three.size();
-        n_psd = (int)psd.size();
-        n_sect = (int)sect.size();
-    }
-    // more than one launch: every launch takes its index list
-    bool mixed() const { return (n_wide > 0) + (n_three > 0) + (n_psd > 0) + (n_sect > 0) > 1; }
-    // the lists back to back in one device array of n_wide + n_three + n_psd + n_sect ints
-    void place(int *ids)
-    {
-        wide_d = ids;
-        three_d = ids + n_wide;
-        psd_d = ids + n_wide + n_three;
-        sect_d = ids + n_wide + n_three + n_psd;
-    }
-    std::vector<int> joined() const
-    {
-        std::vector<int> all(wide);
-        all.insert(all.end(), three.begin(), three.end());
-        all.insert(all.end(), psd.begin(), psd.end());
-        all.insert(all.end(), sect.begin(), sect.end());
-        return all;
-    }
-};
 
 // lanes per row from the mean row length
 int pick_group(long long nnz, int rows)
@@ -949,82 +853,6 @@ private:
 };
 
 
-template <typename F>
-void dispatch_s(int S, F &&f)
-{
-    switch (S) {
-    case 1: f(std::integral_constant<int, 1>{}); break;
-    case 2: f(std::integral_constant<int, 2>{}); break;
-    case 4: f(std::integral_constant<int, 4>{}); break;
-    default: f(std::integral_constant<int, 8>{}); break;
-    }
-}
-
-// Primal step over the cone blocks: the SOC / RSOC blocks with S slots per
-// lane, the 3-slot blocks with one; returns the number of launches.
-template <typename T>
-int launch_primal_cones(const StepData<T> &D, const StepParams &P, const ConeSplit &sp, int S, bool hasq,
-                        cudaStream_t s)
-{
-    int launches = 0;
-    if (sp.n_wide > 0) {
-        // no more blocks than are resident at once: each warp then walks
-        // several cone blocks and the warps drift apart, so one warp's
-        // projection arithmetic overlaps other warps' loads (a full grid
-        // starts every resident warp on its loads together); ~4 % of the
-        // step on 20000 SOC blocks of 50
-        dispatch_s(S, [&](auto SC) {
-            if (hasq) {
-                auto k = primal_cone_kernel<SC.value, T, true, CONES_WIDE>;
-                int grid = std::min(grid_for(sp.n_wide, WARPS), resident_blocks((const void *)k));
-                k<<<grid, TPB, 0, s>>>(D, P, sp.wide_d, sp.n_wide);
-            } else {
-                auto k = primal_cone_kernel<SC.value, T, false, CONES_WIDE>;
-                int grid = std::min(grid_for(sp.n_wide, WARPS), resident_blocks((const void *)k));
-                k<<<grid, TPB, 0, s>>>(D, P, sp.wide_d, sp.n_wide);
-            }
-        });
-        ++launches;
-    }
-    if (sp.n_three > 0) {
-        int grid = grid_for(sp.n_three, WARPS);
-        if (hasq)
-            primal_cone_kernel<1, T, true, CONES_THREE><<<grid, TPB, 0, s>>>(D, P, sp.three_d, sp.n_three);
-        else
-            primal_cone_kernel<1, T, false, CONES_THREE><<<grid, TPB, 0, s>>>(D, P, sp.three_d, sp.n_three);
-        ++launches;
-    }
-    if (sp.n_psd > 0) { // LP path only: diagonal Q with PSD blocks takes the inner BB solve
-        dispatch_s(S, [&](auto SC) {
-            int grid = grid_for(sp.n_psd, WARPS);
-            if (hasq)
-                primal_cone_kernel<SC.value, T, true, CONES_PSD><<<grid, TPB, 0, s>>>(D, P, sp.psd_d, sp.n_psd);
-            else
-                primal_cone_kernel<SC.value, T, false, CONES_PSD><<<grid, TPB, 0, s>>>(D, P, sp.psd_d, sp.n_psd);
-        });
-        ++launches;
-    }
-    if (sp.n_sect > 0) { // blocks with fixed slots: section projectors, one slot class (any block length)
-        int grid = grid_for(sp.n_sect, WARPS);
-        if (hasq)
-            primal_cone_kernel<8, T, true, CONES_SECTION><<<grid, TPB, 0, s>>>(D, P, sp.sect_d, sp.n_sect);
-        else
-            primal_cone_kernel<8, T, false, CONES_SECTION><<<grid, TPB, 0, s>>>(D, P, sp.sect_d, sp.n_sect);
-        ++launches;
-    }
-    return launches;
-}
-
-template <typename F>
-void dispatch_rg(int G, F &&f)
-{
-    switch (G) {
-    case 1: f(std::integral_constant<int, 1>{}); break;
-    case 4: f(std::integral_constant<int, 4>{}); break;
-    default: f(std::integral_constant<int, 32>{}); break;
-    }
-}
-
 // ---- working copy on the device --------------------------------------------
 void Solve::build_host()
 {
@@ -1258,11 +1086,8 @@ void Solve::init_state()
         CK(cudaMemsetAsync(cone_warm_, 0, 3 * (size_t)nc * sizeof(double), s)); // 0 = no warm start
         cone_aux_init_kernel<<<grid_for(nc, TPB), TPB, 0, s>>>(nc, cst_d_, cvdim_d_, ctype_d_, vr_d_, sb_, x0_,
                                                                dp_.fixed_d);
-        dispatch_s(S_, [&](auto SC) {
-            project_cones_kernel<SC.value><<<grid_for(nc, WARPS), TPB, 0, s>>>(
-                nc, cst_d_, clen_d_, ctype_d_, dp_.calpha, x0_, vr_d_, nullptr, 0.0, psd_work_, dp_.psd_off_d,
-                dp_.fixed_d, dp_.cfix_d, cone_warm_);
-        });
+        launch_project_cones(S_, {nc, cst_d_, clen_d_, ctype_d_, dp_.calpha, x0_, vr_d_, nullptr, 0.0, psd_work_,
+                                  dp_.psd_off_d, dp_.fixed_d, dp_.cfix_d, cone_warm_}, s);
     }
     box_clamp_copy_kernel<<<grid_for(n, TPB), TPB, 0, s>>>(n, l_d_, u_d_, x0_, x_, xp_, xr_);
     if (qtype_ == PDHCG_DIAG_Q) {
@@ -1352,22 +1177,7 @@ void Solve::setup_bb()
     int dev = 0, nsm = 0, per_sm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    // problems with fixed cone slots take the widest slot class (one
-    // instantiation per row group serves every block length)
-    dispatch_rg(GQ_, [&](auto GC) {
-        if (dp_.has_fixed)
-            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bb_kernel<GC.value, 8, true>, TPB, 0));
-        else
-            dispatch_s(S_, [&](auto SC) {
-                CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bb_kernel<GC.value, SC.value, false>, TPB,
-                                                                 0));
-            });
-    });
-    int q_per_sm = 0;
-    dispatch_rg(GQ_, [&](auto GC) {
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q_per_sm, q_apply_kernel<GC.value>, TPB, 0));
-    });
-    per_sm = std::min(per_sm, q_per_sm);
+    per_sm = bb_blocks_per_sm(GQ_, S_, dp_.has_fixed);
     if (per_sm < 1)
         throw CudaError("inner BB kernel cannot be made resident");
     bb_grid_ = nsm * std::min(per_sm, 4);
@@ -1440,11 +1250,7 @@ void Solve::setup_bb()
 void Solve::enqueue_q_apply(const double *v, double *qx)
 {
     BBData D = bb_data();
-    int grid = bb_grid_;
-    dispatch_rg(GQ_, [&](auto GC) {
-        void *args[] = {&D, (void *)&v, &qx};
-        CK(cudaLaunchCooperativeKernel((void *)q_apply_kernel<GC.value>, grid, TPB, args, 0, st_));
-    });
+    launch_q_apply(GQ_, bb_grid_, D, v, qx, st_);
     stats_.kernel_launches++;
 }
 
@@ -1593,25 +1399,13 @@ void Solve::launch_dual(const StepData<T> &D, const StepParams &P)
         long_pass(A_, D.A_v, D.xr);
     }
     if (D.n_aff > 0) { // affine cone blocks: one warp each
-        dispatch_s(dp_.S_aff, [&](auto SC) {
-            dual_cone_kernel<SC.value, T><<<grid_for(D.n_aff, WARPS), TPB, 0, s>>>(D, P);
-        });
+        launch_dual_cones(D, P, dp_.S_aff, s);
         stats_.kernel_launches++;
         if (D.n_row_tiles == 0)
             return;
     }
     int grid = grid_for(D.row_tiles ? (long long)D.n_row_tiles : ((long long)m_ + 31) / 32, WARPS);
-    if (eq_rows_) {
-        if (has_g_)
-            dual_kernel<T, true, true><<<grid, TPB, 0, s>>>(D, P);
-        else
-            dual_kernel<T, true, false><<<grid, TPB, 0, s>>>(D, P);
-    } else {
-        if (has_g_)
-            dual_kernel<T, false, true><<<grid, TPB, 0, s>>>(D, P);
-        else
-            dual_kernel<T, false, false><<<grid, TPB, 0, s>>>(D, P);
-    }
+    launch_dual_rows(D, P, eq_rows_, has_g_, grid, s);
     stats_.kernel_launches++;
 }
 
@@ -1652,13 +1446,7 @@ void Solve::enqueue_step_bb(bool store_dual, bool want_fpe, double w)
     }
     BBData D = bb_data();
     BBParams BP{tau, w, prm_.reflection_coefficient, want_fpe ? 1 : 0};
-    dispatch_rg(GQ_, [&](auto GC) {
-        dispatch_s(S_, [&](auto SC) {
-            void *args[] = {&D, &BP};
-            void *k = dp_.has_fixed ? (void *)bb_kernel<GC.value, 8, true> : (void *)bb_kernel<GC.value, SC.value, false>;
-            CK(cudaLaunchCooperativeKernel(k, bb_grid_, TPB, args, 0, s));
-        });
-    });
+    launch_bb(GQ_, S_, dp_.has_fixed, bb_grid_, D, BP, s);
     StepParams P{};
     P.tau = tau;
     P.sigma = step_ * omega_;
@@ -1731,17 +1519,7 @@ void Solve::enqueue_step_t(bool store_primal, bool store_dual, bool want_fpe, do
     if (nfree > 0) {
         int ntiles = D.free_tiles ? D.n_free_tiles : (n_ + 31) / 32;
         int grid = grid_for(ntiles, WARPS);
-        if (hasq) {
-            if (box_free_)
-                primal_free_kernel<T, true, false><<<grid, TPB, 0, s>>>(D, P);
-            else
-                primal_free_kernel<T, true, true><<<grid, TPB, 0, s>>>(D, P);
-        } else {
-            if (box_free_)
-                primal_free_kernel<T, false, false><<<grid, TPB, 0, s>>>(D, P);
-            else
-                primal_free_kernel<T, false, true><<<grid, TPB, 0, s>>>(D, P);
-        }
+        launch_primal_free(D, P, hasq, box_free_, grid, s);
         stats_.kernel_launches++;
     }
     if (D.n_cones > 0)
@@ -1901,10 +1679,7 @@ void Solve::enqueue_residual_t(bool want_dist)
     P.s_aug = sa;
     P.sb = sb_;
     int nb = D.rows_blocks + D.free_blocks + D.cone_blocks + D.aff_blocks;
-    if (dp_.has_fixed) // one slot class for problems with fixed cone slots
-        residual_kernel<8, VT, true><<<nb, TPB, 0, s>>>(D, P);
-    else
-        dispatch_s(std::max(S_, dp_.S_aff), [&](auto SC) { residual_kernel<SC.value, VT, false><<<nb, TPB, 0, s>>>(D, P); });
+    launch_residual(D, P, std::max(S_, dp_.S_aff), dp_.has_fixed, nb, s);
     fold_partials_kernel<<<1, TPB, 0, s>>>(partials_, nb, RS_COUNT, res_ops_d_, scal_d_);
     stats_.kernel_launches += 2;
     stats_.evaluations++;
@@ -2611,18 +2386,12 @@ int step_impl(StepData<double> D, StepParams P, const pdhcg_b200_step_t *t, cuda
     if (nfree > 0) {
         int ntiles = nc > 0 ? D.n_free_tiles : (n + 31) / 32;
         int grid = grid_for(ntiles, WARPS);
-        if (hasq)
-            primal_free_kernel<double, true, true><<<grid, TPB, 0, s>>>(D, P);
-        else
-            primal_free_kernel<double, false, true><<<grid, TPB, 0, s>>>(D, P);
+        launch_primal_free(D, P, hasq, false, grid, s);
     }
     if (nc > 0)
         launch_primal_cones(D, P, split, S, hasq, s);
     int dgrid = grid_for(((long long)t->m + 31) / 32, WARPS);
-    if (t->affine_offset)
-        dual_kernel<double, false, true><<<dgrid, TPB, 0, s>>>(D, P);
-    else
-        dual_kernel<double, false, false><<<dgrid, TPB, 0, s>>>(D, P);
+    launch_dual_rows(D, P, false, t->affine_offset != nullptr, dgrid, s);
     CK(cudaGetLastError());
     if (len_d)
         CK(cudaFreeAsync(len_d, s));
@@ -3005,11 +2774,8 @@ int pdhcg_b200_project_cones(int num_cones, const int *cone_start, const int *co
             return -1;
         }
     }
-    dispatch_s(S, [&](auto SC) {
-        project_cones_kernel<SC.value><<<grid_for(num_cones, WARPS), TPB, 0, s>>>(num_cones, cone_start, len,
-                                                                                 cone_type, cone_alpha, x, d, q,
-                                                                                 tau, psd_work, psd_off_d);
-    });
+    launch_project_cones(S, {num_cones, cone_start, len, cone_type, cone_alpha, x, d, q, tau, psd_work, psd_off_d, nullptr,
+                             nullptr, nullptr}, s);
     cudaFreeAsync(len, s);
     if (psd_work) {
         cudaFreeAsync(psd_work, s);
@@ -3057,10 +2823,8 @@ int pdhcg_b200_project_cone_sections(int num_cones, const int *cone_start, const
         cudaFreeAsync(len, s);
         return -2;
     }
-    dispatch_s(S, [&](auto SC) {
-        project_sections_kernel<SC.value><<<grid_for(num_cones, WARPS), TPB, 0, s>>>(
-            num_cones, cone_start, len, cone_type, cone_alpha, x, d, q, tau, fixed, warm);
-    });
+    launch_project_sections(S, {num_cones, cone_start, len, cone_type, cone_alpha, x, d, q, tau, nullptr, nullptr, fixed,
+                                nullptr, warm}, s);
     cudaFreeAsync(len, s);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
@@ -3095,11 +2859,8 @@ int pdhcg_b200_project_cones_noalloc(int num_cones, const int *cone_start, const
     int S = slots_class(info[0]);
     if (S < 0)
         return -2;
-    dispatch_s(S, [&](auto SC) {
-        project_cones_kernel<SC.value><<<grid_for(num_cones, WARPS), TPB, 0, s>>>(num_cones, cone_start, scratch,
-                                                                                 cone_type, cone_alpha, x, d, q,
-                                                                                 tau, nullptr, nullptr);
-    });
+    launch_project_cones(S, {num_cones, cone_start, scratch, cone_type, cone_alpha, x, d, q, tau, nullptr, nullptr, nullptr,
+                             nullptr, nullptr}, s);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
