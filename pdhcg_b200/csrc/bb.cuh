@@ -392,7 +392,7 @@ __device__ __noinline__ double bb_psd_long_block(const BBData &D, const double *
     const int st = D.cone_start[cb], L = D.cone_len[cb];
     const int n = psd_order(L);
     double *work = D.psd_work + D.psd_off[cb];
-    double *sv = work + 2LL * n * n, *xo_s = sv + L; // candidates, then the values before the step
+    double *sv = psd_stage(work, n), *xo_s = sv + L; // candidates, then the values before the step
     for (int i = lane; i < L; i += 32) {
         const int j = st + i;
         const double mi = D.m_inv ? D.m_inv[j] : 1.0;

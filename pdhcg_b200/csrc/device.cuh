@@ -817,11 +817,19 @@ __device__ inline void exp_cone_point(double r1, double r2, double r3, double d1
 }
 
 // Power cone K_a = {(x, y, z) : x, y >= 0, x^a y^(1-a) >= |z|}: weighted
-// projection min sum w_i (v_i - r_i)^2 over K_a, by the reference's steps
-// (src/kernels/pdhcg_power_cone_kernels.cu:25-133): in-cone and
-// opposite-cone tests, then 80 bisection steps on log |v_z| with x, y the
-// positive roots of the KKT quadratics, on the point scaled by its largest
-// magnitude.
+// projection min sum w_i (v_i - r_i)^2 over K_a (reference
+// src/kernels/pdhcg_power_cone_kernels.cu:25-133): in-cone and opposite-cone
+// tests, then the root in log |v_z| with x, y the positive roots of the KKT
+// quadratics, on the point scaled by its largest magnitude.
+//
+// The reference halves the bracket 80 times.  Each halving is a serial chain
+// of an exp, two hypots, two square roots and two logs, and with one lane at
+// work those 80 chains set the length of the launch (100 us a step on 60
+// such blocks).  The warp instead tests 32 points of the bracket at once and
+// keeps the interval between the last point below the root and the first
+// above it: a factor of 33 per round, so 13 rounds narrow log DBL_MIN ..
+// log |z| past the resolution of a double (708 / 33^13 < 2e-17), the same
+// root to its last bits.  The search also ends when a round cannot narrow it.
 __device__ inline double pow_pos_root(double r, double q)
 {
     if (!(q > 0.0))
@@ -830,8 +838,9 @@ __device__ inline double pow_pos_root(double r, double q)
     return r >= 0.0 ? 0.5 * (r + disc) : (2.0 * q) / (disc - r);
 }
 
+// All lanes of the warp call it with the same block.
 __device__ inline void pow_cone_point(double rx, double ry, double rz, double wx, double wy, double wz, double a,
-                                      double &ox, double &oy, double &oz)
+                                      int lane, double &ox, double &oy, double &oz)
 {
     double s = fmax(fabs(rx), fmax(fabs(ry), fabs(rz)));
     if (!(s > 0.0) || !isfinite(s))
@@ -867,14 +876,19 @@ __device__ inline void pow_cone_point(double rx, double ry, double rz, double wx
         oz = 0.0;
         return;
     }
-    for (int it = 0; it < 80; ++it) {
-        const double lr = lo + 0.5 * (hi - lo), rho = exp(lr);
+    for (int it = 0; it < 13; ++it) {
+        const double w = (hi - lo) * (1.0 / 33.0);
+        const double lr = lo + w * (lane + 1), rho = exp(lr);
         const double x = pow_pos_root(rx, 0.25 * cx * rho * (az - rho));
         const double y = pow_pos_root(ry, 0.25 * cy * rho * (az - rho));
-        if (x > 0.0 && y > 0.0 && a * log(x) + om * log(y) > lr)
-            lo = lr;
-        else
-            hi = lr;
+        const bool below = x > 0.0 && y > 0.0 && a * log(x) + om * log(y) > lr;
+        const unsigned above = ~__ballot_sync(FULL, below);
+        const int c = above ? __ffs(above) - 1 : 32; // points below the root
+        const double l2 = c > 0 ? lo + w * c : lo, h2 = c < 32 ? lo + w * (c + 1) : hi;
+        if (!(h2 - l2 < hi - lo))
+            break;
+        lo = l2;
+        hi = h2;
     }
     const double rho = exp(lo + 0.5 * (hi - lo));
     const double x = pow_pos_root(rx, 0.25 * cx * rho * (az - rho));
@@ -884,32 +898,11 @@ __device__ inline void pow_cone_point(double rx, double ry, double rz, double wx
     oz = (rz >= 0.0 ? 1.0 : -1.0) * fmin(rho, exp(a * log(x) + om * log(y))) * s;
 }
 
-// Projection of one 3-slot EXP (type 2) or POW (type 3) block: metric w,
-// scaling d.  Only the one-slot (S = 1) instantiations of the cone-block
-// bodies reach it, so its Newton / bisection loops stay out of the wide SOC
-// bodies' register allocation.
-__device__ __forceinline__ double3 cone3_point(int type, double3 x, double3 d, double3 w, double alpha)
-{
-    double3 o;
-    if (type == 2) { // exponential: the sqrt(w) change of variables
-        const double s0 = sqrt(w.x > 0.0 ? w.x : 1.0), s1 = sqrt(w.y > 0.0 ? w.y : 1.0),
-                     s2 = sqrt(w.z > 0.0 ? w.z : 1.0);
-        exp_cone_point(s0 * x.x, s1 * x.y, s2 * x.z, s0 * d.x, s1 * d.y, s2 * d.z, o.x, o.y, o.z);
-        o.x /= s0;
-        o.y /= s1;
-        o.z /= s2;
-    } else { // power: scaled space, weights w d^2
-        pow_cone_point(x.x / d.x, x.y / d.y, x.z / d.z, w.x * d.x * d.x, w.y * d.y * d.y, w.z * d.z * d.z, alpha,
-                       o.x, o.y, o.z);
-        o.x *= d.x;
-        o.y *= d.y;
-        o.z *= d.z;
-    }
-    return o;
-}
-
-// A 3-slot block held in lanes 0..2 (S = 1 slot each): lane 0 gathers it,
-// projects it and hands the result back.
+// A 3-slot block held in lanes 0..2 (S = 1 slot each), metric w, scaling d:
+// an exponential block (type 2) is projected by lane 0, a power block (type
+// 3) by the whole warp; the result goes back to the three lanes.  Only the
+// one-slot (S = 1) instantiations of the cone-block bodies reach it, so its
+// loops stay out of the wide SOC bodies' register allocation.
 template <int S>
 __device__ __forceinline__ void warp_project3(int type, WarpSlots<S> &sl, int lane, double alpha)
 {
@@ -924,11 +917,27 @@ __device__ __forceinline__ void warp_project3(int type, WarpSlots<S> &sl, int la
     w.y = __shfl_sync(FULL, sl.w[0], 1);
     w.z = __shfl_sync(FULL, sl.w[0], 2);
     double3 o = make_double3(0.0, 0.0, 0.0);
-    if (lane == 0)
-        o = cone3_point(type, x, d, w, alpha);
-    const double r0 = __shfl_sync(FULL, o.x, 0), r1 = __shfl_sync(FULL, o.y, 0), r2 = __shfl_sync(FULL, o.z, 0);
+    if (type == 2) {
+        if (lane == 0) { // the sqrt(w) change of variables
+            const double s0 = sqrt(w.x > 0.0 ? w.x : 1.0), s1 = sqrt(w.y > 0.0 ? w.y : 1.0),
+                         s2 = sqrt(w.z > 0.0 ? w.z : 1.0);
+            exp_cone_point(s0 * x.x, s1 * x.y, s2 * x.z, s0 * d.x, s1 * d.y, s2 * d.z, o.x, o.y, o.z);
+            o.x /= s0;
+            o.y /= s1;
+            o.z /= s2;
+        }
+        o.x = __shfl_sync(FULL, o.x, 0);
+        o.y = __shfl_sync(FULL, o.y, 0);
+        o.z = __shfl_sync(FULL, o.z, 0);
+    } else { // scaled space, weights w d^2
+        pow_cone_point(x.x / d.x, x.y / d.y, x.z / d.z, w.x * d.x * d.x, w.y * d.y * d.y, w.z * d.z * d.z, alpha, lane,
+                       o.x, o.y, o.z);
+        o.x *= d.x;
+        o.y *= d.y;
+        o.z *= d.z;
+    }
     if (lane < 3)
-        sl.x[0] = lane == 0 ? r0 : (lane == 1 ? r1 : r2);
+        sl.x[0] = lane == 0 ? o.x : (lane == 1 ? o.y : o.z);
 }
 
 // Cone kinds an instantiation carries: SOC / RSOC (any S), and the 3-slot
@@ -939,14 +948,22 @@ __device__ __forceinline__ void warp_project3(int type, WarpSlots<S> &sl, int la
 // reference's packing, src/kernels/pdhcg_psd_cone_kernels.cu:65-91).  The
 // projection is the Frobenius one in the scaled space, as the reference
 // takes it (:415-475; no metric): the warp unpacks X into work[0, n^2)
-// (this block's device scratch, row-major), runs cyclic Jacobi with
-// Rutishauser's rotation on it while accumulating the eigenvectors in
-// work[n^2, 2 n^2), clips the negative eigenvalues and repacks.  Every
-// lane takes the same rotation from the same entries; lane k updates row /
-// column entry k of the two rotated rows and columns, so the arithmetic of
-// each entry is that of the sequential method.  Stops when the
-// off-diagonal mass is below 1e-28 of the whole (at most 100 sweeps).
-// n <= PSD_MAX_ORDER (L <= 256 slots, S <= 8).
+// (this block's device scratch), diagonalises it by Jacobi rotations while
+// accumulating the eigenvectors in work[n^2, 2 n^2), clips the negative
+// eigenvalues and repacks.
+//
+// A sweep visits the pairs in round-robin order (the tournament ordering of
+// Brent and Luk 1985): n - 1 rounds (n for odd n) of n / 2 disjoint pairs.  A
+// round's rotations are independent, so lane i computes the angle of pair
+// i, and the two-sided update splits into 2 x 2 blocks (pair i's rows,
+// pair j's columns) that each read and write only themselves: one barrier
+// between the angles and the update, one after it.  Visiting the pairs one
+// at a time instead (n (n - 1) / 2 angle computations in series, each some
+// 600 cycles of divisions and square roots, and four barriers) took 2 ms for
+// a block of order 20.  The rotation is Rutishauser's; the search stops when
+// the off-diagonal mass is below 1e-28 of the whole (at most 100 sweeps).
+// Blocks of order up to PSD_MAX_ORDER (L <= 256 slots) are held in the warp's
+// registers between the steps, longer ones in memory.
 // ---------------------------------------------------------------------------
 constexpr int PSD_MAX_ORDER = 22;
 constexpr int PSD_MAX_SWEEPS = 100;
@@ -962,6 +979,130 @@ __device__ __forceinline__ void psd_slot_rc(int i, int n, int &row, int &col)
     }
     col = c;
     row = c + (i - first);
+}
+
+// Scratch of one block in doubles: A, the eigenvectors (V^T, one per row),
+// and the cosine and sine of each pair of a round.
+__host__ __device__ constexpr long long psd_work_doubles(long long order)
+{
+    return 2 * order * order + 2 * ((order + 1) / 2);
+}
+
+// Diagonalises the symmetric n x n matrix A (full, row-major) in place by
+// round-robin Jacobi; row e of Vt receives the e-th eigenvector.  Every lane
+// of the warp calls it; A is visible to all of them.
+__device__ inline void warp_jacobi(double *A, double *Vt, double *cs, int n, int lane)
+{
+    for (int e = lane; e < n * n; e += 32)
+        Vt[e] = (e / n == e % n) ? 1.0 : 0.0;
+    __syncwarp();
+    const int m = n + (n & 1), np = m / 2; // odd n: index n is a bye
+    // pair i of round r: {m - 1, r}, then {r + i, r - i} modulo m - 1
+    auto pair_of = [&](int r, int i, int &p, int &q) {
+        int a = m - 1, b = r;
+        if (i > 0) {
+            a = r + i;
+            b = r - i;
+            if (a >= m - 1)
+                a -= m - 1;
+            if (b < 0)
+                b += m - 1;
+        }
+        p = min(a, b);
+        q = max(a, b);
+    };
+    for (int sweep = 0; sweep < PSD_MAX_SWEEPS; ++sweep) {
+        double off = 0.0, all = 0.0;
+        for (int r = 0; r < n; ++r)
+            for (int k = lane; k < n; k += 32) {
+                const double a = A[(size_t)r * n + k], a2 = a * a;
+                all += a2;
+                if (k != r)
+                    off += a2;
+            }
+        off = warp_sum(off);
+        all = warp_sum(all);
+        if (!(off > PSD_OFF_REL * all))
+            break;
+        for (int r = 0; r < m - 1; ++r) {
+            for (int i = lane; i < np; i += 32) {
+                int p, q;
+                pair_of(r, i, p, q);
+                double c = 1.0, sn = 0.0;
+                if (q < n) {
+                    const double apq = A[(size_t)p * n + q];
+                    if (apq != 0.0) {
+                        const double theta = (A[(size_t)q * n + q] - A[(size_t)p * n + p]) / (2.0 * apq);
+                        const double t = fabs(theta) > 1e150
+                                             ? 0.5 / theta
+                                             : (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+                        c = 1.0 / sqrt(t * t + 1.0);
+                        sn = t * c;
+                    }
+                }
+                cs[2 * i] = c;
+                cs[2 * i + 1] = sn;
+            }
+            __syncwarp();
+            // 2 x 2 blocks (i, j), i <= j, and their mirror images
+            for (int t = lane; t < np * (np + 1) / 2; t += 32) {
+                int j = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+                while ((j + 1) * (j + 2) / 2 <= t)
+                    ++j;
+                while (j * (j + 1) / 2 > t)
+                    --j;
+                const int i = t - j * (j + 1) / 2;
+                int pi, qi, pj, qj;
+                pair_of(r, i, pi, qi);
+                pair_of(r, j, pj, qj);
+                const double ci = cs[2 * i], si = cs[2 * i + 1], cj = cs[2 * j], sj = cs[2 * j + 1];
+                const bool fi = qi < n, fj = qj < n; // false: the bye's partner, one row or column
+                const double app = A[(size_t)pi * n + pj], apq = fj ? A[(size_t)pi * n + qj] : 0.0;
+                const double aqp = fi ? A[(size_t)qi * n + pj] : 0.0, aqq = fi && fj ? A[(size_t)qi * n + qj] : 0.0;
+                // columns by pair j, then rows by pair i
+                const double bpp = cj * app - sj * apq, bpq = sj * app + cj * apq;
+                const double bqp = cj * aqp - sj * aqq, bqq = sj * aqp + cj * aqq;
+                const double dpp = ci * bpp - si * bqp, dqp = si * bpp + ci * bqp;
+                double dpq = ci * bpq - si * bqq, dqq = si * bpq + ci * bqq;
+                if (i == j) { // the rotated pair itself
+                    A[(size_t)pi * n + pi] = dpp;
+                    if (fi) {
+                        A[(size_t)qi * n + qi] = dqq;
+                        A[(size_t)pi * n + qi] = 0.0;
+                        A[(size_t)qi * n + pi] = 0.0;
+                    }
+                } else {
+                    A[(size_t)pi * n + pj] = dpp;
+                    A[(size_t)pj * n + pi] = dpp;
+                    if (fj) {
+                        A[(size_t)pi * n + qj] = dpq;
+                        A[(size_t)qj * n + pi] = dpq;
+                    }
+                    if (fi) {
+                        A[(size_t)qi * n + pj] = dqp;
+                        A[(size_t)pj * n + qi] = dqp;
+                    }
+                    if (fi && fj) {
+                        A[(size_t)qi * n + qj] = dqq;
+                        A[(size_t)qj * n + qi] = dqq;
+                    }
+                }
+            }
+            for (int j = 0; j < np; ++j) {
+                int p, q;
+                pair_of(r, j, p, q);
+                if (q >= n)
+                    continue;
+                const double c = cs[2 * j], sn = cs[2 * j + 1];
+                for (int k = lane; k < n; k += 32) {
+                    const double vp = Vt[(size_t)p * n + k], vq = Vt[(size_t)q * n + k];
+                    Vt[(size_t)p * n + k] = c * vp - sn * vq;
+                    Vt[(size_t)q * n + k] = sn * vp + c * vq;
+                }
+            }
+            __syncwarp();
+        }
+    }
 }
 
 template <int S>
@@ -988,7 +1129,7 @@ __device__ void warp_project_psd(WarpSlots<S> &sl, int L, int lane, double *work
         return;
     }
     const double R2 = 1.41421356237309504880, IR2 = 0.70710678118654752440;
-    double *A = work, *V = work + n * n;
+    double *A = work, *Vt = work + n * n;
 #pragma unroll
     for (int s = 0; s < S; ++s) {
         const int i = lane + 32 * s;
@@ -1000,56 +1141,8 @@ __device__ void warp_project_psd(WarpSlots<S> &sl, int L, int lane, double *work
             A[col * n + row] = v;
         }
     }
-    for (int e = lane; e < n * n; e += 32)
-        V[e] = (e / n == e % n) ? 1.0 : 0.0;
     __syncwarp();
-    for (int sweep = 0; sweep < PSD_MAX_SWEEPS; ++sweep) {
-        double off = 0.0, all = 0.0;
-        for (int e = lane; e < n * n; e += 32) {
-            const double a2 = A[e] * A[e];
-            all += a2;
-            if (e / n != e % n)
-                off += a2;
-        }
-        off = warp_sum(off);
-        all = warp_sum(all);
-        if (!(off > PSD_OFF_REL * all))
-            break;
-        for (int p = 0; p < n - 1; ++p)
-            for (int q = p + 1; q < n; ++q) {
-                const double apq = A[p * n + q];
-                if (apq == 0.0)
-                    continue;
-                const double theta = (A[q * n + q] - A[p * n + p]) / (2.0 * apq);
-                const double t = fabs(theta) > 1e150
-                                     ? 0.5 / theta
-                                     : (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-                const double c = 1.0 / sqrt(t * t + 1.0), sn = t * c;
-                __syncwarp(); // every lane has read a_pp, a_qq, a_pq
-                if (lane < n) { // columns p, q of A and V
-                    const int k = lane;
-                    const double akp = A[k * n + p], akq = A[k * n + q];
-                    A[k * n + p] = c * akp - sn * akq;
-                    A[k * n + q] = sn * akp + c * akq;
-                    const double vkp = V[k * n + p], vkq = V[k * n + q];
-                    V[k * n + p] = c * vkp - sn * vkq;
-                    V[k * n + q] = sn * vkp + c * vkq;
-                }
-                __syncwarp();
-                if (lane < n) { // rows p, q of A
-                    const int k = lane;
-                    const double apk = A[p * n + k], aqk = A[q * n + k];
-                    A[p * n + k] = c * apk - sn * aqk;
-                    A[q * n + k] = sn * apk + c * aqk;
-                }
-                __syncwarp();
-                if (lane == 0) {
-                    A[p * n + q] = 0.0;
-                    A[q * n + p] = 0.0;
-                }
-                __syncwarp();
-            }
-    }
+    warp_jacobi(A, Vt, work + 2 * n * n, n, lane);
 #pragma unroll
     for (int s = 0; s < S; ++s) {
         const int i = lane + 32 * s;
@@ -1058,7 +1151,7 @@ __device__ void warp_project_psd(WarpSlots<S> &sl, int L, int lane, double *work
             psd_slot_rc(i, n, row, col);
             double v = 0.0;
             for (int e = 0; e < n; ++e)
-                v += fmax(A[e * n + e], 0.0) * V[row * n + e] * V[col * n + e];
+                v += fmax(A[e * n + e], 0.0) * Vt[e * n + row] * Vt[e * n + col];
             sl.x[s] = row == col ? v : v * R2;
         }
     }
@@ -1067,11 +1160,10 @@ __device__ void warp_project_psd(WarpSlots<S> &sl, int L, int lane, double *work
 
 // PSD blocks of any order ("long" blocks: more slots than a warp's
 // registers hold, L > 32 S).  The svec lies in memory (in, L doubles; out
-// may alias it); the warp unpacks it into work[0, n^2), runs the same
-// cyclic Jacobi as warp_project_psd with every row / column loop strided
-// over the lanes, clips and repacks into out.  Callers stage the block's
-// candidate in its scratch (after the 2 n^2 doubles of the decomposition)
-// and call this instead of the register form.
+// may alias it); the warp unpacks it into work[0, n^2), diagonalises it as
+// above, clips and repacks into out.  Callers stage the block's candidate in
+// its scratch (psd_stage, after the decomposition's doubles) and call this
+// instead of the register form.
 __device__ __forceinline__ int psd_order(int L)
 {
     int n = (int)floor(sqrt(2.0 * L));
@@ -1082,15 +1174,18 @@ __device__ __forceinline__ int psd_order(int L)
     return n;
 }
 
-// L doubles of candidate staging per long block, after its 2 n^2 doubles
-// (the residual stages three vectors, so 3 L are kept)
+__device__ __forceinline__ double *psd_stage(double *work, int n) { return work + psd_work_doubles(n); }
+
+// a block's whole scratch: L doubles of candidate staging per long block,
+// after the decomposition's (the residual stages three vectors, so 3 L are
+// kept)
 __host__ __device__ inline long long psd_scratch_doubles(int order, bool is_long)
 {
     const long long L = (long long)order * (order + 1) / 2;
-    return 2LL * order * order + (is_long ? 3 * L : 0);
+    return psd_work_doubles(order) + (is_long ? 3 * L : 0);
 }
 
-static __device__ void warp_project_psd_mem(const double *in, double *out, int L, int lane, double *work)
+__device__ inline void warp_project_psd_mem(const double *in, double *out, int L, int lane, double *work)
 {
     const int n = psd_order(L);
     if (n == 1) {
@@ -1109,7 +1204,7 @@ static __device__ void warp_project_psd_mem(const double *in, double *out, int L
         return;
     }
     const double R2 = 1.41421356237309504880, IR2 = 0.70710678118654752440;
-    double *A = work, *V = work + (size_t)n * n;
+    double *A = work, *Vt = work + (size_t)n * n;
     for (int col = 0, first = 0; col < n; first += n - col, ++col)
         for (int row = col + lane; row < n; row += 32) {
             const double x = in[first + row - col];
@@ -1117,59 +1212,13 @@ static __device__ void warp_project_psd_mem(const double *in, double *out, int L
             A[(size_t)row * n + col] = v;
             A[(size_t)col * n + row] = v;
         }
-    for (long long e = lane; e < (long long)n * n; e += 32)
-        V[e] = (e / n == e % n) ? 1.0 : 0.0;
     __syncwarp();
-    for (int sweep = 0; sweep < PSD_MAX_SWEEPS; ++sweep) {
-        double off = 0.0, all = 0.0;
-        for (long long e = lane; e < (long long)n * n; e += 32) {
-            const double a2 = A[e] * A[e];
-            all += a2;
-            if (e / n != e % n)
-                off += a2;
-        }
-        off = warp_sum(off);
-        all = warp_sum(all);
-        if (!(off > PSD_OFF_REL * all))
-            break;
-        for (int p = 0; p < n - 1; ++p)
-            for (int q = p + 1; q < n; ++q) {
-                const double apq = A[(size_t)p * n + q];
-                if (apq == 0.0)
-                    continue;
-                const double theta = (A[(size_t)q * n + q] - A[(size_t)p * n + p]) / (2.0 * apq);
-                const double t = fabs(theta) > 1e150
-                                     ? 0.5 / theta
-                                     : (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-                const double c = 1.0 / sqrt(t * t + 1.0), sn = t * c;
-                __syncwarp(); // every lane has read a_pp, a_qq, a_pq
-                for (int k = lane; k < n; k += 32) { // columns p, q of A and V
-                    const double akp = A[(size_t)k * n + p], akq = A[(size_t)k * n + q];
-                    A[(size_t)k * n + p] = c * akp - sn * akq;
-                    A[(size_t)k * n + q] = sn * akp + c * akq;
-                    const double vkp = V[(size_t)k * n + p], vkq = V[(size_t)k * n + q];
-                    V[(size_t)k * n + p] = c * vkp - sn * vkq;
-                    V[(size_t)k * n + q] = sn * vkp + c * vkq;
-                }
-                __syncwarp();
-                for (int k = lane; k < n; k += 32) { // rows p, q of A
-                    const double apk = A[(size_t)p * n + k], aqk = A[(size_t)q * n + k];
-                    A[(size_t)p * n + k] = c * apk - sn * aqk;
-                    A[(size_t)q * n + k] = sn * apk + c * aqk;
-                }
-                __syncwarp();
-                if (lane == 0) {
-                    A[(size_t)p * n + q] = 0.0;
-                    A[(size_t)q * n + p] = 0.0;
-                }
-                __syncwarp();
-            }
-    }
+    warp_jacobi(A, Vt, work + 2 * (size_t)n * n, n, lane);
     for (int col = 0, first = 0; col < n; first += n - col, ++col)
         for (int row = col + lane; row < n; row += 32) {
             double v = 0.0;
             for (int e = 0; e < n; ++e)
-                v += fmax(A[(size_t)e * n + e], 0.0) * V[(size_t)row * n + e] * V[(size_t)col * n + e];
+                v += fmax(A[(size_t)e * n + e], 0.0) * Vt[(size_t)e * n + row] * Vt[(size_t)e * n + col];
             out[first + row - col] = row == col ? v : v * R2;
         }
     __syncwarp(); // the scratch and out may be read by other lanes next
@@ -1177,7 +1226,7 @@ static __device__ void warp_project_psd_mem(const double *in, double *out, int L
 
 // Cone kinds an instantiation carries: SOC / RSOC (any S), the 3-slot
 // exponential / power cones (S = 1 only; callers route those blocks there)
-// and PSD blocks (psd: this block's scratch of 2 n^2 doubles).  Blocks with
+// and PSD blocks (psd: this block's scratch).  Blocks with
 // fixed slots (any type but PSD) are a launch class of their own,
 // CONES_SECTION, projected by section.cuh.
 enum ConeKinds { CONES_WIDE = 1, CONES_THREE = 2, CONES_PSD = 4, CONES_ALL = 7, CONES_SECTION = 8 };

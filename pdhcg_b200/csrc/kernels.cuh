@@ -244,7 +244,7 @@ __device__ __noinline__ void primal_psd_long_block(const StepData<T> &D, const S
     const int st = D.cone_start[cb], L = D.cone_len[cb];
     const int n = psd_order(L);
     double *work = D.psd_work + D.psd_off[cb];
-    double *sv = work + 2LL * n * n;
+    double *sv = psd_stage(work, n);
     for (int c0 = 0; c0 < L; c0 += 32 * S) {
         const int nr = min(32 * S, L - c0);
         double aty[S];

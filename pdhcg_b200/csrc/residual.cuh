@@ -234,7 +234,7 @@ __device__ __forceinline__ void residual_psd_long_block(const ResidualData<VT> &
     const int st = D.cone_start[cb], L = D.cone_len[cb];
     const int n = psd_order(L);
     double *work = D.psd_work + D.psd_off[cb];
-    double *rcv = work + 2LL * n * n, *augv = rcv + L, *atyv = augv + L;
+    double *rcv = psd_stage(work, n), *augv = rcv + L, *atyv = augv + L;
     auto qx_of = [&](int j, double x) {
         return P.qmode == 1 ? D.q[j] * x : (P.qmode == 2 ? D.qx[j] : 0.0);
     };

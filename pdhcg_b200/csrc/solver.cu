@@ -672,7 +672,7 @@ std::unique_ptr<DeviceProblem> make_device_problem(const qp_problem_t *p, cudaSt
                 if (vd > PSD_MAX_ORDER)
                     d.unsupported = "affine PSD blocks of order above 22 are not supported yet";
                 d.has_psd = true;
-                d.psd_total += 2LL * vd * vd;
+                d.psd_total += psd_work_doubles(vd);
             }
             amax = std::max(amax, len);
             for (int i = st; i < st + len && i < d.m; ++i)
@@ -2747,7 +2747,7 @@ int pdhcg_b200_project_cones(int num_cones, const int *cone_start, const int *co
                                     t[i] == CONE_PSD);
             if (t[i] == CONE_PSD) {
                 psd_off[i] = psd_total;
-                psd_total += 2LL * vd[i] * vd[i];
+                psd_total += psd_work_doubles(vd[i]);
             }
         }
     }
