@@ -22,7 +22,9 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -187,6 +189,20 @@ struct SplitWs {
     size_t cap = 0;
 };
 
+int grow_ws(SplitWs &ws, size_t need)
+{
+    if (need <= ws.cap)
+        return 0;
+    if (ws.p)
+        cudaFree(ws.p);
+    ws.p = nullptr;
+    ws.cap = 0;
+    if (cudaMalloc((void **)&ws.p, need * sizeof(float)) != cudaSuccess)
+        return -1;
+    ws.cap = need;
+    return 0;
+}
+
 template <bool TA, bool TB, typename AT, typename BT>
 int gemm(int M, int N, int K, const AT *A, int lda, const BT *B, int ldb, float *C, int ldc, float alpha, float beta,
          cudaStream_t s, SplitWs &ws)
@@ -200,16 +216,8 @@ int gemm(int M, int N, int K, const AT *A, int lda, const BT *B, int ldb, float 
     kchunk = (kchunk + TK - 1) / TK * TK;
     splits = (K + kchunk - 1) / kchunk;
     if (splits > 1) {
-        const size_t need = (size_t)splits * M * N;
-        if (need > ws.cap) {
-            if (ws.p)
-                cudaFree(ws.p);
-            ws.p = nullptr;
-            ws.cap = 0;
-            if (cudaMalloc((void **)&ws.p, need * sizeof(float)) != cudaSuccess)
-                return -1;
-            ws.cap = need;
-        }
+        if (grow_ws(ws, (size_t)splits * M * N))
+            return -1;
         mma_gemm_kernel<TA, TB, AT, BT><<<dim3(gn, gm, splits), 128, 0, s>>>(M, N, K, kchunk, A, lda, B, ldb, C, ldc,
                                                                             alpha, beta, ws.p);
         const long long MN = (long long)M * N;
@@ -344,20 +352,550 @@ __global__ void to_bf16_kernel(long long n, const float *src, bf16 *dst)
         dst[e] = __float2bfloat16_rn(src[e]);
 }
 
-__global__ void adam_kernel(long long n, float *w, const float *g, float *mom, float *vel, float lr, float b1, float b2,
-                            float c1, float c2, float eps)
+int blocks_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 148 * 8); }
+
+// ---------------------------------------------------------------------------
+// The trunk's products for one minibatch (at most SMALL_B rows).  They are
+// latency bound, not throughput bound (64 x 512 x 512 is 34 MFLOP), so a CTA
+// owns only a 32 x 16 tile and its 8 warps split K, loading their fragments
+// straight from L2 (no staging: each element is used by one warp) with every
+// load of a warp in flight at once; the 8 partial tiles are added in warp
+// order in shared memory and the epilogue (bias, ReLU, the ReLU mask of the
+// backward pass, the log-weight head's outer product) runs on the sum.  Same
+// arithmetic as mma_gemm_kernel: BF16 pairs for FP32 operands, FP32 sums.
+// ---------------------------------------------------------------------------
+constexpr int SMALL_B = 128;           // rows up to which the minibatch kernels are used
+constexpr int SM_M = 32, SM_N = 16;    // tile
+constexpr int SM_W = 8;                // warps, K split over them
+
+enum SmallEpi { EPI_PLAIN, EPI_BIAS, EPI_BIAS_RELU, EPI_MASK, EPI_MASK_OUTER };
+
+struct SmallGemm {
+    int M, N, K;
+    const void *A, *B;
+    int lda, ldb;
+    float *C; // ldc = N
+    const float *bias;        // EPI_BIAS*: [N]
+    const float *mask;        // EPI_MASK*: C is kept where mask > 0, 0 elsewhere ([M x N])
+    const float *col, *row;   // EPI_MASK_OUTER: + col[i] * row[j] before the mask
+    __host__ __device__ int tiles() const { return ((M + SM_M - 1) / SM_M) * ((N + SM_N - 1) / SM_N); }
+};
+
+// (v0, v1) as a BF16 pair in one register, hi parts and lo parts
+__device__ __forceinline__ void split2(float v0, float v1, unsigned &hi, unsigned &lo)
 {
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        float gg = g[e];
-        float mm = b1 * mom[e] + (1.0f - b1) * gg;
-        float vv = b2 * vel[e] + (1.0f - b2) * gg * gg;
-        mom[e] = mm;
-        vel[e] = vv;
-        w[e] -= lr * (mm / c1) / (sqrtf(vv / c2) + eps);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
+    const float2 hf = __bfloat1622float2(h);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(v0 - hf.x, v1 - hf.y);
+    hi = *reinterpret_cast<const unsigned *>(&h);
+    lo = *reinterpret_cast<const unsigned *>(&l);
+}
+
+// elements (i, k) and (i, k + 1) of a matrix stored [i][k] (KFAST) or [k][i]
+template <bool KFAST, typename T>
+__device__ __forceinline__ float2 pair_at(const T *p, int ld, int i, int k, int I, int K)
+{
+    float2 v = make_float2(0.0f, 0.0f);
+    if (i < I) {
+        if (k < K)
+            v.x = ::ld(KFAST ? p + (size_t)i * ld + k : p + (size_t)k * ld + i);
+        if (k + 1 < K)
+            v.y = ::ld(KFAST ? p + (size_t)i * ld + k + 1 : p + (size_t)(k + 1) * ld + i);
+    }
+    return v;
+}
+
+template <bool TA, bool TB, typename AT, typename BT, int EPI>
+__device__ __forceinline__ void small_gemm_tile(const SmallGemm &G, int tile, float (*red)[SM_M * SM_N])
+{
+    constexpr bool SA = !std::is_same<AT, bf16>::value, SB = !std::is_same<BT, bf16>::value;
+    const AT *A = (const AT *)G.A;
+    const BT *B = (const BT *)G.B;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int nt_n = (G.N + SM_N - 1) / SM_N;
+    const int i0 = (tile / nt_n) * SM_M, j0 = (tile % nt_n) * SM_N;
+    float acc[2][2][4] = {};
+    const int steps = (G.K + 15) / 16;
+    const int s0 = steps * warp / SM_W, s1 = steps * (warp + 1) / SM_W;
+#pragma unroll 4
+    for (int st = s0; st < s1; ++st) {
+        const int k0 = 16 * st + 2 * t;
+        unsigned a[2][2][4], b[2][2][2];
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float2 v = pair_at<!TA>(A, G.lda, i0 + 16 * mt + g + 8 * (q & 1), k0 + 8 * (q >> 1), G.M, G.K);
+                split2(v.x, v.y, a[0][mt][q], a[1][mt][q]);
+            }
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const float2 v = pair_at<TB>(B, G.ldb, j0 + 8 * nt + g, k0 + 8 * q, G.N, G.K);
+                split2(v.x, v.y, b[0][nt][q], b[1][nt][q]);
+            }
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+                if (SA)
+                    mma_bf16(acc[mt][nt], a[1][mt], b[0][nt]);
+                if (SB)
+                    mma_bf16(acc[mt][nt], a[0][mt], b[1][nt]);
+                mma_bf16(acc[mt][nt], a[0][mt], b[0][nt]);
+            }
+    }
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                red[warp][(16 * mt + g + 8 * (q >> 1)) * SM_N + 8 * nt + 2 * t + (q & 1)] = acc[mt][nt][q];
+    __syncthreads();
+    for (int e = threadIdx.x; e < SM_M * SM_N; e += 32 * SM_W) {
+        float v = red[0][e];
+#pragma unroll
+        for (int w = 1; w < SM_W; ++w)
+            v += red[w][e];
+        const int i = i0 + e / SM_N, j = j0 + e % SM_N;
+        if (i < G.M && j < G.N) {
+            if (EPI == EPI_BIAS || EPI == EPI_BIAS_RELU)
+                v += G.bias[j];
+            if (EPI == EPI_BIAS_RELU)
+                v = fmaxf(v, 0.0f);
+            if (EPI == EPI_MASK_OUTER)
+                v += G.col[i] * G.row[j];
+            if ((EPI == EPI_MASK || EPI == EPI_MASK_OUTER) && !(G.mask[(size_t)i * G.N + j] > 0.0f))
+                v = 0.0f;
+            G.C[(size_t)i * G.N + j] = v;
+        }
     }
 }
 
-int blocks_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 148 * 8); }
+// One layer of the forward pass.  LAST: the low-rank layer's launch carries
+// one more block, the log-weight head: a warp per row of h2, lanes over the
+// hidden units (one thread per row took 512 dependent loads).
+struct HeadArgs {
+    int B, H;
+    const float *h2, *wp, *bp, *tl; // tl NULL: prediction only
+    float *lw, *dlw;
+    double *loss;
+};
+
+template <int EPI, bool LAST>
+__global__ void __launch_bounds__(32 * SM_W) small_layer_kernel(SmallGemm G, HeadArgs h)
+{
+    __shared__ float red[SM_W][SM_M * SM_N];
+    if (LAST && (int)blockIdx.x == G.tiles()) {
+        __shared__ double sq[SM_W];
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        double a = 0.0;
+        for (int b = warp; b < h.B; b += SM_W) {
+            float s = 0.0f;
+            for (int k = lane; k < h.H; k += 32)
+                s += h.wp[k] * h.h2[(size_t)b * h.H + k];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                s += __shfl_xor_sync(0xffffffffu, s, o);
+            s += h.bp[0];
+            if (lane == 0) {
+                h.lw[b] = s;
+                if (h.tl) {
+                    const float r = s - h.tl[b];
+                    h.dlw[b] = 2.0f * r / (float)h.B;
+                    a += (double)r * (double)r;
+                }
+            }
+        }
+        if (lane == 0)
+            sq[warp] = a;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < SM_W; ++w)
+                a += sq[w];
+            h.loss[0] = a / (double)h.B;
+        }
+        return;
+    }
+    small_gemm_tile<false, true, float, bf16, EPI>(G, blockIdx.x, red);
+}
+
+// One layer of the backward pass: the tiles of dX = dY W (masked by the ReLU
+// of the layer below), then the tiles of dW = dY^T X, whose first column of
+// tiles also sums db over the rows; OUTER: then the log-weight head's
+// gradients.  dY: [B x out], X: [B x in].
+struct BackArgs {
+    SmallGemm dx, dw;
+    float *db;
+    const float *dlw, *h2;
+    float *gwp, *gbp;
+    int B, H;
+};
+
+template <bool OUTER, bool DX>
+__global__ void __launch_bounds__(32 * SM_W) small_back_kernel(BackArgs P)
+{
+    __shared__ float red[SM_W][SM_M * SM_N];
+    int tile = blockIdx.x;
+    if (DX) {
+        if (tile < P.dx.tiles()) {
+            small_gemm_tile<false, false, float, bf16, OUTER ? EPI_MASK_OUTER : EPI_MASK>(P.dx, tile, red);
+            return;
+        }
+        tile -= P.dx.tiles();
+    }
+    if (tile < P.dw.tiles()) {
+        small_gemm_tile<true, false, float, float, EPI_PLAIN>(P.dw, tile, red);
+        const int nt_n = (P.dw.N + SM_N - 1) / SM_N;
+        const int i = (tile / nt_n) * SM_M + (int)threadIdx.x;
+        if (tile % nt_n == 0 && threadIdx.x < SM_M && i < P.dw.M) { // rows summed in order
+            const float *dy = (const float *)P.dw.A;
+            float s = 0.0f;
+#pragma unroll 8
+            for (int b = 0; b < P.B; ++b)
+                s += dy[(size_t)b * P.dw.lda + i];
+            P.db[i] = s;
+        }
+        return;
+    }
+    tile -= P.dw.tiles();
+    if (OUTER) {
+        const int k = tile * 32 * SM_W + threadIdx.x;
+        if (k < P.H) {
+            float s = 0.0f;
+#pragma unroll 8
+            for (int b = 0; b < P.B; ++b)
+                s += P.dlw[b] * P.h2[(size_t)b * P.H + k];
+            P.gwp[k] = s;
+        }
+        if (k == 0) {
+            float s = 0.0f;
+            for (int b = 0; b < P.B; ++b)
+                s += P.dlw[b];
+            P.gbp[0] = s;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The output head of a training step in one pass over its tiles of 64
+// outputs (B <= 64 rows, rank <= 64).  It is the step's memory traffic: per
+// output 64 weights with their two moments.  Taken apart into products and
+// element-wise kernels it moved O, T, dO and the gradient through HBM about
+// ten times (0.55 ms a step at 75000 outputs); here a tile is
+//   O = Z U^T + bu, dO = 2 (O - T) / (B out), dbu = column sums,
+//   dU = dO^T Z, dZ += dO U
+// on the tensor cores from shared memory, and with ADAM the tile's weights,
+// moments and BF16 copy are updated in the same pass from the gradient in
+// registers, so a step reads T and reads and writes U's state once.
+// GRAD writes the gradient instead.  PREDICT writes O and stops.
+// Each CTA walks tiles grid-stride and keeps its share of dZ in registers;
+// the shares are written to part and added in CTA order by head_fold_kernel.
+// ---------------------------------------------------------------------------
+constexpr int HB = 64, HR = 64, HJ = 64; // rows, rank, outputs of a tile
+constexpr int HP = 72;                   // pitch of the staged operands (144 bytes: conflict-free fragments)
+enum HeadMode { HEAD_PREDICT, HEAD_GRAD, HEAD_ADAM };
+
+struct AdamArgs {
+    float lr, b1, b2, c1, c2, eps;
+};
+
+__device__ __forceinline__ float adam_update(float w, float g, float &m, float &v, const AdamArgs &a)
+{
+    m = a.b1 * m + (1.0f - a.b1) * g;
+    v = a.b2 * v + (1.0f - a.b2) * g * g;
+    return w - a.lr * (m / a.c1) / (sqrtf(v / a.c2) + a.eps);
+}
+
+struct HeadTile {
+    int B, rank, out;
+    const float *Z, *T;      // [B x rank], [B x out]
+    float *w, *m, *v, *g;    // U: [out x rank]
+    bf16 *wb;
+    float *bw, *bm, *bv, *bg; // bu: [out]
+    float *O;                // HEAD_PREDICT
+    float scale;             // 1 / (B out)
+    float *part;             // [grid][B x rank] shares of dZ
+    double *loss;            // [grid] sums of (o - t)^2
+    AdamArgs a;
+};
+
+// shared memory: Z and dO as BF16 pairs in both orders, U in both orders
+struct HeadSmem {
+    bf16 z[2][HB][HP], u[HJ][HP]; // all that a prediction stages
+    bf16 zt[2][HR][HP], ut[HR][HP];
+    bf16 d[2][HB][HP], dt[2][HJ][HP];
+    float db[4][HJ];
+    double sq[8];
+};
+
+__device__ __forceinline__ void frag_a(unsigned (&a)[4], const bf16 (*s)[HP], int r, int k, int t)
+{
+    a[0] = *(const unsigned *)&s[r][k + 2 * t];
+    a[1] = *(const unsigned *)&s[r + 8][k + 2 * t];
+    a[2] = *(const unsigned *)&s[r][k + 2 * t + 8];
+    a[3] = *(const unsigned *)&s[r + 8][k + 2 * t + 8];
+}
+
+__device__ __forceinline__ void frag_b(unsigned (&b)[2], const bf16 (*s)[HP], int c, int k, int t)
+{
+    b[0] = *(const unsigned *)&s[c][k + 2 * t];
+    b[1] = *(const unsigned *)&s[c][k + 2 * t + 8];
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(256, 2) head_tile_kernel(HeadTile P)
+{
+    extern __shared__ __align__(16) char smem_raw[];
+    HeadSmem &S = *reinterpret_cast<HeadSmem *>(smem_raw);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int m0 = 16 * (warp & 3), n0 = 32 * (warp >> 2); // this warp's 16 x 32 of every 64 x 64 product
+    for (int e = threadIdx.x; e < HB * HR; e += 256) {
+        const int b = e / HR, r = e % HR;
+        bf16 hi, lo;
+        split_bf16(b < P.B && r < P.rank ? P.Z[b * P.rank + r] : 0.0f, hi, lo);
+        S.z[0][b][r] = hi;
+        S.z[1][b][r] = lo;
+        if (MODE != HEAD_PREDICT) {
+            S.zt[0][r][b] = hi;
+            S.zt[1][r][b] = lo;
+        }
+    }
+    float dz[4][4] = {};
+    double sq = 0.0;
+    const int ntiles = (P.out + HJ - 1) / HJ;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int j0 = tile * HJ;
+        __syncthreads(); // the previous tile's operands are read; Z is staged
+        if (P.rank == HR) { // rows of 64: contiguous over the threads
+#pragma unroll 4
+            for (int e = threadIdx.x; e < HJ * HR; e += 256) {
+                const int j = e / HR, r = e % HR;
+                const bf16 x = j0 + j < P.out ? P.wb[(size_t)(j0 + j) * HR + r] : __float2bfloat16_rn(0.0f);
+                S.u[j][r] = x;
+                if (MODE != HEAD_PREDICT)
+                    S.ut[r][j] = x;
+            }
+        } else {
+            for (int e = threadIdx.x; e < HJ * HR; e += 256) {
+                const int j = e / HR, r = e % HR;
+                const bf16 x = j0 + j < P.out && r < P.rank ? P.wb[(size_t)(j0 + j) * P.rank + r]
+                                                            : __float2bfloat16_rn(0.0f);
+                S.u[j][r] = x;
+                if (MODE != HEAD_PREDICT)
+                    S.ut[r][j] = x;
+            }
+        }
+        // this thread's targets and biases, in flight while U is staged
+        float tv[4][4], bu[4][2];
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int j = j0 + n0 + 8 * nt + 2 * t + q;
+                bu[nt][q] = j < P.out ? P.bw[j] : 0.0f;
+            }
+            if (MODE != HEAD_PREDICT) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int b = m0 + g + 8 * (q >> 1), j = j0 + n0 + 8 * nt + 2 * t + (q & 1);
+                    tv[nt][q] = b < P.B && j < P.out ? P.T[(size_t)b * P.out + j] : 0.0f;
+                }
+            }
+        }
+        __syncthreads();
+        float o[4][4] = {};
+#pragma unroll
+        for (int k = 0; k < HR; k += 16) {
+            unsigned ah[4], al[4], b[2];
+            frag_a(ah, S.z[0], m0 + g, k, t);
+            frag_a(al, S.z[1], m0 + g, k, t);
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                frag_b(b, S.u, n0 + 8 * nt + g, k, t);
+                mma_bf16(o[nt], al, b);
+                mma_bf16(o[nt], ah, b);
+            }
+        }
+        if (MODE == HEAD_PREDICT) {
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int b = m0 + g + 8 * (q >> 1), j = j0 + n0 + 8 * nt + 2 * t + (q & 1);
+                    if (b < P.B && j < P.out)
+                        P.O[(size_t)b * P.out + j] = o[nt][q] + bu[nt][q & 1];
+                }
+            continue;
+        }
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+            float cs[2] = {0.0f, 0.0f};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int b = m0 + g + 8 * (q >> 1), jj = n0 + 8 * nt + 2 * t + (q & 1);
+                float d = 0.0f;
+                if (b < P.B && j0 + jj < P.out) {
+                    const float r = o[nt][q] + bu[nt][q & 1] - tv[nt][q];
+                    d = 2.0f * r * P.scale;
+                    sq += (double)r * (double)r;
+                }
+                cs[q & 1] += d;
+                bf16 hi, lo;
+                split_bf16(d, hi, lo);
+                S.d[0][b][jj] = hi;
+                S.d[1][b][jj] = lo;
+                S.dt[0][jj][b] = hi;
+                S.dt[1][jj][b] = lo;
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q) { // column sums over the warp's 16 rows
+#pragma unroll
+                for (int s = 4; s < 32; s <<= 1)
+                    cs[q] += __shfl_xor_sync(0xffffffffu, cs[q], s);
+                if (g == 0)
+                    S.db[warp & 3][n0 + 8 * nt + 2 * t + q] = cs[q];
+            }
+        }
+        __syncthreads();
+        float du[4][4] = {};
+#pragma unroll
+        for (int k = 0; k < HB; k += 16) {
+            unsigned ah[4], al[4], bh[2], bl[2];
+            frag_a(ah, S.dt[0], m0 + g, k, t);
+            frag_a(al, S.dt[1], m0 + g, k, t);
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) { // dU = dO^T Z
+                frag_b(bh, S.zt[0], n0 + 8 * nt + g, k, t);
+                frag_b(bl, S.zt[1], n0 + 8 * nt + g, k, t);
+                mma_bf16(du[nt], al, bh);
+                mma_bf16(du[nt], ah, bl);
+                mma_bf16(du[nt], ah, bh);
+            }
+            frag_a(ah, S.d[0], m0 + g, k, t);
+            frag_a(al, S.d[1], m0 + g, k, t);
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) { // dZ += dO U
+                frag_b(bh, S.ut, n0 + 8 * nt + g, k, t);
+                mma_bf16(dz[nt], al, bh);
+                mma_bf16(dz[nt], ah, bh);
+            }
+        }
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int j = j0 + m0 + g + 8 * (q >> 1), r = n0 + 8 * nt + 2 * t + (q & 1);
+                if (j < P.out && r < P.rank) {
+                    const size_t e = (size_t)j * P.rank + r;
+                    if (MODE == HEAD_GRAD) {
+                        P.g[e] = du[nt][q];
+                    } else {
+                        float m = P.m[e], v = P.v[e];
+                        const float w = adam_update(P.w[e], du[nt][q], m, v, P.a);
+                        P.m[e] = m;
+                        P.v[e] = v;
+                        P.w[e] = w;
+                        P.wb[e] = __float2bfloat16_rn(w);
+                    }
+                }
+            }
+        if (threadIdx.x < HJ && j0 + (int)threadIdx.x < P.out) {
+            const int j = j0 + threadIdx.x;
+            const float gb = ((S.db[0][threadIdx.x] + S.db[1][threadIdx.x]) + S.db[2][threadIdx.x]) +
+                             S.db[3][threadIdx.x];
+            if (MODE == HEAD_GRAD) {
+                P.bg[j] = gb;
+            } else {
+                float m = P.bm[j], v = P.bv[j];
+                P.bw[j] = adam_update(P.bw[j], gb, m, v, P.a);
+                P.bm[j] = m;
+                P.bv[j] = v;
+            }
+        }
+    }
+    if (MODE == HEAD_PREDICT)
+        return;
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int b = m0 + g + 8 * (q >> 1), r = n0 + 8 * nt + 2 * t + (q & 1);
+            if (b < P.B && r < P.rank)
+                P.part[(size_t)blockIdx.x * P.B * P.rank + b * P.rank + r] = dz[nt][q];
+        }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+        sq += __shfl_xor_sync(0xffffffffu, sq, s);
+    if (lane == 0)
+        S.sq[warp] = sq;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w)
+            sq += S.sq[w];
+        P.loss[blockIdx.x] = sq;
+    }
+}
+
+// dZ = the CTAs' shares in CTA order (8 runs of CTAs, then the runs); the
+// last block adds the loss
+__global__ void __launch_bounds__(256) head_fold_kernel(int n, int shares, const float *part, float *dZ,
+                                                        const double *loss, double tot, const double *hloss,
+                                                        double *acc)
+{
+    if (blockIdx.x == gridDim.x - 1) {
+        __shared__ double sh[256];
+        double a = 0.0;
+        for (int b = threadIdx.x; b < shares; b += 256)
+            a += loss[b];
+        sh[threadIdx.x] = a;
+        __syncthreads();
+        for (int w = 128; w > 0; w >>= 1) {
+            if ((int)threadIdx.x < w)
+                sh[threadIdx.x] += sh[threadIdx.x + w];
+            __syncthreads();
+        }
+        if (threadIdx.x == 0)
+            acc[0] += sh[0] / tot + hloss[0];
+        return;
+    }
+    __shared__ float run[8][32];
+    const int e = blockIdx.x * 32 + (threadIdx.x & 31), k = threadIdx.x >> 5;
+    float s = 0.0f;
+    if (e < n) {
+        const int z1 = shares * (k + 1) / 8;
+#pragma unroll 8
+        for (int z = shares * k / 8; z < z1; ++z)
+            s += part[(size_t)z * n + e];
+    }
+    run[k][threadIdx.x & 31] = s;
+    __syncthreads();
+    if (k == 0 && e < n) {
+        for (int q = 1; q < 8; ++q)
+            s += run[q][threadIdx.x];
+        dZ[e] = s;
+    }
+}
+
+// Adam and the BF16 copy for the parameters outside [skip0, skip1) (the
+// output head's, updated in head_tile_kernel)
+__global__ void adam_outer_kernel(long long n, long long skip0, long long skip1, float *w, const float *g, float *mom,
+                                  float *vel, bf16 *wb, AdamArgs a)
+{
+    const long long cnt = n - (skip1 - skip0);
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < cnt;
+         i += (long long)gridDim.x * blockDim.x) {
+        const long long e = i < skip0 ? i : i + (skip1 - skip0);
+        float m = mom[e], v = vel[e];
+        const float x = adam_update(w[e], g[e], m, v, a);
+        mom[e] = m;
+        vel[e] = v;
+        w[e] = x;
+        wb[e] = __float2bfloat16_rn(x);
+    }
+}
 
 } // namespace
 
@@ -418,15 +956,49 @@ int ensure_acts(pdhcg_b200_mlp_s *n, int B)
     return 0;
 }
 
-// forward of B rows already in n->X; with targets (T, TL) also the loss and dO, dLW
-int forward(pdhcg_b200_mlp_s *n, int B, bool with_loss)
+// The minibatch kernels take up to SMALL_B rows (a 64-row step of the
+// default network: 0.55 ms with the tiled products and element-wise passes
+// below); larger batches keep the tiled products, whose operands are staged
+// once per 64 x 64 tile.
+bool small_trunk(int B) { return B <= SMALL_B; }
+// one 64 x 64 tile of Z in a CTA's shared memory
+bool fused_head(const pdhcg_b200_mlp_s *n, int B) { return B <= HB && n->rank <= HR; }
+
+SmallGemm layer(int B, int N, int K, const float *X, const bf16 *W, const float *b, float *Y)
+{
+    SmallGemm G{};
+    G.M = B;
+    G.N = N;
+    G.K = K;
+    G.A = X;
+    G.lda = K;
+    G.B = W;
+    G.ldb = K;
+    G.C = Y;
+    G.bias = b;
+    return G;
+}
+
+// hidden layers, low-rank layer and log-weight head of B rows X; with TL
+// also the head's loss and dLW
+int trunk_forward(pdhcg_b200_mlp_s *n, int B, const float *X, const float *TL)
 {
     cudaStream_t s = n->s;
-    const bf16 *W1 = n->wb + n->off[P_W1], *W2 = n->wb + n->off[P_W2], *W3 = n->wb + n->off[P_W3],
-               *U = n->wb + n->off[P_U];
+    const bf16 *W1 = n->wb + n->off[P_W1], *W2 = n->wb + n->off[P_W2], *W3 = n->wb + n->off[P_W3];
     const float *b1 = n->w + n->off[P_B1], *b2 = n->w + n->off[P_B2], *b3 = n->w + n->off[P_B3],
-                *bu = n->w + n->off[P_BU], *wp = n->w + n->off[P_WP], *bp = n->w + n->off[P_BP];
-    if (gemm<false, true>(B, n->hid, n->in, n->X, n->in, W1, n->in, n->H1, n->hid, 1.0f, 0.0f, s, n->ws))
+                *wp = n->w + n->off[P_WP], *bp = n->w + n->off[P_BP];
+    if (small_trunk(B)) {
+        const HeadArgs h{B, n->hid, n->H2, wp, bp, TL, n->LW, n->dLW, n->hloss};
+        const SmallGemm g1 = layer(B, n->hid, n->in, X, W1, b1, n->H1),
+                        g2 = layer(B, n->hid, n->hid, n->H1, W2, b2, n->H2),
+                        g3 = layer(B, n->rank, n->hid, n->H2, W3, b3, n->Z);
+        small_layer_kernel<EPI_BIAS_RELU, false><<<g1.tiles(), 32 * SM_W, 0, s>>>(g1, h);
+        small_layer_kernel<EPI_BIAS_RELU, false><<<g2.tiles(), 32 * SM_W, 0, s>>>(g2, h);
+        small_layer_kernel<EPI_BIAS, true><<<g3.tiles() + 1, 32 * SM_W, 0, s>>>(g3, h);
+        MCK(cudaGetLastError());
+        return 0;
+    }
+    if (gemm<false, true>(B, n->hid, n->in, X, n->in, W1, n->in, n->H1, n->hid, 1.0f, 0.0f, s, n->ws))
         return -1;
     bias_act_kernel<<<blocks_for((long long)B * n->hid), 256, 0, s>>>(B, n->hid, n->H1, b1, 1);
     if (gemm<false, true>(B, n->hid, n->hid, n->H1, n->hid, W2, n->hid, n->H2, n->hid, 1.0f, 0.0f, s, n->ws))
@@ -435,54 +1007,165 @@ int forward(pdhcg_b200_mlp_s *n, int B, bool with_loss)
     if (gemm<false, true>(B, n->rank, n->hid, n->H2, n->hid, W3, n->hid, n->Z, n->rank, 1.0f, 0.0f, s, n->ws))
         return -1;
     bias_act_kernel<<<blocks_for((long long)B * n->rank), 256, 0, s>>>(B, n->rank, n->Z, b3, 0);
-    if (gemm<false, true>(B, n->out, n->rank, n->Z, n->rank, U, n->rank, n->O, n->out, 1.0f, 0.0f, s, n->ws))
-        return -1;
-    bias_act_kernel<<<blocks_for((long long)B * n->out), 256, 0, s>>>(B, n->out, n->O, bu, 0);
-    head_kernel<<<1, 256, 0, s>>>(B, n->hid, n->H2, wp, bp, with_loss ? n->TL : nullptr, n->LW, n->dLW, n->hloss);
-    if (with_loss) { // the minibatch's loss is added to n->acc on the device (no host wait)
-        long long tot = (long long)B * n->out;
-        int nb = blocks_for(tot);
-        mse_kernel<<<nb, 256, 0, s>>>(tot, n->O, n->T, 1.0f / (float)tot, n->dO, n->part);
-        loss_fold_kernel<<<1, 256, 0, s>>>(n->part, nb, (double)tot, n->hloss, n->acc);
+    head_kernel<<<1, 256, 0, s>>>(B, n->hid, n->H2, wp, bp, TL, n->LW, n->dLW, n->hloss);
+    MCK(cudaGetLastError());
+    return 0;
+}
+
+HeadTile head_tile(const pdhcg_b200_mlp_s *n, int B, const float *T)
+{
+    HeadTile P{};
+    P.B = B;
+    P.rank = n->rank;
+    P.out = n->out;
+    P.Z = n->Z;
+    P.T = T;
+    P.w = n->w + n->off[P_U];
+    P.m = n->mom + n->off[P_U];
+    P.v = n->vel + n->off[P_U];
+    P.g = n->g + n->off[P_U];
+    P.wb = n->wb + n->off[P_U];
+    P.bw = n->w + n->off[P_BU];
+    P.bm = n->mom + n->off[P_BU];
+    P.bv = n->vel + n->off[P_BU];
+    P.bg = n->g + n->off[P_BU];
+    P.O = n->O;
+    P.scale = 1.0f / (float)((long long)B * n->out);
+    P.loss = n->part;
+    return P;
+}
+
+int head_grid(const pdhcg_b200_mlp_s *n) { return std::min((n->out + HJ - 1) / HJ, 2 * 148); }
+constexpr size_t HEAD_SMEM_PREDICT = offsetof(HeadSmem, zt), HEAD_SMEM = sizeof(HeadSmem);
+
+// o of the rows that trunk_forward took, into n->O
+int head_forward(pdhcg_b200_mlp_s *n, int B)
+{
+    cudaStream_t s = n->s;
+    if (fused_head(n, B)) {
+        const int grid = std::min((n->out + HJ - 1) / HJ, 8 * 148);
+        head_tile_kernel<HEAD_PREDICT><<<grid, 256, HEAD_SMEM_PREDICT, s>>>(head_tile(n, B, nullptr));
+    } else {
+        if (gemm<false, true>(B, n->out, n->rank, n->Z, n->rank, n->wb + n->off[P_U], n->rank, n->O, n->out, 1.0f, 0.0f,
+                              s, n->ws))
+            return -1;
+        bias_act_kernel<<<blocks_for((long long)B * n->out), 256, 0, s>>>(B, n->out, n->O, n->w + n->off[P_BU], 0);
     }
     MCK(cudaGetLastError());
     return 0;
 }
 
-// gradient of the loss of the last forward (with targets) into n->g
-int backward(pdhcg_b200_mlp_s *n, int B)
+// Forward and backward of one minibatch: the loss is added to n->acc on the
+// device (no host wait); the gradient goes to n->g, except that with adam
+// the parameters are updated (the fused output head's from registers, the
+// others after the whole gradient is there).
+int step(pdhcg_b200_mlp_s *n, int B, const float *X, const float *T, const float *TL, const AdamArgs *adam)
 {
     cudaStream_t s = n->s;
+    if (trunk_forward(n, B, X, TL))
+        return -1;
     const bf16 *W2 = n->wb + n->off[P_W2], *W3 = n->wb + n->off[P_W3], *U = n->wb + n->off[P_U];
     const float *wp = n->w + n->off[P_WP];
     float *g = n->g;
-    // output head: dU = dO^T Z, dbu = colsum dO, dZ = dO U
-    if (gemm<true, false>(n->out, n->rank, B, n->dO, n->out, n->Z, n->rank, g + n->off[P_U], n->rank, 1.0f, 0.0f, s, n->ws))
-        return -1;
-    colsum_kernel<<<blocks_for(n->out), 256, 0, s>>>(B, n->out, n->dO, g + n->off[P_BU]);
-    if (gemm<false, false>(B, n->rank, n->out, n->dO, n->out, U, n->rank, n->dZ, n->rank, 1.0f, 0.0f, s, n->ws))
-        return -1;
-    // z = W3 h2 + b3
-    if (gemm<true, false>(n->rank, n->hid, B, n->dZ, n->rank, n->H2, n->hid, g + n->off[P_W3], n->hid, 1.0f, 0.0f, s, n->ws))
-        return -1;
-    colsum_kernel<<<blocks_for(n->rank), 256, 0, s>>>(B, n->rank, n->dZ, g + n->off[P_B3]);
-    if (gemm<false, false>(B, n->hid, n->rank, n->dZ, n->rank, W3, n->hid, n->dH2, n->hid, 1.0f, 0.0f, s, n->ws))
-        return -1;
-    // log-weight head
-    head_back_kernel<<<blocks_for(n->hid), 256, 0, s>>>(B, n->hid, n->H2, wp, n->dLW, n->dH2, g + n->off[P_WP],
-                                                         g + n->off[P_BP]);
-    relu_back_kernel<<<blocks_for((long long)B * n->hid), 256, 0, s>>>((long long)B * n->hid, n->dH2, n->H2);
-    // h2 = relu(W2 h1 + b2)
-    if (gemm<true, false>(n->hid, n->hid, B, n->dH2, n->hid, n->H1, n->hid, g + n->off[P_W2], n->hid, 1.0f, 0.0f, s, n->ws))
-        return -1;
-    colsum_kernel<<<blocks_for(n->hid), 256, 0, s>>>(B, n->hid, n->dH2, g + n->off[P_B2]);
-    if (gemm<false, false>(B, n->hid, n->hid, n->dH2, n->hid, W2, n->hid, n->dH1, n->hid, 1.0f, 0.0f, s, n->ws))
-        return -1;
-    relu_back_kernel<<<blocks_for((long long)B * n->hid), 256, 0, s>>>((long long)B * n->hid, n->dH1, n->H1);
-    // h1 = relu(W1 x + b1)
-    if (gemm<true, false>(n->hid, n->in, B, n->dH1, n->hid, n->X, n->in, g + n->off[P_W1], n->in, 1.0f, 0.0f, s, n->ws))
-        return -1;
-    colsum_kernel<<<blocks_for(n->hid), 256, 0, s>>>(B, n->hid, n->dH1, g + n->off[P_B1]);
+    const long long tot = (long long)B * n->out;
+    const bool fused = fused_head(n, B);
+    if (fused) {
+        const int grid = head_grid(n);
+        const size_t need = (size_t)grid * B * n->rank;
+        if (grow_ws(n->ws, need))
+            return -1;
+        HeadTile P = head_tile(n, B, T);
+        P.part = n->ws.p;
+        if (adam) {
+            P.a = *adam;
+            head_tile_kernel<HEAD_ADAM><<<grid, 256, HEAD_SMEM, s>>>(P);
+        } else {
+            head_tile_kernel<HEAD_GRAD><<<grid, 256, HEAD_SMEM, s>>>(P);
+        }
+        head_fold_kernel<<<(B * n->rank + 31) / 32 + 1, 256, 0, s>>>(B * n->rank, grid, n->ws.p, n->dZ, n->part,
+                                                                    (double)tot, n->hloss, n->acc);
+    } else {
+        if (head_forward(n, B))
+            return -1;
+        int nb = blocks_for(tot);
+        mse_kernel<<<nb, 256, 0, s>>>(tot, n->O, T, 1.0f / (float)tot, n->dO, n->part);
+        loss_fold_kernel<<<1, 256, 0, s>>>(n->part, nb, (double)tot, n->hloss, n->acc);
+        // dU = dO^T Z, dbu = colsum dO, dZ = dO U
+        if (gemm<true, false>(n->out, n->rank, B, n->dO, n->out, n->Z, n->rank, g + n->off[P_U], n->rank, 1.0f, 0.0f, s,
+                              n->ws))
+            return -1;
+        colsum_kernel<<<blocks_for(n->out), 256, 0, s>>>(B, n->out, n->dO, g + n->off[P_BU]);
+        if (gemm<false, false>(B, n->rank, n->out, n->dO, n->out, U, n->rank, n->dZ, n->rank, 1.0f, 0.0f, s, n->ws))
+            return -1;
+    }
+    if (small_trunk(B)) {
+        BackArgs b3{}, b2{}, b1{};
+        auto back = [&](BackArgs &b, int out, int in, const float *dY, const bf16 *W, const float *Xin, float *dX,
+                        const float *mask, int pw, int pb) {
+            b.dx.M = B;
+            b.dx.N = in;
+            b.dx.K = out;
+            b.dx.A = dY;
+            b.dx.lda = out;
+            b.dx.B = W;
+            b.dx.ldb = in;
+            b.dx.C = dX;
+            b.dx.mask = mask;
+            b.dw.M = out;
+            b.dw.N = in;
+            b.dw.K = B;
+            b.dw.A = dY;
+            b.dw.lda = out;
+            b.dw.B = Xin;
+            b.dw.ldb = in;
+            b.dw.C = g + n->off[pw];
+            b.db = g + n->off[pb];
+            b.B = B;
+            b.H = n->hid;
+        };
+        back(b3, n->rank, n->hid, n->dZ, W3, n->H2, n->dH2, n->H2, P_W3, P_B3);
+        b3.dx.col = n->dLW;
+        b3.dx.row = wp;
+        b3.dlw = n->dLW;
+        b3.h2 = n->H2;
+        b3.gwp = g + n->off[P_WP];
+        b3.gbp = g + n->off[P_BP];
+        back(b2, n->hid, n->hid, n->dH2, W2, n->H1, n->dH1, n->H1, P_W2, P_B2);
+        back(b1, n->hid, n->in, n->dH1, nullptr, X, nullptr, nullptr, P_W1, P_B1);
+        const int hb = (n->hid + 32 * SM_W - 1) / (32 * SM_W);
+        small_back_kernel<true, true><<<b3.dx.tiles() + b3.dw.tiles() + hb, 32 * SM_W, 0, s>>>(b3);
+        small_back_kernel<false, true><<<b2.dx.tiles() + b2.dw.tiles(), 32 * SM_W, 0, s>>>(b2);
+        small_back_kernel<false, false><<<b1.dw.tiles(), 32 * SM_W, 0, s>>>(b1);
+    } else {
+        // z = W3 h2 + b3
+        if (gemm<true, false>(n->rank, n->hid, B, n->dZ, n->rank, n->H2, n->hid, g + n->off[P_W3], n->hid, 1.0f, 0.0f, s,
+                              n->ws))
+            return -1;
+        colsum_kernel<<<blocks_for(n->rank), 256, 0, s>>>(B, n->rank, n->dZ, g + n->off[P_B3]);
+        if (gemm<false, false>(B, n->hid, n->rank, n->dZ, n->rank, W3, n->hid, n->dH2, n->hid, 1.0f, 0.0f, s, n->ws))
+            return -1;
+        // log-weight head
+        head_back_kernel<<<blocks_for(n->hid), 256, 0, s>>>(B, n->hid, n->H2, wp, n->dLW, n->dH2, g + n->off[P_WP],
+                                                             g + n->off[P_BP]);
+        relu_back_kernel<<<blocks_for((long long)B * n->hid), 256, 0, s>>>((long long)B * n->hid, n->dH2, n->H2);
+        // h2 = relu(W2 h1 + b2)
+        if (gemm<true, false>(n->hid, n->hid, B, n->dH2, n->hid, n->H1, n->hid, g + n->off[P_W2], n->hid, 1.0f, 0.0f, s,
+                              n->ws))
+            return -1;
+        colsum_kernel<<<blocks_for(n->hid), 256, 0, s>>>(B, n->hid, n->dH2, g + n->off[P_B2]);
+        if (gemm<false, false>(B, n->hid, n->hid, n->dH2, n->hid, W2, n->hid, n->dH1, n->hid, 1.0f, 0.0f, s, n->ws))
+            return -1;
+        relu_back_kernel<<<blocks_for((long long)B * n->hid), 256, 0, s>>>((long long)B * n->hid, n->dH1, n->H1);
+        // h1 = relu(W1 x + b1)
+        if (gemm<true, false>(n->hid, n->in, B, n->dH1, n->hid, X, n->in, g + n->off[P_W1], n->in, 1.0f, 0.0f, s, n->ws))
+            return -1;
+        colsum_kernel<<<blocks_for(n->hid), 256, 0, s>>>(B, n->hid, n->dH1, g + n->off[P_B1]);
+    }
+    if (adam) {
+        const long long skip0 = fused ? n->off[P_U] : n->total, skip1 = fused ? n->off[P_WP] : n->total;
+        adam_outer_kernel<<<blocks_for(n->total - (skip1 - skip0)), 256, 0, s>>>(n->total, skip0, skip1, n->w, n->g,
+                                                                                n->mom, n->vel, n->wb, *adam);
+    }
     MCK(cudaGetLastError());
     return 0;
 }
@@ -549,7 +1232,12 @@ pdhcg_b200_mlp_t *pdhcg_b200_mlp_create(int in_dim, int hidden, int rank, int ou
         cudaMalloc((void **)&n->wb, o * sizeof(bf16)) != cudaSuccess ||
         cudaMemcpy(n->w, h.data(), o * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(n->mom, 0, o * sizeof(float)) != cudaSuccess ||
-        cudaMemset(n->vel, 0, o * sizeof(float)) != cudaSuccess || refresh_bf16(n) != 0) {
+        cudaMemset(n->vel, 0, o * sizeof(float)) != cudaSuccess ||
+        cudaFuncSetAttribute(head_tile_kernel<HEAD_GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)HEAD_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(head_tile_kernel<HEAD_ADAM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)HEAD_SMEM) != cudaSuccess ||
+        refresh_bf16(n) != 0) {
         std::fprintf(stderr, "[pdhcg_b200_mlp_create] device allocation failed.\n");
         pdhcg_b200_mlp_free(n);
         return nullptr;
@@ -600,7 +1288,7 @@ int pdhcg_b200_mlp_predict(pdhcg_b200_mlp_t *n, int batch, const float *theta, f
     if (ensure_acts(n, batch))
         return -1;
     MCK(cudaMemcpyAsync(n->X, theta, (size_t)batch * n->in * sizeof(float), cudaMemcpyHostToDevice, n->s));
-    if (forward(n, batch, false))
+    if (trunk_forward(n, batch, n->X, nullptr) || head_forward(n, batch))
         return -1;
     MCK(cudaMemcpyAsync(out, n->O, (size_t)batch * n->out * sizeof(float), cudaMemcpyDeviceToHost, n->s));
     if (logw)
@@ -620,7 +1308,7 @@ int pdhcg_b200_mlp_loss_grad(pdhcg_b200_mlp_t *n, int batch, const float *theta,
     MCK(cudaMemcpyAsync(n->T, target, (size_t)batch * n->out * sizeof(float), cudaMemcpyHostToDevice, n->s));
     MCK(cudaMemcpyAsync(n->TL, target_logw, batch * sizeof(float), cudaMemcpyHostToDevice, n->s));
     MCK(cudaMemsetAsync(n->acc, 0, sizeof(double), n->s));
-    if (forward(n, batch, true) || backward(n, batch))
+    if (step(n, batch, n->X, n->T, n->TL, nullptr))
         return -1;
     if (grad)
         MCK(cudaMemcpyAsync(grad, n->g, n->total * sizeof(float), cudaMemcpyDeviceToHost, n->s));
@@ -653,21 +1341,10 @@ int pdhcg_b200_mlp_train(pdhcg_b200_mlp_t *n, int count, const float *theta, con
             rc = -1;
         nbat = 0;
         for (int b0 = 0; b0 + batch <= count && rc == 0; b0 += batch, ++nbat) { // full minibatches in order
-            cudaMemcpyAsync(n->X, dth + (size_t)b0 * n->in, (size_t)batch * n->in * sizeof(float),
-                            cudaMemcpyDeviceToDevice, n->s);
-            cudaMemcpyAsync(n->T, dt + (size_t)b0 * n->out, (size_t)batch * n->out * sizeof(float),
-                            cudaMemcpyDeviceToDevice, n->s);
-            cudaMemcpyAsync(n->TL, dtl + b0, batch * sizeof(float), cudaMemcpyDeviceToDevice, n->s);
-            rc = forward(n, batch, true);
-            if (rc == 0)
-                rc = backward(n, batch);
-            if (rc == 0) {
-                ++n->step;
-                float c1 = 1.0f - std::pow(b1, (float)n->step), c2 = 1.0f - std::pow(b2, (float)n->step);
-                adam_kernel<<<blocks_for(n->total), 256, 0, n->s>>>(n->total, n->w, n->g, n->mom, n->vel, lr, b1, b2,
-                                                                    c1, c2, eps);
-                rc = refresh_bf16(n);
-            }
+            ++n->step;
+            const AdamArgs adam{lr, b1, b2, 1.0f - std::pow(b1, (float)n->step), 1.0f - std::pow(b2, (float)n->step),
+                                eps};
+            rc = step(n, batch, dth + (size_t)b0 * n->in, dt + (size_t)b0 * n->out, dtl + b0, &adam);
         }
     }
     double acc = 0.0;
