@@ -281,7 +281,7 @@ __global__ void mse_kernel(long long n, const float *o, const float *t, float sc
 }
 
 // acc += (sum of the nb block partials, in order) / tot + the head's loss
-__global__ void loss_fold_kernel(const double *part, int nb, double tot, const double *hloss, double *acc)
+__global__ void loss_fold_kernel(const double *part, int nb, double tot, const double *hloss, int nhloss, double *acc)
 {
     __shared__ double sh[256];
     double a = 0.0;
@@ -294,8 +294,12 @@ __global__ void loss_fold_kernel(const double *part, int nb, double tot, const d
             sh[threadIdx.x] += sh[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0)
-        acc[0] += sh[0] / tot + hloss[0];
+    if (threadIdx.x == 0) {
+        double v = sh[0] / tot;
+        for (int b = 0; b < nhloss; ++b)
+            v += hloss[b];
+        acc[0] += v;
+    }
 }
 
 // log-weight head: lw[b] = wp . h2[b] + bp; dlw = 2 (lw - tl) / B; loss partial
@@ -361,8 +365,10 @@ int blocks_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 1
 // straight from L2 (no staging: each element is used by one warp) with every
 // load of a warp in flight at once; the 8 partial tiles are added in warp
 // order in shared memory and the epilogue (bias, ReLU, the ReLU mask of the
-// backward pass, the log-weight head's outer product) runs on the sum.  Same
-// arithmetic as mma_gemm_kernel: BF16 pairs for FP32 operands, FP32 sums.
+// backward pass, the log-weight head's outer product) runs on the sum.  FP32
+// sums; an FP32 operand enters a product with BF16 weights as three BF16
+// parts (exact; the third product costs nothing here), one with another FP32
+// operand as a pair, as in mma_gemm_kernel.
 // ---------------------------------------------------------------------------
 constexpr int SMALL_B = 128;           // rows up to which the minibatch kernels are used
 constexpr int SM_M = 32, SM_N = 16;    // tile
@@ -378,6 +384,7 @@ struct SmallGemm {
     const float *bias;        // EPI_BIAS*: [N]
     const float *mask;        // EPI_MASK*: C is kept where mask > 0, 0 elsewhere ([M x N])
     const float *col, *row;   // EPI_MASK_OUTER: + col[i] * row[j] before the mask
+    int vec;                  // word loads of pairs along K (see small_gemm_tile)
     __host__ __device__ int tiles() const { return ((M + SM_M - 1) / SM_M) * ((N + SM_N - 1) / SM_N); }
 };
 
@@ -389,6 +396,15 @@ __device__ __forceinline__ void split2(float v0, float v1, unsigned &hi, unsigne
     const __nv_bfloat162 l = __floats2bfloat162_rn(v0 - hf.x, v1 - hf.y);
     hi = *reinterpret_cast<const unsigned *>(&h);
     lo = *reinterpret_cast<const unsigned *>(&l);
+}
+
+// (v0, v1) as three BF16 pairs: all 24 bits of an FP32 value
+__device__ __forceinline__ void split3(float v0, float v1, unsigned &hi, unsigned &mid, unsigned &lo)
+{
+    const __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
+    const float2 hf = __bfloat1622float2(h);
+    hi = *reinterpret_cast<const unsigned *>(&h);
+    split2(v0 - hf.x, v1 - hf.y, mid, lo);
 }
 
 // elements (i, k) and (i, k + 1) of a matrix stored [i][k] (KFAST) or [k][i]
@@ -405,7 +421,20 @@ __device__ __forceinline__ float2 pair_at(const T *p, int ld, int i, int k, int 
     return v;
 }
 
-template <bool TA, bool TB, typename AT, typename BT, int EPI>
+// the same as a BF16 pair (hi) of a BF16 matrix, VEC: one 4-byte load
+template <bool KFAST, bool VEC>
+__device__ __forceinline__ unsigned bf16_pair_at(const bf16 *p, int ld, int i, int k, int I, int K)
+{
+    if (VEC && KFAST)
+        return i < I && k < K ? *reinterpret_cast<const unsigned *>(p + (size_t)i * ld + k) : 0u;
+    const float2 v = pair_at<KFAST>(p, ld, i, k, I, K);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
+    return *reinterpret_cast<const unsigned *>(&h);
+}
+
+// VEC: pairs along K that are contiguous are loaded as one word (even K and
+// leading dimension, 8-byte aligned FP32, 4-byte aligned BF16)
+template <bool TA, bool TB, bool VEC, typename AT, typename BT, int EPI>
 __device__ __forceinline__ void small_gemm_tile(const SmallGemm &G, int tile, float (*red)[SM_M * SM_N])
 {
     constexpr bool SA = !std::is_same<AT, bf16>::value, SB = !std::is_same<BT, bf16>::value;
@@ -420,27 +449,43 @@ __device__ __forceinline__ void small_gemm_tile(const SmallGemm &G, int tile, fl
 #pragma unroll 4
     for (int st = s0; st < s1; ++st) {
         const int k0 = 16 * st + 2 * t;
-        unsigned a[2][2][4], b[2][2][2];
+        unsigned a[3][2][4], b[2][2][2];
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const float2 v = pair_at<!TA>(A, G.lda, i0 + 16 * mt + g + 8 * (q & 1), k0 + 8 * (q >> 1), G.M, G.K);
-                split2(v.x, v.y, a[0][mt][q], a[1][mt][q]);
+                const int i = i0 + 16 * mt + g + 8 * (q & 1), k = k0 + 8 * (q >> 1);
+                float2 v = make_float2(0.0f, 0.0f);
+                if (VEC && !TA) {
+                    if (i < G.M && k < G.K)
+                        v = *reinterpret_cast<const float2 *>(A + (size_t)i * G.lda + k);
+                } else {
+                    v = pair_at<!TA>(A, G.lda, i, k, G.M, G.K);
+                }
+                if (SB)
+                    split2(v.x, v.y, a[0][mt][q], a[1][mt][q]);
+                else
+                    split3(v.x, v.y, a[0][mt][q], a[1][mt][q], a[2][mt][q]);
             }
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
-                const float2 v = pair_at<TB>(B, G.ldb, j0 + 8 * nt + g, k0 + 8 * q, G.N, G.K);
-                split2(v.x, v.y, b[0][nt][q], b[1][nt][q]);
+                if constexpr (SB) {
+                    const float2 v = pair_at<TB>(B, G.ldb, j0 + 8 * nt + g, k0 + 8 * q, G.N, G.K);
+                    split2(v.x, v.y, b[0][nt][q], b[1][nt][q]);
+                } else {
+                    b[0][nt][q] = bf16_pair_at<TB, VEC>(B, G.ldb, j0 + 8 * nt + g, k0 + 8 * q, G.N, G.K);
+                }
             }
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
-                if (SA)
-                    mma_bf16(acc[mt][nt], a[1][mt], b[0][nt]);
+                static_assert(SA, "the left operand is FP32");
+                if (!SB)
+                    mma_bf16(acc[mt][nt], a[2][mt], b[0][nt]);
+                mma_bf16(acc[mt][nt], a[1][mt], b[0][nt]);
                 if (SB)
                     mma_bf16(acc[mt][nt], a[0][mt], b[1][nt]);
                 mma_bf16(acc[mt][nt], a[0][mt], b[0][nt]);
@@ -475,25 +520,27 @@ __device__ __forceinline__ void small_gemm_tile(const SmallGemm &G, int tile, fl
 }
 
 // One layer of the forward pass.  LAST: the low-rank layer's launch carries
-// one more block, the log-weight head: a warp per row of h2, lanes over the
-// hidden units (one thread per row took 512 dependent loads).
+// the log-weight head in SM_W rows per further block: a warp per row of h2,
+// lanes over the hidden units (one thread per row took 512 dependent loads).
 struct HeadArgs {
     int B, H;
     const float *h2, *wp, *bp, *tl; // tl NULL: prediction only
     float *lw, *dlw;
-    double *loss;
+    double *loss; // per block of SM_W rows
 };
 
 template <int EPI, bool LAST>
 __global__ void __launch_bounds__(32 * SM_W) small_layer_kernel(SmallGemm G, HeadArgs h)
 {
     __shared__ float red[SM_W][SM_M * SM_N];
-    if (LAST && (int)blockIdx.x == G.tiles()) {
+    if (LAST && (int)blockIdx.x >= G.tiles()) {
         __shared__ double sq[SM_W];
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int blk = (int)blockIdx.x - G.tiles(), b = blk * SM_W + warp;
         double a = 0.0;
-        for (int b = warp; b < h.B; b += SM_W) {
+        if (b < h.B) {
             float s = 0.0f;
+#pragma unroll 8
             for (int k = lane; k < h.H; k += 32)
                 s += h.wp[k] * h.h2[(size_t)b * h.H + k];
 #pragma unroll
@@ -505,7 +552,7 @@ __global__ void __launch_bounds__(32 * SM_W) small_layer_kernel(SmallGemm G, Hea
                 if (h.tl) {
                     const float r = s - h.tl[b];
                     h.dlw[b] = 2.0f * r / (float)h.B;
-                    a += (double)r * (double)r;
+                    a = (double)r * (double)r;
                 }
             }
         }
@@ -515,11 +562,14 @@ __global__ void __launch_bounds__(32 * SM_W) small_layer_kernel(SmallGemm G, Hea
         if (threadIdx.x == 0) {
             for (int w = 1; w < SM_W; ++w)
                 a += sq[w];
-            h.loss[0] = a / (double)h.B;
+            h.loss[blk] = a / (double)h.B;
         }
         return;
     }
-    small_gemm_tile<false, true, float, bf16, EPI>(G, blockIdx.x, red);
+    if (G.vec)
+        small_gemm_tile<false, true, true, float, bf16, EPI>(G, blockIdx.x, red);
+    else
+        small_gemm_tile<false, true, false, float, bf16, EPI>(G, blockIdx.x, red);
 }
 
 // One layer of the backward pass: the tiles of dX = dY W (masked by the ReLU
@@ -541,13 +591,17 @@ __global__ void __launch_bounds__(32 * SM_W) small_back_kernel(BackArgs P)
     int tile = blockIdx.x;
     if (DX) {
         if (tile < P.dx.tiles()) {
-            small_gemm_tile<false, false, float, bf16, OUTER ? EPI_MASK_OUTER : EPI_MASK>(P.dx, tile, red);
+            constexpr int EPI = OUTER ? EPI_MASK_OUTER : EPI_MASK;
+            if (P.dx.vec)
+                small_gemm_tile<false, false, true, float, bf16, EPI>(P.dx, tile, red);
+            else
+                small_gemm_tile<false, false, false, float, bf16, EPI>(P.dx, tile, red);
             return;
         }
         tile -= P.dx.tiles();
     }
     if (tile < P.dw.tiles()) {
-        small_gemm_tile<true, false, float, float, EPI_PLAIN>(P.dw, tile, red);
+        small_gemm_tile<true, false, false, float, float, EPI_PLAIN>(P.dw, tile, red);
         const int nt_n = (P.dw.N + SM_N - 1) / SM_N;
         const int i = (tile / nt_n) * SM_M + (int)threadIdx.x;
         if (tile % nt_n == 0 && threadIdx.x < SM_M && i < P.dw.M) { // rows summed in order
@@ -591,11 +645,15 @@ __global__ void __launch_bounds__(32 * SM_W) small_back_kernel(BackArgs P)
 // moments and BF16 copy are updated in the same pass from the gradient in
 // registers, so a step reads T and reads and writes U's state once.
 // GRAD writes the gradient instead.  PREDICT writes O and stops.
+// Every operand is staged once and read by ldmatrix, transposed where a
+// product needs it, and U's state moves as pairs: 53 us at 75000 outputs (97
+// with transposed copies stored 2 bytes at a time and scalar accesses of the
+// state; its 125 MB take 19 us at HBM's rate).
 // Each CTA walks tiles grid-stride and keeps its share of dZ in registers;
 // the shares are written to part and added in CTA order by head_fold_kernel.
 // ---------------------------------------------------------------------------
 constexpr int HB = 64, HR = 64, HJ = 64; // rows, rank, outputs of a tile
-constexpr int HP = 72;                   // pitch of the staged operands (144 bytes: conflict-free fragments)
+constexpr int HP = 72;                   // pitch of the staged operands (144 bytes: conflict-free ldmatrix rows)
 enum HeadMode { HEAD_PREDICT, HEAD_GRAD, HEAD_ADAM };
 
 struct AdamArgs {
@@ -622,30 +680,61 @@ struct HeadTile {
     AdamArgs a;
 };
 
-// shared memory: Z and dO as BF16 pairs in both orders, U in both orders
+// shared memory: Z as three BF16 parts, U, and dO as a BF16 pair, each once,
+// row-major; the products read them as they are or transposed by ldmatrix
 struct HeadSmem {
-    bf16 z[2][HB][HP], u[HJ][HP]; // all that a prediction stages
-    bf16 zt[2][HR][HP], ut[HR][HP];
-    bf16 d[2][HB][HP], dt[2][HJ][HP];
+    bf16 z[3][HB][HP], u[HJ][HP]; // all that a prediction stages
+    bf16 d[2][HB][HP];
     float db[4][HJ];
     double sq[8];
 };
 
-__device__ __forceinline__ void frag_a(unsigned (&a)[4], const bf16 (*s)[HP], int r, int k, int t)
+// four 8 x 8 matrices; lane l passes the address of row l & 7 of matrix l >> 3
+template <bool TRANS>
+__device__ __forceinline__ void ldsm4(unsigned (&r)[4], const bf16 *p)
 {
-    a[0] = *(const unsigned *)&s[r][k + 2 * t];
-    a[1] = *(const unsigned *)&s[r + 8][k + 2 * t];
-    a[2] = *(const unsigned *)&s[r][k + 2 * t + 8];
-    a[3] = *(const unsigned *)&s[r + 8][k + 2 * t + 8];
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+    if (TRANS)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(a));
+    else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(a));
 }
 
-__device__ __forceinline__ void frag_b(unsigned (&b)[2], const bf16 (*s)[HP], int c, int k, int t)
+// left operand rows i.., columns k.. of s[i][k]
+__device__ __forceinline__ void frag_a(unsigned (&a)[4], const bf16 (*s)[HP], int i, int k, int lane)
 {
-    b[0] = *(const unsigned *)&s[c][k + 2 * t];
-    b[1] = *(const unsigned *)&s[c][k + 2 * t + 8];
+    ldsm4<false>(a, &s[i + (lane & 15)][k + (lane >> 4) * 8]);
+}
+// the same of s[k][i]
+__device__ __forceinline__ void frag_at(unsigned (&a)[4], const bf16 (*s)[HP], int i, int k, int lane)
+{
+    ldsm4<true>(a, &s[k + (lane >> 4) * 8 + (lane & 7)][i + ((lane >> 3) & 1) * 8]);
+}
+// right operands of two 8-column tiles n.., n + 8.. (registers 0, 1 and 2, 3) of s[n][k]
+__device__ __forceinline__ void frag_b2(unsigned (&b)[4], const bf16 (*s)[HP], int n, int k, int lane)
+{
+    ldsm4<false>(b, &s[n + (lane >> 4) * 8 + (lane & 7)][k + ((lane >> 3) & 1) * 8]);
+}
+// the same of s[k][n]
+__device__ __forceinline__ void frag_bt2(unsigned (&b)[4], const bf16 (*s)[HP], int n, int k, int lane)
+{
+    ldsm4<true>(b, &s[k + (lane & 15)][n + (lane >> 4) * 8]);
 }
 
-template <int MODE>
+__device__ __forceinline__ void mma_pair(float (&c0)[4], float (&c1)[4], const unsigned (&a)[4], const unsigned (&b)[4])
+{
+    const unsigned b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
+    mma_bf16(c0, a, b0);
+    mma_bf16(c1, a, b1);
+}
+
+// VEC: rank 64, even out, U's arrays and T on word boundaries: 16-byte loads
+// of U, pairs of everything else
+template <int MODE, bool VEC>
 __global__ void __launch_bounds__(256, 2) head_tile_kernel(HeadTile P)
 {
     extern __shared__ __align__(16) char smem_raw[];
@@ -655,13 +744,11 @@ __global__ void __launch_bounds__(256, 2) head_tile_kernel(HeadTile P)
     for (int e = threadIdx.x; e < HB * HR; e += 256) {
         const int b = e / HR, r = e % HR;
         bf16 hi, lo;
-        split_bf16(b < P.B && r < P.rank ? P.Z[b * P.rank + r] : 0.0f, hi, lo);
+        const float zv = b < P.B && r < P.rank ? P.Z[b * P.rank + r] : 0.0f;
+        split_bf16(zv, hi, lo);
         S.z[0][b][r] = hi;
         S.z[1][b][r] = lo;
-        if (MODE != HEAD_PREDICT) {
-            S.zt[0][r][b] = hi;
-            S.zt[1][r][b] = lo;
-        }
+        S.z[2][b][r] = __float2bfloat16_rn((zv - __bfloat162float(hi)) - __bfloat162float(lo));
     }
     float dz[4][4] = {};
     double sq = 0.0;
@@ -669,39 +756,45 @@ __global__ void __launch_bounds__(256, 2) head_tile_kernel(HeadTile P)
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int j0 = tile * HJ;
         __syncthreads(); // the previous tile's operands are read; Z is staged
-        if (P.rank == HR) { // rows of 64: contiguous over the threads
-#pragma unroll 4
-            for (int e = threadIdx.x; e < HJ * HR; e += 256) {
-                const int j = e / HR, r = e % HR;
-                const bf16 x = j0 + j < P.out ? P.wb[(size_t)(j0 + j) * HR + r] : __float2bfloat16_rn(0.0f);
-                S.u[j][r] = x;
-                if (MODE != HEAD_PREDICT)
-                    S.ut[r][j] = x;
+        if (VEC) { // 8 values a load, rows of 64: contiguous over the threads
+#pragma unroll
+            for (int e = threadIdx.x; e < HJ * HR / 8; e += 256) {
+                const int j = e / (HR / 8), r = e % (HR / 8) * 8;
+                uint4 x = make_uint4(0u, 0u, 0u, 0u);
+                if (j0 + j < P.out)
+                    x = *reinterpret_cast<const uint4 *>(P.wb + (size_t)(j0 + j) * HR + r);
+                *reinterpret_cast<uint4 *>(&S.u[j][r]) = x;
             }
         } else {
             for (int e = threadIdx.x; e < HJ * HR; e += 256) {
                 const int j = e / HR, r = e % HR;
-                const bf16 x = j0 + j < P.out && r < P.rank ? P.wb[(size_t)(j0 + j) * P.rank + r]
-                                                            : __float2bfloat16_rn(0.0f);
-                S.u[j][r] = x;
-                if (MODE != HEAD_PREDICT)
-                    S.ut[r][j] = x;
+                S.u[j][r] = j0 + j < P.out && r < P.rank ? P.wb[(size_t)(j0 + j) * P.rank + r]
+                                                         : __float2bfloat16_rn(0.0f);
             }
         }
         // this thread's targets and biases, in flight while U is staged
         float tv[4][4], bu[4][2];
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
+            const int j = j0 + n0 + 8 * nt + 2 * t;
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const int j = j0 + n0 + 8 * nt + 2 * t + q;
-                bu[nt][q] = j < P.out ? P.bw[j] : 0.0f;
-            }
+            for (int q = 0; q < 2; ++q)
+                bu[nt][q] = j + q < P.out ? P.bw[j + q] : 0.0f;
             if (MODE != HEAD_PREDICT) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int b = m0 + g + 8 * (q >> 1), j = j0 + n0 + 8 * nt + 2 * t + (q & 1);
-                    tv[nt][q] = b < P.B && j < P.out ? P.T[(size_t)b * P.out + j] : 0.0f;
+                for (int h = 0; h < 2; ++h) {
+                    const int b = m0 + g + 8 * h;
+                    if (VEC) { // even out: a pair is in or out
+                        float2 v = make_float2(0.0f, 0.0f);
+                        if (b < P.B && j < P.out)
+                            v = *reinterpret_cast<const float2 *>(P.T + (size_t)b * P.out + j);
+                        tv[nt][2 * h] = v.x;
+                        tv[nt][2 * h + 1] = v.y;
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 2; ++q)
+                            tv[nt][2 * h + q] = b < P.B && j + q < P.out ? P.T[(size_t)b * P.out + j + q] : 0.0f;
+                    }
                 }
             }
         }
@@ -709,46 +802,60 @@ __global__ void __launch_bounds__(256, 2) head_tile_kernel(HeadTile P)
         float o[4][4] = {};
 #pragma unroll
         for (int k = 0; k < HR; k += 16) {
-            unsigned ah[4], al[4], b[2];
-            frag_a(ah, S.z[0], m0 + g, k, t);
-            frag_a(al, S.z[1], m0 + g, k, t);
+            unsigned ah[4], al[4], a2[4], b[4];
+            frag_a(ah, S.z[0], m0, k, lane);
+            frag_a(al, S.z[1], m0, k, lane);
+            frag_a(a2, S.z[2], m0, k, lane);
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                frag_b(b, S.u, n0 + 8 * nt + g, k, t);
-                mma_bf16(o[nt], al, b);
-                mma_bf16(o[nt], ah, b);
+            for (int nt = 0; nt < 4; nt += 2) {
+                frag_b2(b, S.u, n0 + 8 * nt, k, lane);
+                mma_pair(o[nt], o[nt + 1], a2, b);
+                mma_pair(o[nt], o[nt + 1], al, b);
+                mma_pair(o[nt], o[nt + 1], ah, b);
             }
         }
         if (MODE == HEAD_PREDICT) {
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int b = m0 + g + 8 * (q >> 1), j = j0 + n0 + 8 * nt + 2 * t + (q & 1);
-                    if (b < P.B && j < P.out)
-                        P.O[(size_t)b * P.out + j] = o[nt][q] + bu[nt][q & 1];
+                for (int h = 0; h < 2; ++h) {
+                    const int b = m0 + g + 8 * h, j = j0 + n0 + 8 * nt + 2 * t;
+                    if (b >= P.B || j >= P.out)
+                        continue;
+                    const float v0 = o[nt][2 * h] + bu[nt][0], v1 = o[nt][2 * h + 1] + bu[nt][1];
+                    float *dst = P.O + (size_t)b * P.out + j;
+                    if (VEC) {
+                        *reinterpret_cast<float2 *>(dst) = make_float2(v0, v1);
+                    } else {
+                        dst[0] = v0;
+                        if (j + 1 < P.out)
+                            dst[1] = v1;
+                    }
                 }
             continue;
         }
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
             float cs[2] = {0.0f, 0.0f};
+            const int jj = n0 + 8 * nt + 2 * t;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int b = m0 + g + 8 * (q >> 1), jj = n0 + 8 * nt + 2 * t + (q & 1);
-                float d = 0.0f;
-                if (b < P.B && j0 + jj < P.out) {
-                    const float r = o[nt][q] + bu[nt][q & 1] - tv[nt][q];
-                    d = 2.0f * r * P.scale;
-                    sq += (double)r * (double)r;
+            for (int h = 0; h < 2; ++h) {
+                const int b = m0 + g + 8 * h;
+                float d[2];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    d[q] = 0.0f;
+                    if (b < P.B && j0 + jj + q < P.out) {
+                        const float r = o[nt][2 * h + q] + bu[nt][q] - tv[nt][2 * h + q];
+                        d[q] = 2.0f * r * P.scale;
+                        sq += (double)r * (double)r;
+                    }
+                    cs[q] += d[q];
                 }
-                cs[q & 1] += d;
-                bf16 hi, lo;
-                split_bf16(d, hi, lo);
-                S.d[0][b][jj] = hi;
-                S.d[1][b][jj] = lo;
-                S.dt[0][jj][b] = hi;
-                S.dt[1][jj][b] = lo;
+                unsigned hi, lo;
+                split2(d[0], d[1], hi, lo);
+                *reinterpret_cast<unsigned *>(&S.d[0][b][jj]) = hi;
+                *reinterpret_cast<unsigned *>(&S.d[1][b][jj]) = lo;
             }
 #pragma unroll
             for (int q = 0; q < 2; ++q) { // column sums over the warp's 16 rows
@@ -756,52 +863,97 @@ __global__ void __launch_bounds__(256, 2) head_tile_kernel(HeadTile P)
                 for (int s = 4; s < 32; s <<= 1)
                     cs[q] += __shfl_xor_sync(0xffffffffu, cs[q], s);
                 if (g == 0)
-                    S.db[warp & 3][n0 + 8 * nt + 2 * t + q] = cs[q];
+                    S.db[warp & 3][jj + q] = cs[q];
             }
         }
         __syncthreads();
         float du[4][4] = {};
 #pragma unroll
         for (int k = 0; k < HB; k += 16) {
-            unsigned ah[4], al[4], bh[2], bl[2];
-            frag_a(ah, S.dt[0], m0 + g, k, t);
-            frag_a(al, S.dt[1], m0 + g, k, t);
+            unsigned ah[4], al[4], bh[4], bl[4];
+            frag_at(ah, S.d[0], m0, k, lane);
+            frag_at(al, S.d[1], m0, k, lane);
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) { // dU = dO^T Z
-                frag_b(bh, S.zt[0], n0 + 8 * nt + g, k, t);
-                frag_b(bl, S.zt[1], n0 + 8 * nt + g, k, t);
-                mma_bf16(du[nt], al, bh);
-                mma_bf16(du[nt], ah, bl);
-                mma_bf16(du[nt], ah, bh);
+            for (int nt = 0; nt < 4; nt += 2) { // dU = dO^T Z
+                frag_bt2(bh, S.z[0], n0 + 8 * nt, k, lane);
+                frag_bt2(bl, S.z[1], n0 + 8 * nt, k, lane);
+                mma_pair(du[nt], du[nt + 1], al, bh);
+                mma_pair(du[nt], du[nt + 1], ah, bl);
+                mma_pair(du[nt], du[nt + 1], ah, bh);
             }
-            frag_a(ah, S.d[0], m0 + g, k, t);
-            frag_a(al, S.d[1], m0 + g, k, t);
+            frag_a(ah, S.d[0], m0, k, lane);
+            frag_a(al, S.d[1], m0, k, lane);
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) { // dZ += dO U
-                frag_b(bh, S.ut, n0 + 8 * nt + g, k, t);
-                mma_bf16(dz[nt], al, bh);
-                mma_bf16(dz[nt], ah, bh);
+            for (int nt = 0; nt < 4; nt += 2) { // dZ += dO U
+                frag_bt2(bh, S.u, n0 + 8 * nt, k, lane);
+                mma_pair(dz[nt], dz[nt + 1], al, bh);
+                mma_pair(dz[nt], dz[nt + 1], ah, bh);
             }
         }
+        // U's state, half of this thread's entries loaded before any is stored
+        // (with a load behind each store a tile took 28 us)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int h = 0; h < 2; ++h) {
+            float2 w[4], m[4], v[4]; // entry pairs (row j, ranks r, r + 1) of the four column tiles
+            const int j = j0 + m0 + g + 8 * h;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int j = j0 + m0 + g + 8 * (q >> 1), r = n0 + 8 * nt + 2 * t + (q & 1);
-                if (j < P.out && r < P.rank) {
-                    const size_t e = (size_t)j * P.rank + r;
-                    if (MODE == HEAD_GRAD) {
-                        P.g[e] = du[nt][q];
-                    } else {
-                        float m = P.m[e], v = P.v[e];
-                        const float w = adam_update(P.w[e], du[nt][q], m, v, P.a);
-                        P.m[e] = m;
-                        P.v[e] = v;
-                        P.w[e] = w;
-                        P.wb[e] = __float2bfloat16_rn(w);
+            for (int nt = 0; nt < 4 && MODE == HEAD_ADAM; ++nt) {
+                const int r = n0 + 8 * nt + 2 * t;
+                w[nt] = m[nt] = v[nt] = make_float2(0.0f, 0.0f);
+                const size_t e = (size_t)j * P.rank + r;
+                if (VEC) {
+                    if (j < P.out) {
+                        w[nt] = *reinterpret_cast<const float2 *>(P.w + e);
+                        m[nt] = *reinterpret_cast<const float2 *>(P.m + e);
+                        v[nt] = *reinterpret_cast<const float2 *>(P.v + e);
+                    }
+                } else if (j < P.out && r < P.rank) {
+                    w[nt].x = P.w[e];
+                    m[nt].x = P.m[e];
+                    v[nt].x = P.v[e];
+                    if (r + 1 < P.rank) {
+                        w[nt].y = P.w[e + 1];
+                        m[nt].y = P.m[e + 1];
+                        v[nt].y = P.v[e + 1];
                     }
                 }
             }
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                const int r = n0 + 8 * nt + 2 * t;
+                if (j >= P.out || r >= P.rank)
+                    continue;
+                const size_t e = (size_t)j * P.rank + r;
+                const float g0 = du[nt][2 * h], g1 = du[nt][2 * h + 1];
+                const bool two = VEC || r + 1 < P.rank;
+                if (MODE == HEAD_GRAD) {
+                    P.g[e] = g0;
+                    if (two)
+                        P.g[e + 1] = g1;
+                    continue;
+                }
+                float2 x;
+                x.x = adam_update(w[nt].x, g0, m[nt].x, v[nt].x, P.a);
+                x.y = adam_update(w[nt].y, g1, m[nt].y, v[nt].y, P.a);
+                if (VEC) {
+                    *reinterpret_cast<float2 *>(P.m + e) = m[nt];
+                    *reinterpret_cast<float2 *>(P.v + e) = v[nt];
+                    *reinterpret_cast<float2 *>(P.w + e) = x;
+                    *reinterpret_cast<__nv_bfloat162 *>(P.wb + e) = __floats2bfloat162_rn(x.x, x.y);
+                } else {
+                    P.m[e] = m[nt].x;
+                    P.v[e] = v[nt].x;
+                    P.w[e] = x.x;
+                    P.wb[e] = __float2bfloat16_rn(x.x);
+                    if (two) {
+                        P.m[e + 1] = m[nt].y;
+                        P.v[e + 1] = v[nt].y;
+                        P.w[e + 1] = x.y;
+                        P.wb[e + 1] = __float2bfloat16_rn(x.y);
+                    }
+                }
+            }
+        }
         if (threadIdx.x < HJ && j0 + (int)threadIdx.x < P.out) {
             const int j = j0 + threadIdx.x;
             const float gb = ((S.db[0][threadIdx.x] + S.db[1][threadIdx.x]) + S.db[2][threadIdx.x]) +
@@ -839,11 +991,27 @@ __global__ void __launch_bounds__(256, 2) head_tile_kernel(HeadTile P)
     }
 }
 
+// word boundaries of the head's arrays (and of T's rows, where there are any)
+bool head_vec(const HeadTile &P)
+{
+    return P.rank == HR && P.out % 2 == 0 && (size_t)P.wb % 16 == 0 &&
+           ((size_t)P.w | (size_t)P.m | (size_t)P.v | (size_t)P.T | (size_t)P.O) % 8 == 0;
+}
+
+template <int MODE>
+void launch_head(const HeadTile &P, int grid, size_t smem, cudaStream_t s)
+{
+    if (head_vec(P))
+        head_tile_kernel<MODE, true><<<grid, 256, smem, s>>>(P);
+    else
+        head_tile_kernel<MODE, false><<<grid, 256, smem, s>>>(P);
+}
+
 // dZ = the CTAs' shares in CTA order (8 runs of CTAs, then the runs); the
 // last block adds the loss
 __global__ void __launch_bounds__(256) head_fold_kernel(int n, int shares, const float *part, float *dZ,
                                                         const double *loss, double tot, const double *hloss,
-                                                        double *acc)
+                                                        int nhloss, double *acc)
 {
     if (blockIdx.x == gridDim.x - 1) {
         __shared__ double sh[256];
@@ -857,8 +1025,12 @@ __global__ void __launch_bounds__(256) head_fold_kernel(int n, int shares, const
                 sh[threadIdx.x] += sh[threadIdx.x + w];
             __syncthreads();
         }
-        if (threadIdx.x == 0)
-            acc[0] += sh[0] / tot + hloss[0];
+        if (threadIdx.x == 0) {
+            double v = sh[0] / tot;
+            for (int b = 0; b < nhloss; ++b)
+                v += hloss[b];
+            acc[0] += v;
+        }
         return;
     }
     __shared__ float run[8][32];
@@ -947,7 +1119,7 @@ int ensure_acts(pdhcg_b200_mlp_s *n, int B)
         al(&n->T, (long long)B * n->out) || al(&n->TL, B) || al(&n->dO, (long long)B * n->out) ||
         al(&n->dZ, (long long)B * n->rank) || al(&n->dH2, (long long)B * n->hid) ||
         al(&n->dH1, (long long)B * n->hid) || al(&n->dLW, B) ||
-        cudaMalloc((void **)&n->part, 148 * 8 * sizeof(double)) || cudaMalloc((void **)&n->hloss, sizeof(double)) ||
+        cudaMalloc((void **)&n->part, 148 * 8 * sizeof(double)) || cudaMalloc((void **)&n->hloss, (SMALL_B / SM_W) * sizeof(double)) ||
         cudaMalloc((void **)&n->acc, sizeof(double))) {
         std::fprintf(stderr, "[pdhcg_b200_mlp] activation allocation failed.\n");
         return -1;
@@ -964,6 +1136,12 @@ bool small_trunk(int B) { return B <= SMALL_B; }
 // one 64 x 64 tile of Z in a CTA's shared memory
 bool fused_head(const pdhcg_b200_mlp_s *n, int B) { return B <= HB && n->rank <= HR; }
 
+// K pairs of X (FP32, K a row) and of W (BF16) on word boundaries
+bool word_pairs(int K, const float *X, const bf16 *W)
+{
+    return (K & 1) == 0 && (size_t)X % 8 == 0 && (size_t)W % 4 == 0;
+}
+
 SmallGemm layer(int B, int N, int K, const float *X, const bf16 *W, const float *b, float *Y)
 {
     SmallGemm G{};
@@ -976,6 +1154,7 @@ SmallGemm layer(int B, int N, int K, const float *X, const bf16 *W, const float 
     G.ldb = K;
     G.C = Y;
     G.bias = b;
+    G.vec = word_pairs(K, X, W);
     return G;
 }
 
@@ -994,7 +1173,7 @@ int trunk_forward(pdhcg_b200_mlp_s *n, int B, const float *X, const float *TL)
                         g3 = layer(B, n->rank, n->hid, n->H2, W3, b3, n->Z);
         small_layer_kernel<EPI_BIAS_RELU, false><<<g1.tiles(), 32 * SM_W, 0, s>>>(g1, h);
         small_layer_kernel<EPI_BIAS_RELU, false><<<g2.tiles(), 32 * SM_W, 0, s>>>(g2, h);
-        small_layer_kernel<EPI_BIAS, true><<<g3.tiles() + 1, 32 * SM_W, 0, s>>>(g3, h);
+        small_layer_kernel<EPI_BIAS, true><<<g3.tiles() + (B + SM_W - 1) / SM_W, 32 * SM_W, 0, s>>>(g3, h);
         MCK(cudaGetLastError());
         return 0;
     }
@@ -1036,7 +1215,7 @@ HeadTile head_tile(const pdhcg_b200_mlp_s *n, int B, const float *T)
 }
 
 int head_grid(const pdhcg_b200_mlp_s *n) { return std::min((n->out + HJ - 1) / HJ, 2 * 148); }
-constexpr size_t HEAD_SMEM_PREDICT = offsetof(HeadSmem, zt), HEAD_SMEM = sizeof(HeadSmem);
+constexpr size_t HEAD_SMEM_PREDICT = offsetof(HeadSmem, d), HEAD_SMEM = sizeof(HeadSmem);
 
 // o of the rows that trunk_forward took, into n->O
 int head_forward(pdhcg_b200_mlp_s *n, int B)
@@ -1044,7 +1223,7 @@ int head_forward(pdhcg_b200_mlp_s *n, int B)
     cudaStream_t s = n->s;
     if (fused_head(n, B)) {
         const int grid = std::min((n->out + HJ - 1) / HJ, 8 * 148);
-        head_tile_kernel<HEAD_PREDICT><<<grid, 256, HEAD_SMEM_PREDICT, s>>>(head_tile(n, B, nullptr));
+        launch_head<HEAD_PREDICT>(head_tile(n, B, nullptr), grid, HEAD_SMEM_PREDICT, s);
     } else {
         if (gemm<false, true>(B, n->out, n->rank, n->Z, n->rank, n->wb + n->off[P_U], n->rank, n->O, n->out, 1.0f, 0.0f,
                               s, n->ws))
@@ -1078,18 +1257,20 @@ int step(pdhcg_b200_mlp_s *n, int B, const float *X, const float *T, const float
         P.part = n->ws.p;
         if (adam) {
             P.a = *adam;
-            head_tile_kernel<HEAD_ADAM><<<grid, 256, HEAD_SMEM, s>>>(P);
+            launch_head<HEAD_ADAM>(P, grid, HEAD_SMEM, s);
         } else {
-            head_tile_kernel<HEAD_GRAD><<<grid, 256, HEAD_SMEM, s>>>(P);
+            launch_head<HEAD_GRAD>(P, grid, HEAD_SMEM, s);
         }
         head_fold_kernel<<<(B * n->rank + 31) / 32 + 1, 256, 0, s>>>(B * n->rank, grid, n->ws.p, n->dZ, n->part,
-                                                                    (double)tot, n->hloss, n->acc);
+                                                                    (double)tot, n->hloss, (B + SM_W - 1) / SM_W,
+                                                                    n->acc);
     } else {
         if (head_forward(n, B))
             return -1;
         int nb = blocks_for(tot);
         mse_kernel<<<nb, 256, 0, s>>>(tot, n->O, T, 1.0f / (float)tot, n->dO, n->part);
-        loss_fold_kernel<<<1, 256, 0, s>>>(n->part, nb, (double)tot, n->hloss, n->acc);
+        loss_fold_kernel<<<1, 256, 0, s>>>(n->part, nb, (double)tot, n->hloss,
+                                           small_trunk(B) ? (B + SM_W - 1) / SM_W : 1, n->acc);
         // dU = dO^T Z, dbu = colsum dO, dZ = dO U
         if (gemm<true, false>(n->out, n->rank, B, n->dO, n->out, n->Z, n->rank, g + n->off[P_U], n->rank, 1.0f, 0.0f, s,
                               n->ws))
@@ -1111,6 +1292,7 @@ int step(pdhcg_b200_mlp_s *n, int B, const float *X, const float *T, const float
             b.dx.ldb = in;
             b.dx.C = dX;
             b.dx.mask = mask;
+            b.dx.vec = word_pairs(out, dY, nullptr);
             b.dw.M = out;
             b.dw.N = in;
             b.dw.K = B;
@@ -1177,6 +1359,17 @@ int refresh_bf16(pdhcg_b200_mlp_s *n)
     return 0;
 }
 
+cudaError_t head_attributes()
+{
+    for (auto k : {head_tile_kernel<HEAD_GRAD, false>, head_tile_kernel<HEAD_GRAD, true>,
+                   head_tile_kernel<HEAD_ADAM, false>, head_tile_kernel<HEAD_ADAM, true>}) {
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HEAD_SMEM);
+        if (e != cudaSuccess)
+            return e;
+    }
+    return cudaSuccess;
+}
+
 // splitmix64 -> uniform in [-1, 1)
 double unif(unsigned long long &st)
 {
@@ -1230,14 +1423,11 @@ pdhcg_b200_mlp_t *pdhcg_b200_mlp_create(int in_dim, int hidden, int rank, int ou
         cudaMalloc((void **)&n->mom, o * sizeof(float)) != cudaSuccess ||
         cudaMalloc((void **)&n->vel, o * sizeof(float)) != cudaSuccess ||
         cudaMalloc((void **)&n->wb, o * sizeof(bf16)) != cudaSuccess ||
-        cudaMemcpy(n->w, h.data(), o * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemset(n->mom, 0, o * sizeof(float)) != cudaSuccess ||
-        cudaMemset(n->vel, 0, o * sizeof(float)) != cudaSuccess ||
-        cudaFuncSetAttribute(head_tile_kernel<HEAD_GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)HEAD_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(head_tile_kernel<HEAD_ADAM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)HEAD_SMEM) != cudaSuccess ||
-        refresh_bf16(n) != 0) {
+        cudaMemcpyAsync(n->w, h.data(), o * sizeof(float), cudaMemcpyHostToDevice, n->s) != cudaSuccess ||
+        cudaMemsetAsync(n->mom, 0, o * sizeof(float), n->s) != cudaSuccess ||
+        cudaMemsetAsync(n->vel, 0, o * sizeof(float), n->s) != cudaSuccess ||
+        head_attributes() != cudaSuccess ||
+        refresh_bf16(n) != 0 || cudaStreamSynchronize(n->s) != cudaSuccess) {
         std::fprintf(stderr, "[pdhcg_b200_mlp_create] device allocation failed.\n");
         pdhcg_b200_mlp_free(n);
         return nullptr;
@@ -1266,7 +1456,8 @@ int pdhcg_b200_mlp_get_params(const pdhcg_b200_mlp_t *n, float *out)
 {
     if (!n || !out)
         return -1;
-    MCK(cudaMemcpy(out, n->w, n->total * sizeof(float), cudaMemcpyDeviceToHost));
+    MCK(cudaMemcpyAsync(out, n->w, n->total * sizeof(float), cudaMemcpyDeviceToHost, n->s));
+    MCK(cudaStreamSynchronize(n->s));
     return 0;
 }
 
@@ -1274,11 +1465,16 @@ int pdhcg_b200_mlp_set_params(pdhcg_b200_mlp_t *n, const float *in)
 {
     if (!n || !in)
         return -1;
-    MCK(cudaMemcpy(n->w, in, n->total * sizeof(float), cudaMemcpyHostToDevice));
+    // in the network's stream: a copy from pageable memory may return before
+    // its last part has arrived, and this stream does not wait for others
+    MCK(cudaMemcpyAsync(n->w, in, n->total * sizeof(float), cudaMemcpyHostToDevice, n->s));
     n->step = 0;
-    MCK(cudaMemset(n->mom, 0, n->total * sizeof(float)));
-    MCK(cudaMemset(n->vel, 0, n->total * sizeof(float)));
-    return refresh_bf16(n);
+    MCK(cudaMemsetAsync(n->mom, 0, n->total * sizeof(float), n->s));
+    MCK(cudaMemsetAsync(n->vel, 0, n->total * sizeof(float), n->s));
+    if (refresh_bf16(n))
+        return -1;
+    MCK(cudaStreamSynchronize(n->s));
+    return 0;
 }
 
 int pdhcg_b200_mlp_predict(pdhcg_b200_mlp_t *n, int batch, const float *theta, float *out, float *logw)
@@ -1330,9 +1526,9 @@ int pdhcg_b200_mlp_train(pdhcg_b200_mlp_t *n, int count, const float *theta, con
     MCK(cudaMalloc((void **)&dth, (size_t)count * n->in * sizeof(float)));
     MCK(cudaMalloc((void **)&dt, (size_t)count * n->out * sizeof(float)));
     MCK(cudaMalloc((void **)&dtl, count * sizeof(float)));
-    MCK(cudaMemcpy(dth, theta, (size_t)count * n->in * sizeof(float), cudaMemcpyHostToDevice));
-    MCK(cudaMemcpy(dt, target, (size_t)count * n->out * sizeof(float), cudaMemcpyHostToDevice));
-    MCK(cudaMemcpy(dtl, target_logw, count * sizeof(float), cudaMemcpyHostToDevice));
+    MCK(cudaMemcpyAsync(dth, theta, (size_t)count * n->in * sizeof(float), cudaMemcpyHostToDevice, n->s));
+    MCK(cudaMemcpyAsync(dt, target, (size_t)count * n->out * sizeof(float), cudaMemcpyHostToDevice, n->s));
+    MCK(cudaMemcpyAsync(dtl, target_logw, count * sizeof(float), cudaMemcpyHostToDevice, n->s));
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     int rc = 0, nbat = 0;
     for (int ep = 0; ep < epochs && rc == 0; ++ep) {
