@@ -111,36 +111,30 @@ __device__ __forceinline__ int warp_max_int(int v)
 // segments' partials in segment order, each lane for its own row.  The
 // partials belong to the last vector passed to that kernel: every product
 // of a matrix with long rows is preceded by its pass.
+//
+// A segment whose columns are consecutive (a dense row, or a long dense part
+// of one: budget and factor-exposure rows) is read without its column
+// indices: seg_col holds its first column, -1 elsewhere.  That is 8 instead
+// of 12 bytes per entry of a pass that HBM bounds, and the vector is read
+// coalesced instead of gathered.
 // ---------------------------------------------------------------------------
 constexpr int LONG_ROW = STREAM_ROW_MAX; // every row beyond stream mode
 constexpr int LONG_SEG = 4096;
 
 struct LongRows {
     const int *rows;      // [n] long row ids, ascending
+    const int *index;     // [rows of the matrix] a long row's index in rows, -1 for the others
     const int *seg_first; // [n + 1] first segment of each long row
     const int2 *seg;      // [nseg] entry range {begin, end} of each segment
+    const int *seg_col;   // [nseg] first column of a segment of consecutive columns, else -1
     double *part;         // [nseg] partial products of the last pass
     int n, nseg;
 };
 
-// index of the first long row >= row (L.n when none)
-__device__ __forceinline__ int long_lower_bound(const LongRows &L, int row)
-{
-    int lo = 0, hi = L.n;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(L.rows + mid) < row)
-            lo = mid + 1;
-        else
-            hi = mid;
-    }
-    return lo;
-}
-
 // the same sum computed by the whole warp for one row (every lane calls it)
 __device__ __forceinline__ double long_row_sum_warp(const LongRows &L, int row, int lane)
 {
-    const int i = long_lower_bound(L, row);
+    const int i = __ldg(L.index + row);
     const int f = __ldg(L.seg_first + i), e = __ldg(L.seg_first + i + 1);
     double a = 0.0;
     for (int k = f + lane; k < e; k += 32)
@@ -153,13 +147,36 @@ __device__ __forceinline__ double long_row_fold(const LongRows &L, int i)
 {
     const int f = __ldg(L.seg_first + i), e = __ldg(L.seg_first + i + 1);
     double a = 0.0;
-    for (int k = f; k < e; ++k)
+    // eight partials' loads in flight, added in segment order
+    int k = f;
+    for (; k + 8 <= e; k += 8) {
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            v[u] = L.part[k + u];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            a += v[u];
+    }
+    for (; k < e; ++k)
         a += L.part[k];
     return a;
 }
 
+// An entry of the vector of a product.  CG: the vector is written by other
+// blocks of the same launch (persistent kernels), so the load goes to L2
+// instead of the read-only path, which is not coherent within a launch.
+template <bool CG, typename X>
+__device__ __forceinline__ X load_x(const X *x)
+{
+    if constexpr (CG)
+        return __ldcg(x);
+    else
+        return __ldg(x);
+}
+
 // one warp's dot product over entries [b, e), lane-strided, 4 partial sums
-template <typename V, typename X>
+template <bool CG = false, typename V, typename X>
 __device__ __forceinline__ double warp_range_dot(const int *__restrict__ ci, const V *__restrict__ val,
                                                  const X *__restrict__ x, int b, int e, int lane)
 {
@@ -178,7 +195,7 @@ __device__ __forceinline__ double warp_range_dot(const int *__restrict__ ci, con
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u)
-            w[u] = (double)__ldg(x + c[u]);
+            w[u] = (double)load_x<CG>(x + c[u]);
         a0 += v[0] * w[0];
         a1 += v[1] * w[1];
         a2 += v[2] * w[2];
@@ -189,10 +206,10 @@ __device__ __forceinline__ double warp_range_dot(const int *__restrict__ ci, con
         a3 += v[7] * w[7];
     }
     for (; k + 96 < e; k += 128) {
-        a0 += (double)__ldg(val + k) * (double)__ldg(x + __ldg(ci + k));
-        a1 += (double)__ldg(val + k + 32) * (double)__ldg(x + __ldg(ci + k + 32));
-        a2 += (double)__ldg(val + k + 64) * (double)__ldg(x + __ldg(ci + k + 64));
-        a3 += (double)__ldg(val + k + 96) * (double)__ldg(x + __ldg(ci + k + 96));
+        a0 += (double)__ldg(val + k) * (double)load_x<CG>(x + __ldg(ci + k));
+        a1 += (double)__ldg(val + k + 32) * (double)load_x<CG>(x + __ldg(ci + k + 32));
+        a2 += (double)__ldg(val + k + 64) * (double)load_x<CG>(x + __ldg(ci + k + 64));
+        a3 += (double)__ldg(val + k + 96) * (double)load_x<CG>(x + __ldg(ci + k + 96));
     }
     // at most three strides remain (k + 96 >= e): their loads are issued
     // together, then added to a0 in stride order
@@ -200,8 +217,8 @@ __device__ __forceinline__ double warp_range_dot(const int *__restrict__ ci, con
     const int c0 = p0 ? __ldg(ci + k) : 0, c1 = p1 ? __ldg(ci + k + 32) : 0, c2 = p2 ? __ldg(ci + k + 64) : 0;
     const double v0 = p0 ? (double)__ldg(val + k) : 0.0, v1 = p1 ? (double)__ldg(val + k + 32) : 0.0,
                  v2 = p2 ? (double)__ldg(val + k + 64) : 0.0;
-    const double x0 = p0 ? (double)__ldg(x + c0) : 0.0, x1 = p1 ? (double)__ldg(x + c1) : 0.0,
-                 x2 = p2 ? (double)__ldg(x + c2) : 0.0;
+    const double x0 = p0 ? (double)load_x<CG>(x + c0) : 0.0, x1 = p1 ? (double)load_x<CG>(x + c1) : 0.0,
+                 x2 = p2 ? (double)load_x<CG>(x + c2) : 0.0;
     if (p0)
         a0 += v0 * x0;
     if (p1)
@@ -211,9 +228,40 @@ __device__ __forceinline__ double warp_range_dot(const int *__restrict__ ci, con
     return warp_sum((a0 + a1) + (a2 + a3));
 }
 
+// the same over entries [b, e) whose columns are the consecutive ones from
+// x's start on (x points at the first): no indices, two times eight loads in
+// flight; the partial sums and their order are those of warp_range_dot
+template <bool CG = false, typename V, typename X>
+__device__ __forceinline__ double warp_range_dot_run(const V *__restrict__ val, const X *__restrict__ x, int len,
+                                                     int lane)
+{
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    int k = lane;
+    for (; k + 480 < len; k += 512) {
+        V v[16];
+        X w[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            v[u] = __ldg(val + k + 32 * u);
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            w[u] = load_x<CG>(x + k + 32 * u);
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            a[u & 3] += (double)v[u] * (double)w[u];
+    }
+    for (; k + 96 < len; k += 128)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            a[u] += (double)__ldg(val + k + 32 * u) * (double)load_x<CG>(x + k + 32 * u);
+    for (; k < len; k += 32) // at most three strides
+        a[0] += (double)__ldg(val + k) * (double)load_x<CG>(x + k);
+    return warp_sum((a[0] + a[1]) + (a[2] + a[3]));
+}
+
 // the segment pass over warps gw, gw + nw, ... (a kernel body, or a phase
 // of a cooperative kernel followed by a grid barrier)
-template <typename V, typename X>
+template <bool CG = false, typename V, typename X>
 __device__ __forceinline__ void long_partials(const LongRows &L, const int *__restrict__ ci,
                                               const V *__restrict__ val, const X *__restrict__ x, int gw, int nw,
                                               int lane)
@@ -221,12 +269,16 @@ __device__ __forceinline__ void long_partials(const LongRows &L, const int *__re
     // the next segment's bounds are loaded before this segment's sum, so a
     // warp that walks many short segments does not wait for them each time
     int2 r = gw < L.nseg ? L.seg[gw] : make_int2(0, 0);
+    int c = gw < L.nseg ? L.seg_col[gw] : -1;
     for (int sg = gw; sg < L.nseg; sg += nw) {
         const int2 rn = sg + nw < L.nseg ? L.seg[sg + nw] : make_int2(0, 0);
-        const double a = warp_range_dot(ci, val, x, r.x, r.y, lane);
+        const int cn = sg + nw < L.nseg ? L.seg_col[sg + nw] : -1;
+        const double a = c >= 0 ? warp_range_dot_run<CG>(val + r.x, x + c, r.y - r.x, lane)
+                                : warp_range_dot<CG>(ci, val, x, r.x, r.y, lane);
         if (lane == 0)
             L.part[sg] = a;
         r = rn;
+        c = cn;
     }
 }
 
@@ -235,6 +287,28 @@ __global__ void __launch_bounds__(256) long_partials_kernel(LongRows L, const in
 {
     long_partials(L, ci, val, x, (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5),
                   (int)((gridDim.x * blockDim.x) >> 5), (int)(threadIdx.x & 31));
+}
+
+// first column of every segment whose columns are consecutive, else -1; a
+// warp per segment.  Short segments keep their indices (a run of them gains
+// nothing over the gather).
+constexpr int LONG_RUN_MIN = 256;
+
+static __global__ void long_seg_col_kernel(LongRows L, const int *ci, int *seg_col)
+{
+    const int lane = threadIdx.x & 31;
+    for (int sg = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); sg < L.nseg;
+         sg += (int)((gridDim.x * blockDim.x) >> 5)) {
+        const int2 r = L.seg[sg];
+        const int c0 = ci[r.x];
+        bool run = r.y - r.x >= LONG_RUN_MIN;
+        if (run)
+            for (int k = r.x + lane; k < r.y; k += 32)
+                run = run && ci[k] == c0 + (k - r.x);
+        run = __all_sync(FULL, run);
+        if (lane == 0)
+            seg_col[sg] = run ? c0 : -1;
+    }
 }
 
 // number of rows longer than LONG_ROW entries
@@ -253,7 +327,7 @@ static __global__ void long_count_kernel(int rows, const int *rp, int *count)
 // holding such a row is otherwise reduced one row at a time by the whole
 // warp (no table, lr.n = 0; or S > 2, where the lane-wise form would cost
 // the wide cone kernels their registers).
-template <int S, typename V, typename X>
+template <int S, bool CG = false, typename V, typename X>
 __device__ __forceinline__ void warp_stream_rows(const int *__restrict__ rp, const int *__restrict__ ci,
                                                  const V *__restrict__ val, const X *__restrict__ x, int r0, int nr,
                                                  int lane, double *stage, double (&out)[S], const LongRows &lr)
@@ -292,7 +366,7 @@ __device__ __forceinline__ void warp_stream_rows(const int *__restrict__ rp, con
             }
 #pragma unroll
             for (int u = 0; u < STREAM_U; ++u)
-                stage[32 * u + lane] = col[u] >= 0 ? v[u] * (double)__ldg(x + col[u]) : 0.0;
+                stage[32 * u + lane] = col[u] >= 0 ? v[u] * (double)load_x<CG>(x + col[u]) : 0.0;
             __syncwarp();
             const int ce = min(e, cb + STREAM_CHUNK);
 #pragma unroll
@@ -307,24 +381,19 @@ __device__ __forceinline__ void warp_stream_rows(const int *__restrict__ rp, con
         }
     } else if (S <= 2 && lr.n > 0) {
         // every row longer than LONG_ROW is in lr: each lane folds its own
-        // long row's partials (its table index from one search per tile and
-        // a ballot) or adds its own short row in entry order
-        const int base = long_lower_bound(lr, r0);
-        int before = 0;
+        // long row's partials or adds its own short row in entry order
 #pragma unroll
         for (int s = 0; s < S; ++s) {
             const bool valid = lane + 32 * s < nr;
             const bool lg = valid && re[s] - rb[s] > LONG_ROW;
-            const unsigned mask = __ballot_sync(FULL, lg);
             if (lg) {
-                out[s] = long_row_fold(lr, base + before + __popc(mask & ((1u << lane) - 1u)));
+                out[s] = long_row_fold(lr, __ldg(lr.index + r0 + lane + 32 * s));
             } else if (valid) {
                 double a = 0.0;
                 for (int k = rb[s]; k < re[s]; ++k)
-                    a += (double)__ldg(val + k) * (double)__ldg(x + __ldg(ci + k));
+                    a += (double)__ldg(val + k) * (double)load_x<CG>(x + __ldg(ci + k));
                 out[s] = a;
             }
-            before += __popc(mask);
         }
     } else {
         for (int i = 0; i < nr; ++i) {
@@ -339,7 +408,7 @@ __device__ __forceinline__ void warp_stream_rows(const int *__restrict__ rp, con
             ei = __shfl_sync(FULL, ei, i & 31);
             // (wide tiles with a long-row table: the warp folds each long row)
             const double a = (lr.n > 0 && ei - bi > LONG_ROW) ? long_row_sum_warp(lr, r0 + i, lane)
-                                                                : warp_range_dot(ci, val, x, bi, ei, lane);
+                                                                : warp_range_dot<CG>(ci, val, x, bi, ei, lane);
 #pragma unroll
             for (int s = 0; s < S; ++s)
                 if (s == (i >> 5) && lane == (i & 31))

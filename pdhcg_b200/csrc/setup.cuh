@@ -8,6 +8,7 @@
 
 #include <cooperative_groups.h>
 
+#include "gridsum.cuh"
 #include "kernels.cuh"
 
 namespace pdhcg {
@@ -144,18 +145,38 @@ __global__ void row_absmax_kernel(const int *rp, const double *v, int rows, doub
     }
 }
 
+// Long rows of the set-up passes: one block per row, or one warp where the
+// rows are short of a block's width (2e5 rows of 102 entries: 340 us a pass
+// with a block per row, whose reduction outweighs the row).
+constexpr int LONG_WARP_MEAN = 1024; // mean entries up to which a warp takes a row
+
+// f(row, first lane, lanes) for every long row; WARP: a warp per row
+template <bool WARP, typename F>
+__device__ __forceinline__ void for_long_rows(const LongRows &L, F &&f)
+{
+    if (WARP) {
+        const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+        for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < L.n; i += nw)
+            f(L.rows[i], lane, 32);
+    } else {
+        for (int i = blockIdx.x; i < L.n; i += gridDim.x)
+            f(L.rows[i], (int)threadIdx.x, (int)blockDim.x);
+    }
+}
+
 // the maximum is exact in any order, so a long row's value is the same
+template <bool WARP>
 __global__ void long_row_absmax_kernel(LongRows L, const int *rp, const double *v, double *out)
 {
-    for (int i = blockIdx.x; i < L.n; i += gridDim.x) {
-        const int r = L.rows[i];
+    for_long_rows<WARP>(L, [&](int r, int at, int step) {
         double mx = 0.0;
-        for (int k = rp[r] + threadIdx.x; k < rp[r + 1]; k += blockDim.x)
+#pragma unroll 4
+        for (int k = rp[r] + at; k < rp[r + 1]; k += step)
             mx = fmax(mx, fabs(v[k]));
-        mx = block_max(mx);
-        if (threadIdx.x == 0)
+        mx = WARP ? warp_max(mx) : block_max(mx);
+        if (at == 0)
             out[r] = mx;
-    }
+    });
 }
 
 // sum_k |a_k|^p per row; p == 1 uses |a| itself (pow(x, 1) == x exactly)
@@ -175,19 +196,20 @@ __global__ void row_powsum_kernel(const int *rp, const double *v, int rows, doub
 
 // a long row's sum in a fixed order (thread-strided, then a tree): the same
 // on every run, but associated differently from a sequential sum
+template <bool WARP>
 __global__ void long_row_powsum_kernel(LongRows L, const int *rp, const double *v, double p, double *out)
 {
-    for (int i = blockIdx.x; i < L.n; i += gridDim.x) {
-        const int r = L.rows[i];
-        double s = 0.0;
-        for (int k = rp[r] + threadIdx.x; k < rp[r + 1]; k += blockDim.x) {
+    for_long_rows<WARP>(L, [&](int r, int at, int step) {
+        double t = 0.0;
+#pragma unroll 4
+        for (int k = rp[r] + at; k < rp[r + 1]; k += step) {
             const double a = fabs(v[k]);
-            s += (p == 1.0) ? a : pow(a, p);
+            t += (p == 1.0) ? a : pow(a, p);
         }
-        s = block_sum_fixed(s);
-        if (threadIdx.x == 0)
-            out[r] = s;
-    }
+        t = WARP ? warp_sum(t) : block_sum_fixed(t);
+        if (at == 0)
+            out[r] = t;
+    });
 }
 
 __global__ void sqrt_or_one_kernel(double *v, int n)
@@ -278,17 +300,18 @@ __global__ void scale_csr_kernel(const int *rp, const int *ci, double *v, int ro
     }
 }
 
+template <bool WARP>
 __global__ void long_scale_csr_kernel(LongRows L, const int *rp, const int *ci, double *v, const double *rs,
                                       const double *cs, int cr_first)
 {
-    for (int i = blockIdx.x; i < L.n; i += gridDim.x) {
-        const int r = L.rows[i];
+    for_long_rows<WARP>(L, [&](int r, int at, int step) {
         const double a = rs[r];
-        for (int k = rp[r] + threadIdx.x; k < rp[r + 1]; k += blockDim.x) {
+#pragma unroll 4
+        for (int k = rp[r] + at; k < rp[r + 1]; k += step) {
             const double b = cs[ci[k]];
             v[k] /= cr_first ? (b * a) : (a * b);
         }
-    }
+    });
 }
 
 // v_k /= rs[r] for every entry of row r (rows of at most LONG_ROW entries:
@@ -510,117 +533,110 @@ __global__ void result_kernel(int n, int m, const int *At_rp, const int *At_ci, 
 }
 
 // ---------------------------------------------------------------------------
-// Power method for sigma_max(A) on A A^T, one cooperative launch (reference
-// estimate_maximum_singular_value, src/pdhg_core_op.cu:1673-1788): the same
-// sequence of operations, with the vector reductions done as fixed-order
-// block folds shared by every block after each grid barrier.
+// Lanczos process of A A^T (m x m) for the step size, `steps` more steps in
+// one cooperative launch.  Vectors are kept unnormalised with their scale
+// (q_j = inv u_j); a step is
+//   z = A^T q_j;  alpha_j = |z|^2;
+//   u_{j+1} = A z - beta_{j-1} q_{j-1} - alpha_j q_j  (over u_{j-1});
+//   beta_j = |u_{j+1}|
+// with two grid-wide sums, which are also its barriers.  One block of 32
+// warps per SM (fewer on small problems: the barrier's cost grows with the
+// blocks).
 // ---------------------------------------------------------------------------
-static __device__ double coop_fold(const double *part, int nb)
-{
-    __shared__ double sh[TPB];
-    double a = 0.0;
-    for (int b = threadIdx.x; b < nb; b += TPB)
-        a += part[b];
-    sh[threadIdx.x] = a;
-    __syncthreads();
-    for (int o = TPB / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    double r = sh[0];
-    __syncthreads();
-    return r;
-}
+constexpr int LANCZOS_MAX = 512, LANCZOS_CHUNK = 16, LANCZOS_TPB = 1024;
+constexpr int LANCZOS_SMEM = (LANCZOS_TPB / 32) * STREAM_CHUNK * (int)sizeof(double);
 
-static __device__ void coop_block_partial(double v, double *part)
+struct LanczosData {
+    int m, n;
+    const int *A_rp, *A_ci;
+    const double *A_v;
+    const int *At_rp, *At_ci;
+    const double *At_v;
+    LongRows A_long, At_long;
+    double *u[2]; // the start vector in u[0]
+    double *z;
+    double *out; // [0] inv of the current vector, [1] inv of the previous, [2] beta between them,
+                 // [3] steps done, then alpha[LANCZOS_MAX], beta[LANCZOS_MAX]
+};
+
+static __global__ void __launch_bounds__(LANCZOS_TPB) lanczos_kernel(LanczosData L, GridSlots S, int j0, int steps)
 {
-    __shared__ double sh[WARPS];
-    double w = warp_sum(v);
-    if ((threadIdx.x & 31) == 0)
-        sh[threadIdx.x >> 5] = w;
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    extern __shared__ double lanczos_stage[];
+    __shared__ double sh[LANCZOS_TPB / 32 + 1];
+    const int NW = LANCZOS_TPB / 32;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int gw = blockIdx.x * NW + wib, nw = gridDim.x * NW;
+    double *stage = lanczos_stage + wib * STREAM_CHUNK;
+    double inv, inv_prev = 0.0, beta = 0.0;
+    grid_begin(S);
+    if (j0 == 0) {
         double a = 0.0;
-        for (int i = 0; i < WARPS; ++i)
-            a += sh[i];
-        part[blockIdx.x] = a;
+        for (int i = blockIdx.x * LANCZOS_TPB + threadIdx.x; i < L.m; i += gridDim.x * LANCZOS_TPB)
+            a += L.u[0][i] * L.u[0][i];
+        inv = 1.0 / sqrt(grid_sum<NW>(a, S, sh));
+    } else {
+        inv = L.out[0];
+        inv_prev = L.out[1];
+        beta = L.out[2];
+        grid_barrier(S); // every block has read the state that block 0 will write
     }
-    __syncthreads();
-}
-
-template <typename MT>
-__global__ void __launch_bounds__(TPB) power_sigma_kernel(int m, int n, const int *A_rp, const int *A_ci,
-                                                          const MT *A_v, const int *At_rp, const int *At_ci,
-                                                          const MT *At_v, double *v, double *nv, double *dp,
-                                                          double *part /* 4 * gridDim */, int max_iter, double tol,
-                                                          double *out /* [sigma, iterations] */, LongRows A_long,
-                                                          LongRows At_long)
-{
-    // The iterate is u with |u| = 1 / inv (v = inv * u is the unit vector):
-    //   dp = inv * A^T u;  w = A dp = A A^T v
-    //   s2 = v . w = inv * (u . w);  |w - s2 v|^2 = |w|^2 - s2^2  (|v| = 1)
-    // then u <- w, inv <- 1 / |w|: two grid barriers per iteration, the
-    // buffers of u and w alternate.
-    cg::grid_group grid = cg::this_grid();
-    __shared__ double stage_all[WARPS][STREAM_CHUNK];
-    const int nb = gridDim.x;
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-    const int lane = threadIdx.x & 31, gw = blockIdx.x * WARPS + (threadIdx.x >> 5), nw = gridDim.x * WARPS;
-    double *stage = stage_all[threadIdx.x >> 5];
-    double *p0 = part, *p1 = part + nb, *p2 = part + 2 * nb;
-    double a = 0.0;
-    for (int i = tid; i < m; i += nth)
-        a += v[i] * v[i];
-    coop_block_partial(a, p0);
-    grid.sync();
-    double inv = 1.0 / sqrt(coop_fold(p0, nb));
-    double *u = v, *w = nv;
-    double s2 = 1.0;
-    int it = 0;
-    for (; it < max_iter; ++it) {
-        if (At_long.n > 0) { // segment pass of the long rows, then the rows
-            long_partials(At_long, At_ci, At_v, u, gw, nw, lane);
-            grid.sync();
+    int j = j0;
+    double last = 0.0; // scale of T, for the exhaustion test
+    for (; j < j0 + steps; ++j) {
+        double *u = L.u[j & 1], *up = L.u[(j & 1) ^ 1];
+        if (L.At_long.n > 0) { // segment pass of the long rows, then the rows
+            long_partials<true>(L.At_long, L.At_ci, L.At_v, u, gw, nw, lane);
+            grid_barrier(S);
         }
-        for (int t = gw; t < (n + 31) / 32; t += nw) {
-            const int r0 = 32 * t, nr = min(32, n - r0);
+        double a = 0.0;
+        for (int t = gw; t < (L.n + 31) / 32; t += nw) {
+            const int r0 = 32 * t, nr = min(32, L.n - r0);
             double r[1];
-            warp_stream_rows<1>(At_rp, At_ci, At_v, u, r0, nr, lane, stage, r, At_long);
-            if (lane < nr)
-                dp[r0 + lane] = r[0] * inv;
-        }
-        grid.sync();
-        if (A_long.n > 0) {
-            long_partials(A_long, A_ci, A_v, dp, gw, nw, lane);
-            grid.sync();
-        }
-        double uw = 0.0, ww = 0.0;
-        for (int t = gw; t < (m + 31) / 32; t += nw) {
-            const int r0 = 32 * t, nr = min(32, m - r0);
-            double r[1];
-            warp_stream_rows<1>(A_rp, A_ci, A_v, dp, r0, nr, lane, stage, r, A_long);
+            warp_stream_rows<1, true>(L.At_rp, L.At_ci, L.At_v, u, r0, nr, lane, stage, r, L.At_long);
             if (lane < nr) {
-                w[r0 + lane] = r[0];
-                uw += r[0] * u[r0 + lane];
-                ww += r[0] * r[0];
+                const double z = r[0] * inv;
+                L.z[r0 + lane] = z;
+                a += z * z;
             }
         }
-        coop_block_partial(uw, p1);
-        coop_block_partial(ww, p2);
-        grid.sync();
-        s2 = inv * coop_fold(p1, nb);
-        const double w2 = coop_fold(p2, nb);
-        if (sqrt(fmax(w2 - s2 * s2, 0.0)) < tol)
+        const double alpha = grid_sum<NW>(a, S, sh);
+        if (L.A_long.n > 0) {
+            long_partials<true>(L.A_long, L.A_ci, L.A_v, L.z, gw, nw, lane);
+            grid_barrier(S);
+        }
+        a = 0.0;
+        for (int t = gw; t < (L.m + 31) / 32; t += nw) {
+            const int r0 = 32 * t, nr = min(32, L.m - r0);
+            double r[1];
+            warp_stream_rows<1, true>(L.A_rp, L.A_ci, L.A_v, L.z, r0, nr, lane, stage, r, L.A_long);
+            if (lane < nr) {
+                const int i = r0 + lane;
+                const double prev = j > 0 ? beta * inv_prev * __ldcg(up + i) : 0.0;
+                const double w = (r[0] - prev) - alpha * inv * __ldcg(u + i);
+                up[i] = w;
+                a += w * w;
+            }
+        }
+        const double b = sqrt(grid_sum<NW>(a, S, sh));
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            L.out[4 + j] = alpha;
+            L.out[4 + LANCZOS_MAX + j] = b;
+        }
+        last = fmax(last, alpha);
+        if (!(b > 1e-14 * last)) { // the Krylov space is exhausted: T is exact
+            ++j;
             break;
-        inv = 1.0 / sqrt(w2);
-        double *t = u;
-        u = w;
-        w = t;
+        }
+        beta = b;
+        inv_prev = inv;
+        inv = 1.0 / b;
     }
-    if (tid == 0) {
-        out[0] = sqrt(s2);
-        out[1] = (double)it;
+    grid_end(S);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        L.out[0] = inv;
+        L.out[1] = inv_prev;
+        L.out[2] = beta;
+        L.out[3] = (double)j;
     }
 }
 

@@ -280,6 +280,7 @@ struct DevCsr {
     double *v = nullptr;
     LongRows lr{}; // rows of more than LONG_ROW entries, cut into segments (n = 0: none)
     long long long_nnz = 0; // entries in those rows
+    int max_row = 0;        // the longest of them
 };
 
 // The long rows of M and their segments.  A count on the device decides
@@ -300,24 +301,60 @@ void build_long_rows(DevCsr &M, Arena &ar, cudaStream_t s)
     std::vector<int> rp(M.rows + 1);
     CK(cudaMemcpyAsync(rp.data(), M.rp, rp.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    std::vector<int> rows, first{0};
+    std::vector<int> rows, first{0}, index(M.rows, -1);
     std::vector<int2> seg;
     M.long_nnz = 0;
+    // The segment length that fills whole rounds of the pass's resident warps
+    // (a warp takes a segment; 5450 segments of 4096 entries over 3552 warps ran
+    // half of the second round empty): the shortest multiple of 128, at least
+    // 512, whose segments fit the rounds that segments of LONG_SEG need.
+    const int warps = WARPS * resident_blocks((const void *)long_partials_kernel<double, double>);
+    auto count_segs = [&](int len) {
+        long long c = 0;
+        for (int r = 0; r < M.rows; ++r)
+            if (rp[r + 1] - rp[r] > LONG_ROW)
+                c += (rp[r + 1] - rp[r] + len - 1) / len;
+        return c;
+    };
+    int seg_len = LONG_SEG;
+    {
+        const long long full = count_segs(LONG_SEG), rounds = (full + warps - 1) / warps;
+        int lo = 512; // shorter ones only add partials
+        if (count_segs(lo) <= rounds * warps) {
+            seg_len = lo;
+        } else if (rounds <= 8) {
+            int hi = LONG_SEG; // lo's segments do not fit `rounds` rounds, hi's do
+            while (hi - lo > 128) {
+                const int mid = (lo + hi) / 256 * 128;
+                if (count_segs(mid) <= rounds * warps)
+                    hi = mid;
+                else
+                    lo = mid;
+            }
+            seg_len = hi;
+        }
+    }
     for (int r = 0; r < M.rows; ++r) {
         if (rp[r + 1] - rp[r] <= LONG_ROW)
             continue;
         M.long_nnz += rp[r + 1] - rp[r];
+        M.max_row = std::max(M.max_row, rp[r + 1] - rp[r]);
+        index[r] = (int)rows.size();
         rows.push_back(r);
-        for (int b = rp[r]; b < rp[r + 1]; b += LONG_SEG)
-            seg.push_back(make_int2(b, std::min(rp[r + 1], b + LONG_SEG)));
+        for (int b = rp[r]; b < rp[r + 1]; b += seg_len)
+            seg.push_back(make_int2(b, std::min(rp[r + 1], b + seg_len)));
         first.push_back((int)seg.size());
     }
     M.lr.rows = ar.upload(rows.data(), rows.size(), s);
+    M.lr.index = ar.upload(index.data(), index.size(), s);
     M.lr.seg_first = ar.upload(first.data(), first.size(), s);
     M.lr.seg = ar.upload(seg.data(), seg.size(), s);
     M.lr.part = ar.alloc<double>(seg.size());
     M.lr.n = (int)rows.size();
     M.lr.nseg = (int)seg.size();
+    int *seg_col = ar.alloc<int>(seg.size());
+    long_seg_col_kernel<<<grid_for(M.lr.nseg, WARPS), TPB, 0, s>>>(M.lr, M.ci, seg_col);
+    M.lr.seg_col = seg_col;
     CK(cudaStreamSynchronize(s)); // the host tables go out of scope
 }
 
@@ -741,6 +778,9 @@ private:
     void rescale();
     void init_state();
     void step_size();
+    double power_sigma2(double *v0);
+    GridSlots make_slots(int blocks, int values);
+    void check_slots(const GridSlots &S, const char *what);
     void loop();
     void enqueue_step(bool store_primal, bool store_dual, bool want_fpe, double w);
     void enqueue_step_bb(bool store_dual, bool want_fpe, double w);
@@ -938,6 +978,15 @@ void Solve::upload_and_preprocess()
     free_d_ = dp_.free_d;
 }
 
+// a set-up pass over M's long rows, by warps or by blocks
+#define PDHCG_LONG(kernel, M, ...)                                                                                     \
+    do {                                                                                                               \
+        if (M.long_nnz <= (long long)LONG_WARP_MEAN * M.lr.n)                                                          \
+            kernel<true><<<grid_for(M.lr.n, WARPS), TPB, 0, s>>>(M.lr, __VA_ARGS__);                                   \
+        else                                                                                                           \
+            kernel<false><<<std::min(M.lr.n, 148 * 16), TPB, 0, s>>>(M.lr, __VA_ARGS__);                               \
+    } while (0)
+
 // ---- rescaling (reference rescale_problem, src/preconditioner.c:654-713) --
 void Solve::rescale()
 {
@@ -955,9 +1004,9 @@ void Solve::rescale()
         scale_csr_kernel<<<grid_for(m, TPB), TPB, 0, s>>>(A_.rp, A_.ci, A_.v, m, fcr, fvr, 0, A_.lr.n > 0);
         scale_csr_kernel<<<grid_for(n, TPB), TPB, 0, s>>>(At_.rp, At_.ci, At_.v, n, fvr, fcr, 1, At_.lr.n > 0);
         if (A_.lr.n > 0)
-            long_scale_csr_kernel<<<std::min(A_.lr.n, 148 * 16), TPB, 0, s>>>(A_.lr, A_.rp, A_.ci, A_.v, fcr, fvr, 0);
+            PDHCG_LONG(long_scale_csr_kernel, A_, A_.rp, A_.ci, A_.v, fcr, fvr, 0);
         if (At_.lr.n > 0)
-            long_scale_csr_kernel<<<std::min(At_.lr.n, 148 * 16), TPB, 0, s>>>(At_.lr, At_.rp, At_.ci, At_.v, fvr,
+            PDHCG_LONG(long_scale_csr_kernel, At_, At_.rp, At_.ci, At_.v, fvr,
                                                                              fcr, 1);
         if (Q_.nnz > 0)
             scale_csr_kernel<<<grid_for(n, TPB), TPB, 0, s>>>(Q_.rp, Q_.ci, Q_.v, n, fvr, fvr, 0, 0);
@@ -1016,9 +1065,9 @@ void Solve::rescale()
         row_absmax_kernel<<<grid_for(m, TPB), TPB, 0, s>>>(A_.rp, A_.v, m, fcr, A_.lr.n > 0);
         row_absmax_kernel<<<grid_for(n, TPB), TPB, 0, s>>>(At_.rp, At_.v, n, fvr, At_.lr.n > 0);
         if (A_.lr.n > 0)
-            long_row_absmax_kernel<<<std::min(A_.lr.n, 148 * 16), TPB, 0, s>>>(A_.lr, A_.rp, A_.v, fcr);
+            PDHCG_LONG(long_row_absmax_kernel, A_, A_.rp, A_.v, fcr);
         if (At_.lr.n > 0)
-            long_row_absmax_kernel<<<std::min(At_.lr.n, 148 * 16), TPB, 0, s>>>(At_.lr, At_.rp, At_.v, fvr);
+            PDHCG_LONG(long_row_absmax_kernel, At_, At_.rp, At_.v, fvr);
         apply(1);
     }
     if (prm_.has_pock_chambolle_alpha) {
@@ -1026,15 +1075,15 @@ void Solve::rescale()
         row_powsum_kernel<<<grid_for(m, TPB), TPB, 0, s>>>(A_.rp, A_.v, m, a, fcr, A_.lr.n > 0);
         row_powsum_kernel<<<grid_for(n, TPB), TPB, 0, s>>>(At_.rp, At_.v, n, 2.0 - a, fvr, At_.lr.n > 0);
         if (A_.lr.n > 0)
-            long_row_powsum_kernel<<<std::min(A_.lr.n, 148 * 16), TPB, 0, s>>>(A_.lr, A_.rp, A_.v, a, fcr);
+            PDHCG_LONG(long_row_powsum_kernel, A_, A_.rp, A_.v, a, fcr);
         if (At_.lr.n > 0)
-            long_row_powsum_kernel<<<std::min(At_.lr.n, 148 * 16), TPB, 0, s>>>(At_.lr, At_.rp, At_.v, 2.0 - a, fvr);
+            PDHCG_LONG(long_row_powsum_kernel, At_, At_.rp, At_.v, 2.0 - a, fvr);
         apply(0);
     }
     if (prm_.bound_objective_rescaling) {
         int nb = grid_for((long long)n + m, TPB, 148 * 4);
         norms_kernel<<<nb, TPB, 0, s>>>(n, m, c_d_, lc_d_, uc_d_, g_d_, partials_);
-        fold_partials_kernel<<<1, TPB, 0, s>>>(partials_, nb, NS_COUNT, norm_ops_d_, scal_d_);
+        fold_partials_kernel<<<NS_COUNT, TPB, 0, s>>>(partials_, nb, NS_COUNT, norm_ops_d_, scal_d_);
         double h[NS_COUNT];
         CK(cudaMemcpyAsync(h, scal_d_, sizeof(h), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
@@ -1254,6 +1303,123 @@ void Solve::enqueue_q_apply(const double *v, double *qx)
     stats_.kernel_launches++;
 }
 
+// arrival counter and partials of the persistent kernels (gridsum.cuh)
+GridSlots Solve::make_slots(int blocks, int values)
+{
+    GridSlots S{};
+    S.stride = blocks * values;
+    S.part = ar_.alloc<double>(2 * (size_t)S.stride);
+    S.state = ar_.alloc<unsigned long long>(3);
+    S.err = (int *)(S.state + 2);
+    CK(cudaMemsetAsync(S.state, 0, 3 * sizeof(unsigned long long), st_));
+    return S;
+}
+
+void Solve::check_slots(const GridSlots &S, const char *what)
+{
+    int bad = 0;
+    CK(cudaMemcpyAsync(&bad, S.err, sizeof(int), cudaMemcpyDeviceToHost, st_));
+    CK(cudaStreamSynchronize(st_));
+    if (bad)
+        throw CudaError(std::string("a wait of the blocks for one another ran out (") + what + ")");
+}
+
+// What the power method on A A^T from v0 returns (reference
+// estimate_maximum_singular_value, src/pdhg_core_op.cu:1673-1788: Rayleigh
+// quotients of the normalised iterates until the residual |A A^T v - s2 v| is
+// below sv_tol), from a few Lanczos steps.
+//
+// The iterates of the power method stay in the Krylov space of v0, where A
+// A^T is the tridiagonal T of its Lanczos process: its k-th Rayleigh
+// quotient and residual are those of k power steps with T on the first unit
+// vector, exactly while k is below half the order, and to rounding once T
+// holds the top of the spectrum (a Gauss quadrature of the moments v0' (A
+// A^T)^p v0).  So the products with A are done j times for T, and the
+// hundreds of power steps on the host with a j x j tridiagonal.  The order
+// grows by LANCZOS_CHUNK until two orders agree on the iteration that stops
+// and on its value to 1e-13.  On a scaled random A the power method takes 180
+// to 1250 iterations and T 32 to 112 steps, with the same stopping iteration
+// and a value 1e-15 to 1e-12 apart.
+static double power_on_tridiagonal(const std::vector<double> &al, const std::vector<double> &be, int max_iter,
+                                   double tol, int &its)
+{
+    const int j = (int)al.size();
+    std::vector<double> u(j, 0.0), w(j);
+    u[0] = 1.0;
+    double s2 = 1.0;
+    for (its = 0; its < max_iter; ++its) {
+        s2 = 0.0;
+        for (int i = 0; i < j; ++i) {
+            w[i] = al[i] * u[i] + (i > 0 ? be[i - 1] * u[i - 1] : 0.0) + (i + 1 < j ? be[i] * u[i + 1] : 0.0);
+            s2 += u[i] * w[i];
+        }
+        double r2 = 0.0, w2 = 0.0;
+        for (int i = 0; i < j; ++i) {
+            r2 += (w[i] - s2 * u[i]) * (w[i] - s2 * u[i]);
+            w2 += w[i] * w[i];
+        }
+        if (std::sqrt(r2) < tol || !(w2 > 0.0))
+            break;
+        const double inv = 1.0 / std::sqrt(w2);
+        for (int i = 0; i < j; ++i)
+            u[i] = w[i] * inv;
+    }
+    return s2;
+}
+
+double Solve::power_sigma2(double *v0)
+{
+    cudaStream_t s = st_;
+    const int m = m_, n = n_, max_iter = prm_.sv_max_iter;
+    if (max_iter < 1)
+        return 1.0;
+    CK(cudaFuncSetAttribute((const void *)lanczos_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LANCZOS_SMEM));
+    const int limit = std::min(LANCZOS_MAX, std::min(m, 2 * max_iter) + 1); // steps at which T is exact or given up
+    int dev = 0, nsm = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    const int grid = std::max(1, std::min(nsm, (std::max(m, n) + LANCZOS_TPB - 1) / LANCZOS_TPB));
+    LanczosData L{};
+    L.m = m;
+    L.n = n;
+    L.A_rp = A_.rp;
+    L.A_ci = A_.ci;
+    L.A_v = A_.v;
+    L.At_rp = At_.rp;
+    L.At_ci = At_.ci;
+    L.At_v = At_.v;
+    L.A_long = A_.lr;
+    L.At_long = At_.lr;
+    L.u[0] = v0;
+    L.u[1] = ar_.alloc<double>(m);
+    L.z = ar_.alloc<double>(n);
+    L.out = ar_.alloc<double>(2 * LANCZOS_MAX + 4);
+    GridSlots S = make_slots(grid, 1);
+    std::vector<double> al, be, h;
+    double s2 = 1.0, last = -1.0;
+    int its = 0, last_its = -1;
+    for (int j = 0; j < limit;) {
+        int steps = std::min(j == 0 ? 2 * LANCZOS_CHUNK : LANCZOS_CHUNK, limit - j);
+        void *args[] = {&L, &S, &j, &steps};
+        CK(cudaLaunchCooperativeKernel((const void *)lanczos_kernel, grid, LANCZOS_TPB, args, LANCZOS_SMEM, s));
+        stats_.kernel_launches++;
+        j += steps;
+        h.resize(4 + 2 * (size_t)LANCZOS_MAX);
+        CK(cudaMemcpyAsync(h.data(), L.out, h.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        check_slots(S, "Lanczos process");
+        const int have = (int)h[3]; // fewer than j: the Krylov space is exhausted
+        al.assign(h.begin() + 4, h.begin() + 4 + have);
+        be.assign(h.begin() + 4 + LANCZOS_MAX, h.begin() + 4 + LANCZOS_MAX + have);
+        s2 = power_on_tridiagonal(al, be, max_iter, prm_.sv_tol, its);
+        if (have < j || 2 * its + 1 < have || (its == last_its && std::fabs(s2 - last) <= 1e-13 * s2))
+            break;
+        last = s2;
+        last_its = its;
+    }
+    return s2;
+}
+
 // ---- step size (reference initialize_step_size_and_primal_weight,
 // src/pdhg_core_op.cu:933-971) -------------------------------------------
 void Solve::step_size()
@@ -1269,24 +1435,7 @@ void Solve::step_size()
         unsigned int seed = 1234;
         for (int i = 0; i < m; ++i)
             v0[i] = ((double)rand_r(&seed) / (double)RAND_MAX) * 2.0 - 1.0;
-        double *v = ar_.upload(v0.data(), m, s), *nv = ar_.alloc<double>(m), *dp = ar_.alloc<double>(n);
-        double *out = ar_.alloc<double>(2);
-        int dev = 0, nsm = 0, per_sm = 0;
-        CK(cudaGetDevice(&dev));
-        CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, power_sigma_kernel<double>, TPB, 0));
-        int grid = std::max(1, std::min(nsm * std::max(per_sm, 1), nsm * 4));
-        double *part = ar_.alloc<double>((size_t)4 * grid);
-        int max_iter = prm_.sv_max_iter;
-        double tol = prm_.sv_tol;
-        LongRows al = A_.lr, atl = At_.lr;
-        void *args[] = {&m, &n, &A_.rp, &A_.ci, &A_.v, &At_.rp, &At_.ci, &At_.v, &v, &nv, &dp, &part, &max_iter,
-                        &tol, &out, &al, &atl};
-        CK(cudaLaunchCooperativeKernel((void *)power_sigma_kernel<double>, grid, TPB, args, 0, s));
-        double h[2];
-        CK(cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        double sv = h[0];
+        const double sv = std::sqrt(power_sigma2(ar_.upload(v0.data(), m, s)));
         step_ = sv < 1e-12 ? 1.0 : 0.998 / sv;
     }
     omega_ = prm_.bound_objective_rescaling ? 1.0 : (cnorm_ + 1.0) / (bnorm_ + 1.0);
@@ -1680,7 +1829,7 @@ void Solve::enqueue_residual_t(bool want_dist)
     P.sb = sb_;
     int nb = D.rows_blocks + D.free_blocks + D.cone_blocks + D.aff_blocks;
     launch_residual(D, P, std::max(S_, dp_.S_aff), dp_.has_fixed, nb, s);
-    fold_partials_kernel<<<1, TPB, 0, s>>>(partials_, nb, RS_COUNT, res_ops_d_, scal_d_);
+    fold_partials_kernel<<<RS_COUNT, TPB, 0, s>>>(partials_, nb, RS_COUNT, res_ops_d_, scal_d_);
     stats_.kernel_launches += 2;
     stats_.evaluations++;
 }
@@ -1699,7 +1848,7 @@ void Solve::enqueue_fpe(int slot)
         fpe_kernel<double><<<nb, TPB, 0, s>>>(n_, m_, At_.rp, At_.ci, At_.v, dx_, dy_, part, fpe_col_blocks_,
                                               At_.lr);
     }
-    fold_partials_kernel<<<1, TPB, 0, s>>>(part, nb, FP_COUNT, fpe_ops_d_, scal_d_ + RS_COUNT + slot * FP_COUNT);
+    fold_partials_kernel<<<FP_COUNT, TPB, 0, s>>>(part, nb, FP_COUNT, fpe_ops_d_, scal_d_ + RS_COUNT + slot * FP_COUNT);
     stats_.kernel_launches += 2;
     if (bb_) {
         bb_tol_update_kernel<<<1, 1, 0, s>>>(scal_d_ + RS_COUNT + slot * FP_COUNT + FP_DX2, step_, omega_, bb_min_tol_,
@@ -1721,7 +1870,7 @@ void Solve::compute_infeasibility()
         ray_project_kernel<float><<<nb, TPB, 0, s>>>(n_, m_, f_.dx, f_.dy, l_d_, u_d_, lc_d_, uc_d_, partials_);
     else
         ray_project_kernel<double><<<nb, TPB, 0, s>>>(n_, m_, dx_, dy_, l_d_, u_d_, lc_d_, uc_d_, partials_);
-    fold_partials_kernel<<<1, TPB, 0, s>>>(partials_, nb, RN_COUNT, rayn_ops_d_, ray_d_);
+    fold_partials_kernel<<<RN_COUNT, TPB, 0, s>>>(partials_, nb, RN_COUNT, rayn_ops_d_, ray_d_);
     if (fp32_)
         ray_scale_kernel<float><<<grid_for(n_, TPB), TPB, 0, s>>>(n_, f_.dx, ray_d_);
     else
@@ -1763,7 +1912,7 @@ void Solve::compute_infeasibility()
         long_pass(At_, At_.v, dy_);
         ray_kernel<double><<<grid, TPB, 0, s>>>(D, dx_, dy_);
     }
-    fold_partials_kernel<<<1, TPB, 0, s>>>(partials_, grid, RY_COUNT, ray_ops_d_, ray_d_ + RN_COUNT);
+    fold_partials_kernel<<<RY_COUNT, TPB, 0, s>>>(partials_, grid, RY_COUNT, ray_ops_d_, ray_d_ + RN_COUNT);
     stats_.kernel_launches += 6;
     double h[RN_COUNT + RY_COUNT];
     CK(cudaMemcpyAsync(h, ray_d_, sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -2265,7 +2414,7 @@ pdhcg_result_t *Solve::run()
     {
         int nb = grid_for((long long)n_ + m_, TPB, 148 * 4);
         norms_kernel<<<nb, TPB, 0, st_>>>(n_, m_, c_d_, lc_d_, uc_d_, g_d_, partials_);
-        fold_partials_kernel<<<1, TPB, 0, st_>>>(partials_, nb, NS_COUNT, norm_ops_d_, scal_d_);
+        fold_partials_kernel<<<NS_COUNT, TPB, 0, st_>>>(partials_, nb, NS_COUNT, norm_ops_d_, scal_d_);
         double h[NS_COUNT];
         CK(cudaMemcpyAsync(h, scal_d_, sizeof(h), cudaMemcpyDeviceToHost, st_));
         CK(cudaStreamSynchronize(st_));
