@@ -225,7 +225,7 @@ int pdhcg_b200_csr_spmv(int rows, const int *row_ptr, const int *col_ind, const 
  * exponential blocks, power blocks (exponents in cone_alpha, which may be
  * NULL without power blocks) and PSD blocks of order v_dim <= 22 (svec
  * packing, projected in the plain Frobenius metric as the reference does:
- * d and q do not enter; 2 v_dim^2 doubles of temporary scratch each); -3
+ * d and q do not enter; 2 v_dim^2 + v_dim + 1 doubles of temporary scratch each); -3
  * for a power block without cone_alpha or an unknown type, -2 for a longer
  * block.  Waits for the stream (it reads the block lengths on the host). */
 int pdhcg_b200_project_cones(int num_cones, const int *cone_start, const int *cone_vdim, const int *cone_type,

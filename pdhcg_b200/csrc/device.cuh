@@ -892,18 +892,19 @@ __device__ inline void exp_cone_point(double r1, double r2, double r3, double d1
 // quadratics, on the point scaled by its largest magnitude.
 //
 // The reference halves the bracket 80 times.  Each halving is a serial chain
-// of an exp, two hypots, two square roots and two logs, and with one lane at
-// work those 80 chains set the length of the launch (100 us a step on 60
-// such blocks).  The warp instead tests 32 points of the bracket at once and
-// keeps the interval between the last point below the root and the first
-// above it: a factor of 33 per round, so 13 rounds narrow log DBL_MIN ..
-// log |z| past the resolution of a double (708 / 33^13 < 2e-17), the same
-// root to its last bits.  The search also ends when a round cannot narrow it.
+// of an exp, square roots and two logs, and with one lane at work those 80
+// chains set the length of the launch (76 us on 60 such blocks).  The warp
+// instead tests 32 points of the bracket at once and keeps the interval
+// between the last point below the root and the first above it, a factor of
+// 33: four rounds narrow log DBL_MIN .. log |z| to 6e-4, from where Newton's
+// method on the same function (kept inside the bracket) reaches the
+// resolution of a double in about three steps.  If it has not after eight,
+// further rounds narrow the bracket past it.
 __device__ inline double pow_pos_root(double r, double q)
 {
     if (!(q > 0.0))
         return fmax(r, 0.0);
-    const double disc = hypot(r, 2.0 * sqrt(q));
+    const double disc = sqrt(r * r + 4.0 * q); // |r| <= 1: the point is scaled
     return r >= 0.0 ? 0.5 * (r + disc) : (2.0 * q) / (disc - r);
 }
 
@@ -945,7 +946,8 @@ __device__ inline void pow_cone_point(double rx, double ry, double rz, double wx
         oz = 0.0;
         return;
     }
-    for (int it = 0; it < 13; ++it) {
+    // one round: 32 points, the bracket a 33rd
+    auto narrow = [&]() {
         const double w = (hi - lo) * (1.0 / 33.0);
         const double lr = lo + w * (lane + 1), rho = exp(lr);
         const double x = pow_pos_root(rx, 0.25 * cx * rho * (az - rho));
@@ -954,12 +956,47 @@ __device__ inline void pow_cone_point(double rx, double ry, double rz, double wx
         const unsigned above = ~__ballot_sync(FULL, below);
         const int c = above ? __ffs(above) - 1 : 32; // points below the root
         const double l2 = c > 0 ? lo + w * c : lo, h2 = c < 32 ? lo + w * (c + 1) : hi;
-        if (!(h2 - l2 < hi - lo))
-            break;
+        const bool moved = h2 - l2 < hi - lo;
         lo = l2;
         hi = h2;
+        return moved;
+    };
+    bool more = true;
+    for (int it = 0; more && it < 4; ++it)
+        more = narrow();
+    // Newton on f(lr) = a log x + om log y - lr, every lane alike
+    double lr = lo + 0.5 * (hi - lo);
+    bool done = false;
+    for (int it = 0; more && !done && it < 8; ++it) {
+        const double rho = exp(lr), qs = 0.25 * rho * (az - rho), dq = 0.25 * rho * (az - 2.0 * rho);
+        const double x = pow_pos_root(rx, cx * qs), y = pow_pos_root(ry, cy * qs);
+        if (!(x > 0.0 && y > 0.0 && qs > 0.0))
+            break;
+        const double f = a * log(x) + om * log(y) - lr;
+        if (f > 0.0)
+            lo = lr;
+        else
+            hi = lr;
+        // x' = cx dq / (2 x - rx): x^2 - rx x = cx qs
+        const double df = a * cx * dq / ((2.0 * x - rx) * x) + om * cy * dq / ((2.0 * y - ry) * y) - 1.0;
+        const double nx = lr - f / df;
+        if (!(nx > lo && nx < hi)) {
+            // outside the bracket: at the resolution of lr the bracket has closed on it
+            done = fabs(f / df) <= 4.0 * DBL_EPSILON * (1.0 + fabs(lr));
+            if (!done && !isfinite(nx))
+                break;
+            lr = done ? lr : lo + 0.5 * (hi - lo);
+            continue;
+        }
+        done = fabs(nx - lr) <= 4.0 * DBL_EPSILON * (1.0 + fabs(lr));
+        lr = nx;
     }
-    const double rho = exp(lo + 0.5 * (hi - lo));
+    if (!done) {
+        for (int it = 0; more && it < 13; ++it)
+            more = narrow();
+        lr = lo + 0.5 * (hi - lo);
+    }
+    const double rho = exp(lr);
     const double x = pow_pos_root(rx, 0.25 * cx * rho * (az - rho));
     const double y = pow_pos_root(ry, 0.25 * cy * rho * (az - rho));
     ox = x * s;
@@ -1038,16 +1075,18 @@ constexpr int PSD_MAX_ORDER = 22;
 constexpr int PSD_MAX_SWEEPS = 100;
 constexpr double PSD_OFF_REL = 1e-28;
 
-// (row, col) of svec slot i of an order-n block
+// (row, col) of svec slot i of an order-n block: column c starts at slot
+// c n - c (c - 1) / 2
 __device__ __forceinline__ void psd_slot_rc(int i, int n, int &row, int &col)
 {
-    int c = 0, first = 0;
-    while (i >= first + (n - c)) {
-        first += n - c;
+    const float b = 2.0f * (float)n + 1.0f;
+    int c = max(0, min(n - 1, (int)((b - sqrtf(fmaxf(b * b - 8.0f * (float)i, 0.0f))) * 0.5f)));
+    while (c > 0 && i < c * n - c * (c - 1) / 2)
+        --c;
+    while (i >= (c + 1) * n - (c + 1) * c / 2)
         ++c;
-    }
     col = c;
-    row = c + (i - first);
+    row = c + (i - (c * n - c * (c - 1) / 2));
 }
 
 // Scratch of one block in doubles: A, the eigenvectors (V^T, one per row),
@@ -1055,6 +1094,106 @@ __device__ __forceinline__ void psd_slot_rc(int i, int n, int &row, int &col)
 __host__ __device__ constexpr long long psd_work_doubles(long long order)
 {
     return 2 * order * order + 2 * ((order + 1) / 2);
+}
+
+// Rotation for a pair: the tangent of the smaller angle that annihilates a_pq
+// is t = a2 / (h + sign(h) sqrt(h^2 + a2^2)), h = a_qq - a_pp, a2 = 2 a_pq.
+// The rounds are chains of these angles, and FP64 square roots and divisions
+// are a few hundred cycles each, so t is formed in FP32 on the pair scaled by
+// its larger magnitude (a power of two), and only the cosine, which makes
+// (c, t c) a rotation to FP64 rounding, in FP64: 1 / sqrt(1 + t^2) by two
+// Newton steps from its FP32 value (errors 1e-7, 1e-14, below rounding).  An
+// angle 1e-7 off leaves 1e-7 of a_pq behind, which is kept, not set to zero;
+// the next sweep takes it.
+__device__ __forceinline__ void jacobi_angle(double app, double aqq, double apq, double &c, double &sn)
+{
+    c = 1.0;
+    sn = 0.0;
+    const double h = aqq - app, a2 = 2.0 * apq, mag = fmax(fabs(h), fabs(a2));
+    if (!(mag > 0.0) || !(mag < 8e307)) // nothing to rotate (or out of range)
+        return;
+    // 2^-e with e the exponent of mag (a subnormal pair is left as it is)
+    const int e = (int)((__double_as_longlong(mag) >> 52) & 0x7ff);
+    if (e < 2 || e > 2045)
+        return;
+    const double scale = __longlong_as_double((long long)(2046 - e) << 52);
+    const float hf = (float)(h * scale), af = (float)(a2 * scale);
+    const float tf = af / (hf + copysignf(sqrtf(hf * hf + af * af), hf));
+    const double t = (double)tf, r = fma(t, t, 1.0);
+    double y = (double)rsqrtf((float)r);
+    y = y * fma(-0.5 * r * y, y, 1.5);
+    y = y * fma(-0.5 * r * y, y, 1.5);
+    c = y;
+    sn = t * y;
+}
+
+// pair i of round r over m players: {m - 1, r}, then {r + i, r - i} modulo m - 1
+__device__ __forceinline__ void jacobi_pair(int m, int r, int i, int &p, int &q)
+{
+    int a = m - 1, b = r;
+    if (i > 0) {
+        a = r + i;
+        b = r - i;
+        if (a >= m - 1)
+            a -= m - 1;
+        if (b < 0)
+            b += m - 1;
+    }
+    p = min(a, b);
+    q = max(a, b);
+}
+
+// (i, j), i <= j, of index t of the upper triangle, columns in order
+__device__ __forceinline__ void jacobi_block(int t, int &i, int &j)
+{
+    j = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while ((j + 1) * (j + 2) / 2 <= t)
+        ++j;
+    while (j * (j + 1) / 2 > t)
+        --j;
+    i = t - j * (j + 1) / 2;
+}
+
+// A <- J' A J on the rows of pair i and the columns of pair j (i <= j; an
+// index n is the bye of an odd order) and on the mirror image
+__device__ __forceinline__ void jacobi_update(double *A, int n, int m, int r, int i, int j, const double *cs)
+{
+    int pi, qi, pj, qj;
+    jacobi_pair(m, r, i, pi, qi);
+    jacobi_pair(m, r, j, pj, qj);
+    const double ci = cs[2 * i], si = cs[2 * i + 1], cj = cs[2 * j], sj = cs[2 * j + 1];
+    const bool fi = qi < n, fj = qj < n;
+    const double app = A[(size_t)pi * n + pj], apq = fj ? A[(size_t)pi * n + qj] : 0.0;
+    const double aqp = fi ? A[(size_t)qi * n + pj] : 0.0, aqq = fi && fj ? A[(size_t)qi * n + qj] : 0.0;
+    // columns by pair j, then rows by pair i
+    const double bpp = cj * app - sj * apq, bpq = sj * app + cj * apq;
+    const double bqp = cj * aqp - sj * aqq, bqq = sj * aqp + cj * aqq;
+    const double dpp = ci * bpp - si * bqp, dqp = si * bpp + ci * bqp;
+    const double dpq = ci * bpq - si * bqq, dqq = si * bpq + ci * bqq;
+    if (i == j) { // the rotated pair itself
+        A[(size_t)pi * n + pi] = dpp;
+        if (fi) {
+            const double off = 0.5 * (dpq + dqp); // what the angle's rounding left
+            A[(size_t)qi * n + qi] = dqq;
+            A[(size_t)pi * n + qi] = off;
+            A[(size_t)qi * n + pi] = off;
+        }
+        return;
+    }
+    A[(size_t)pi * n + pj] = dpp;
+    A[(size_t)pj * n + pi] = dpp;
+    if (fj) {
+        A[(size_t)pi * n + qj] = dpq;
+        A[(size_t)qj * n + pi] = dpq;
+    }
+    if (fi) {
+        A[(size_t)qi * n + pj] = dqp;
+        A[(size_t)pj * n + qi] = dqp;
+    }
+    if (fi && fj) {
+        A[(size_t)qi * n + qj] = dqq;
+        A[(size_t)qj * n + qi] = dqq;
+    }
 }
 
 // Diagonalises the symmetric n x n matrix A (full, row-major) in place by
@@ -1066,20 +1205,6 @@ __device__ inline void warp_jacobi(double *A, double *Vt, double *cs, int n, int
         Vt[e] = (e / n == e % n) ? 1.0 : 0.0;
     __syncwarp();
     const int m = n + (n & 1), np = m / 2; // odd n: index n is a bye
-    // pair i of round r: {m - 1, r}, then {r + i, r - i} modulo m - 1
-    auto pair_of = [&](int r, int i, int &p, int &q) {
-        int a = m - 1, b = r;
-        if (i > 0) {
-            a = r + i;
-            b = r - i;
-            if (a >= m - 1)
-                a -= m - 1;
-            if (b < 0)
-                b += m - 1;
-        }
-        p = min(a, b);
-        q = max(a, b);
-    };
     for (int sweep = 0; sweep < PSD_MAX_SWEEPS; ++sweep) {
         double off = 0.0, all = 0.0;
         for (int r = 0; r < n; ++r)
@@ -1096,70 +1221,22 @@ __device__ inline void warp_jacobi(double *A, double *Vt, double *cs, int n, int
         for (int r = 0; r < m - 1; ++r) {
             for (int i = lane; i < np; i += 32) {
                 int p, q;
-                pair_of(r, i, p, q);
+                jacobi_pair(m, r, i, p, q);
                 double c = 1.0, sn = 0.0;
-                if (q < n) {
-                    const double apq = A[(size_t)p * n + q];
-                    if (apq != 0.0) {
-                        const double theta = (A[(size_t)q * n + q] - A[(size_t)p * n + p]) / (2.0 * apq);
-                        const double t = fabs(theta) > 1e150
-                                             ? 0.5 / theta
-                                             : (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-                        c = 1.0 / sqrt(t * t + 1.0);
-                        sn = t * c;
-                    }
-                }
+                if (q < n)
+                    jacobi_angle(A[(size_t)p * n + p], A[(size_t)q * n + q], A[(size_t)p * n + q], c, sn);
                 cs[2 * i] = c;
                 cs[2 * i + 1] = sn;
             }
             __syncwarp();
-            // 2 x 2 blocks (i, j), i <= j, and their mirror images
             for (int t = lane; t < np * (np + 1) / 2; t += 32) {
-                int j = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
-                while ((j + 1) * (j + 2) / 2 <= t)
-                    ++j;
-                while (j * (j + 1) / 2 > t)
-                    --j;
-                const int i = t - j * (j + 1) / 2;
-                int pi, qi, pj, qj;
-                pair_of(r, i, pi, qi);
-                pair_of(r, j, pj, qj);
-                const double ci = cs[2 * i], si = cs[2 * i + 1], cj = cs[2 * j], sj = cs[2 * j + 1];
-                const bool fi = qi < n, fj = qj < n; // false: the bye's partner, one row or column
-                const double app = A[(size_t)pi * n + pj], apq = fj ? A[(size_t)pi * n + qj] : 0.0;
-                const double aqp = fi ? A[(size_t)qi * n + pj] : 0.0, aqq = fi && fj ? A[(size_t)qi * n + qj] : 0.0;
-                // columns by pair j, then rows by pair i
-                const double bpp = cj * app - sj * apq, bpq = sj * app + cj * apq;
-                const double bqp = cj * aqp - sj * aqq, bqq = sj * aqp + cj * aqq;
-                const double dpp = ci * bpp - si * bqp, dqp = si * bpp + ci * bqp;
-                double dpq = ci * bpq - si * bqq, dqq = si * bpq + ci * bqq;
-                if (i == j) { // the rotated pair itself
-                    A[(size_t)pi * n + pi] = dpp;
-                    if (fi) {
-                        A[(size_t)qi * n + qi] = dqq;
-                        A[(size_t)pi * n + qi] = 0.0;
-                        A[(size_t)qi * n + pi] = 0.0;
-                    }
-                } else {
-                    A[(size_t)pi * n + pj] = dpp;
-                    A[(size_t)pj * n + pi] = dpp;
-                    if (fj) {
-                        A[(size_t)pi * n + qj] = dpq;
-                        A[(size_t)qj * n + pi] = dpq;
-                    }
-                    if (fi) {
-                        A[(size_t)qi * n + pj] = dqp;
-                        A[(size_t)pj * n + qi] = dqp;
-                    }
-                    if (fi && fj) {
-                        A[(size_t)qi * n + qj] = dqq;
-                        A[(size_t)qj * n + qi] = dqq;
-                    }
-                }
+                int i, j;
+                jacobi_block(t, i, j);
+                jacobi_update(A, n, m, r, i, j, cs);
             }
             for (int j = 0; j < np; ++j) {
                 int p, q;
-                pair_of(r, j, p, q);
+                jacobi_pair(m, r, j, p, q);
                 if (q >= n)
                     continue;
                 const double c = cs[2 * j], sn = cs[2 * j + 1];
@@ -1170,6 +1247,80 @@ __device__ inline void warp_jacobi(double *A, double *Vt, double *cs, int n, int
                 }
             }
             __syncwarp();
+        }
+    }
+}
+
+// The same by a block of NT threads, A, Vt and cs in its shared memory; red:
+// 2 NT / 32 doubles.  A round's work is spread so thin over the warps (order
+// 20: 10 angles, 55 blocks, 200 rotated eigenvector entries) that its length
+// is one angle and one update's latency.
+template <int NT>
+__device__ inline void cta_jacobi(double *A, double *Vt, double *cs, double *red, int n)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int e = tid; e < n * n; e += NT)
+        Vt[e] = (e / n == e % n) ? 1.0 : 0.0;
+    const int m = n + (n & 1), np = m / 2, nblk = np * (np + 1) / 2, nv = np * n;
+    int i0 = 0, j0 = 0; // this thread's first block and eigenvector entry
+    if (tid < nblk)
+        jacobi_block(tid, i0, j0);
+    const int vj0 = tid / n, vk0 = tid - vj0 * n;
+    __syncthreads();
+    for (int sweep = 0; sweep < PSD_MAX_SWEEPS; ++sweep) {
+        double off = 0.0, all = 0.0;
+        for (int e = tid; e < n * n; e += NT) {
+            const double a2 = A[e] * A[e];
+            all += a2;
+            if (e / n != e % n)
+                off += a2;
+        }
+        off = warp_sum(off);
+        all = warp_sum(all);
+        if (lane == 0) {
+            red[2 * warp] = off;
+            red[2 * warp + 1] = all;
+        }
+        __syncthreads();
+        off = all = 0.0;
+        for (int w = 0; w < NT / 32; ++w) {
+            off += red[2 * w];
+            all += red[2 * w + 1];
+        }
+        if (!(off > PSD_OFF_REL * all))
+            break;
+        for (int r = 0; r < m - 1; ++r) {
+            for (int i = tid; i < np; i += NT) {
+                int p, q;
+                jacobi_pair(m, r, i, p, q);
+                double c = 1.0, sn = 0.0;
+                if (q < n)
+                    jacobi_angle(A[p * n + p], A[q * n + q], A[p * n + q], c, sn);
+                cs[2 * i] = c;
+                cs[2 * i + 1] = sn;
+            }
+            __syncthreads();
+            for (int t = tid; t < nv; t += NT) {
+                int j = vj0, k = vk0;
+                if (t != tid) {
+                    j = t / n;
+                    k = t - j * n;
+                }
+                int p, q;
+                jacobi_pair(m, r, j, p, q);
+                if (q < n) {
+                    const double c = cs[2 * j], sn = cs[2 * j + 1], vp = Vt[p * n + k], vq = Vt[q * n + k];
+                    Vt[p * n + k] = c * vp - sn * vq;
+                    Vt[q * n + k] = sn * vp + c * vq;
+                }
+            }
+            for (int t = tid; t < nblk; t += NT) {
+                int i = i0, j = j0;
+                if (t != tid)
+                    jacobi_block(t, i, j);
+                jacobi_update(A, n, m, r, i, j, cs);
+            }
+            __syncthreads();
         }
     }
 }

@@ -71,6 +71,7 @@ struct StepData {
     LongRows A_long, At_long; // long rows of A (pass over x_refl) and of A^T (pass over y)
     double *psd_work;         // PSD blocks' projection scratch (NULL: no PSD blocks)
     const long long *psd_off; // per cone block: offset of its scratch in psd_work
+    int psd_max;              // largest order of a PSD block
     // affine cones F x + g in K over blocks of rows: the rows outside them as
     // tiles of <= 32 consecutive rows {first, count} (NULL: all rows in tiles
     // of 32), and the blocks themselves (projected with d = 1 / cr)
@@ -280,6 +281,79 @@ __device__ __noinline__ void primal_psd_long_block(const StepData<T> &D, const S
     __syncwarp();
 }
 
+// One PSD block per thread block, its matrix, eigenvectors and rotations in
+// shared memory: A^T y and the prox candidate by warps of 32 slots, the
+// decomposition by the whole block, then the projection, reflection and
+// Halpern average slot by slot.  The blocks of a problem are few and their
+// decompositions long chains of small rounds, so a warp on global scratch
+// (each rotation's stores and loads through L2) left the step at 600 us for 38
+// blocks of orders 2 to 20; this takes 110 to 150.
+template <typename T, bool HAS_Q, int NT>
+__global__ void __launch_bounds__(NT) psd_step_kernel(StepData<T> D, StepParams P, const int *ids, int nids)
+{
+    extern __shared__ double psd_dyn[];
+    __shared__ double stage_all[NT / 32][STREAM_CHUNK], red[2 * NT / 32];
+    __shared__ int bad;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double R2 = 1.41421356237309504880, IR2 = 0.70710678118654752440;
+    for (int ib = blockIdx.x; ib < nids; ib += gridDim.x) {
+        const int cb = ids ? ids[ib] : ib, st = D.cone_start[cb], L = D.cone_len[cb], n = psd_order(L);
+        double *A = psd_dyn, *Vt = A + n * n, *cs = Vt + n * n;
+        if (tid == 0)
+            bad = 0;
+        __syncthreads();
+        for (int c0 = 32 * warp; c0 < L; c0 += NT) {
+            const int nr = min(32, L - c0);
+            double aty[1];
+            warp_stream_rows<1>(D.At_rp, D.At_ci, D.At_v, D.y, st + c0, nr, lane, stage_all[warp], aty, D.At_long);
+            if (lane < nr) {
+                const int j = st + c0 + lane;
+                double t = (double)D.x[j] - P.tau * ((double)D.c[j] - aty[0]);
+                if (HAS_Q)
+                    t /= 1.0 + P.tau * (double)D.q[j];
+                const double xc = P.cone_box ? clampd(D.l[j], t, D.u[j]) : t;
+                if (P.lp_slack)
+                    D.dual_slack[j] = (T)((xc - t) / P.tau);
+                int row, col;
+                psd_slot_rc(c0 + lane, n, row, col);
+                const double v = row == col ? xc : xc * IR2;
+                A[row * n + col] = v;
+                A[col * n + row] = v;
+                if (!isfinite(xc))
+                    bad = 1;
+            }
+        }
+        __syncthreads();
+        const bool nan = bad != 0; // the reference's failed decomposition gives NaN
+        if (!nan && n > 1)
+            cta_jacobi<NT>(A, Vt, cs, red, n);
+        for (int i = tid; i < L; i += NT) {
+            const int j = st + i;
+            double p;
+            if (nan) {
+                p = __longlong_as_double(0x7ff8000000000000LL);
+            } else if (n == 1) {
+                p = fmax(A[0], 0.0);
+            } else {
+                int row, col;
+                psd_slot_rc(i, n, row, col);
+                double v = 0.0;
+                for (int e = 0; e < n; ++e)
+                    v += fmax(A[e * n + e], 0.0) * Vt[e * n + row] * Vt[e * n + col];
+                p = row == col ? v : v * R2;
+            }
+            const double xi = D.x[j], xr = 2.0 * p - xi;
+            D.xr[j] = (T)xr;
+            D.xp[j] = (T)p;
+            if (P.want_fpe)
+                D.dx[j] = (T)(xr - xi);
+            const double refl = P.rho * xr + (1.0 - P.rho) * xi;
+            D.x[j] = (T)(P.w * refl + (1.0 - P.w) * (double)D.x0[j]);
+        }
+        __syncthreads(); // the matrix is read
+    }
+}
+
 // One warp per cone block of the list ids (NULL: blocks 0 .. nids - 1);
 // KINDS = CONES_WIDE for SOC / RSOC blocks, CONES_THREE (S = 1) for the
 // 3-slot exponential and power blocks, CONES_PSD for PSD blocks (those
@@ -302,6 +376,38 @@ __global__ void __launch_bounds__(TPB) primal_cone_kernel(StepData<T> D, StepPar
         }
         primal_cone_block<S, T, HAS_Q, KINDS>(D, P, cb, lane, stage);
     }
+}
+
+// The free variables, the SOC / RSOC blocks and the 3-slot blocks of a problem
+// in one launch, block ranges [0, fb), [fb, fb + wb) and the rest: on a
+// problem that fills only a part of the device the three launches run one
+// after the other for the length of their longest chains (5 + 9 + 23 us on
+// 2000 free variables, 260 cones and 120 3-slot blocks), here side by side.
+template <int S, typename T, bool HAS_Q>
+__global__ void __launch_bounds__(TPB) primal_mixed_kernel(StepData<T> D, StepParams P, int fb, const int *wide,
+                                                           int n_wide, int wb, const int *three, int n_three)
+{
+    __shared__ double stage_all[WARPS][STREAM_CHUNK];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    double *stage = stage_all[wib];
+    int b = blockIdx.x;
+    if (b < fb) {
+        for (int t = b * WARPS + wib; t < D.n_free_tiles; t += fb * WARPS) {
+            const int2 ft = D.free_tiles[t];
+            primal_free_tile<T, HAS_Q, true>(D, P, ft.x, ft.y, lane, stage);
+        }
+        return;
+    }
+    b -= fb;
+    if (b < wb) {
+        for (int i = b * WARPS + wib; i < n_wide; i += wb * WARPS)
+            primal_cone_block<S, T, HAS_Q, CONES_WIDE>(D, P, wide ? wide[i] : i, lane, stage);
+        return;
+    }
+    b -= wb;
+    const int tb = gridDim.x - fb - wb;
+    for (int i = b * WARPS + wib; i < n_three; i += tb * WARPS)
+        primal_cone_block<1, T, HAS_Q, CONES_THREE>(D, P, three ? three[i] : i, lane, stage);
 }
 
 // One tile of 32 consecutive rows of A: A x_refl by stream-mode products,

@@ -139,8 +139,13 @@ template <typename T>
 void launch_primal_free(const StepData<T> &D, const StepParams &P, bool hasq, bool box_free, int grid, cudaStream_t s);
 // cone blocks of the primal step; returns the number of launches
 template <typename T>
-int launch_primal_cones(const StepData<T> &D, const StepParams &P, const ConeSplit &sp, int S, bool hasq,
+int launch_primal_cones(const StepData<T> &D, const StepParams &P, const ConeSplit &sp, int S, bool hasq, bool mixed,
                         cudaStream_t s);
+// free variables, SOC / RSOC and 3-slot blocks in one launch; false: not for
+// this problem
+template <typename T>
+bool launch_primal_mixed(const StepData<T> &D, const StepParams &P, const ConeSplit &sp, int S, bool hasq,
+                         cudaStream_t s);
 template <typename T>
 void launch_dual_cones(const StepData<T> &D, const StepParams &P, int S, cudaStream_t s);
 template <typename T>
@@ -150,6 +155,14 @@ void launch_dual_rows(const StepData<T> &D, const StepParams &P, bool eq_rows, b
 template <typename VT>
 void launch_residual(const ResidualData<VT> &D, const ResidualParams &P, int S, bool fixed, int blocks,
                      cudaStream_t s);
+
+// the variables' PSD blocks of the residual, a thread block each, partials
+// from row `first` on; fits: whether a block of this order fits in one's shared
+// memory
+bool residual_psd_fits(int order);
+template <typename VT>
+void launch_residual_psd(const ResidualData<VT> &D, const ResidualParams &P, const int *ids, int nids, int max_order,
+                         int first, int blocks, cudaStream_t s);
 
 // inner.cu: the inner BB solve and the Q apply (G lanes per row of Q, S
 // slots per lane of a cone block)

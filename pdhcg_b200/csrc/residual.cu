@@ -1,19 +1,12 @@
-// residual.cu -- the residual kernel (residual.cuh) and its launcher.
-#include "launch.cuh"
+// residual.cu -- the residual kernels with FP64 iterates.
+#include "residual_impl.cuh"
 
 namespace pdhcg {
 
-template <typename VT>
-void launch_residual(const ResidualData<VT> &D, const ResidualParams &P, int S, bool fixed, int blocks, cudaStream_t s)
-{
-    if (fixed) // one slot class for problems with fixed cone slots
-        residual_kernel<8, VT, true><<<blocks, TPB, 0, s>>>(D, P);
-    else
-        dispatch_s(S, [&](auto SC) { residual_kernel<SC.value, VT, false><<<blocks, TPB, 0, s>>>(D, P); });
-}
+bool residual_psd_fits(int order) { return residual_psd_smem(order) <= 190 * 1024; }
 
-template void launch_residual<double>(const ResidualData<double> &, const ResidualParams &, int, bool, int,
+template void launch_residual<double>(const ResidualData<double> &, const ResidualParams &, int, bool, int, cudaStream_t);
+template void launch_residual_psd<double>(const ResidualData<double> &, const ResidualParams &, const int *, int, int, int, int,
                                       cudaStream_t);
-template void launch_residual<float>(const ResidualData<float> &, const ResidualParams &, int, bool, int, cudaStream_t);
 
 } // namespace pdhcg

@@ -69,6 +69,8 @@ struct ResidualData {
     LongRows A_long, At_long; // passes over x_pdhg and y_pdhg
     double *psd_work;         // PSD blocks' projection scratch (NULL: none)
     const long long *psd_off;
+    int psd_separate; // the variables' PSD blocks are taken by residual_psd_kernel
+    int psd_shared; // doubles of dynamic shared memory per warp: the scratch of the blocks held in registers
     // affine cone blocks of rows and the rows outside them (tiles; NULL: all)
     const int2 *row_tiles;
     int n_row_tiles;
@@ -77,6 +79,15 @@ struct ResidualData {
     const long long *aff_psd_off;
     int n_aff, aff_blocks;
 };
+
+// this warp's part of the dynamic shared memory: PSD blocks held in registers
+// are diagonalised there (in global scratch every rotation's stores and loads
+// went to L2: 2 ms for the two projections of a block of order 20)
+__device__ __forceinline__ double *residual_psd_scratch(int doubles)
+{
+    extern __shared__ double residual_dyn[];
+    return residual_dyn + (size_t)(threadIdx.x >> 5) * doubles;
+}
 
 __device__ __forceinline__ double norm_term(double v, int l2) { return l2 ? v * v : abs_or_inf(v); }
 
@@ -136,7 +147,7 @@ __device__ __forceinline__ void residual_cone_block(const ResidualData<VT> &D, c
             fold(RS_CONE_COMPL, norm_term(cplx, P.l2));
     } else {
     bool uni = warp_uniform_unit<S>(aug, L, lane); // d uniform <=> 1/d uniform
-    double *psd = D.psd_work ? D.psd_work + D.psd_off[cb] : nullptr;
+    double *psd = type == 4 ? residual_psd_scratch(D.psd_shared) : nullptr;
     if (type == 0 || type == 1 || type == 4) {
         // self-dual: projection onto the dual cone in the 1/d metric
         // (PSD: without a metric, as the reference projects it)
@@ -299,7 +310,7 @@ __device__ __forceinline__ void residual_affine_block(const ResidualData<VT> &D,
     auto fold = [&](int s, double v) { acc[s] = ops[s] == RMAX ? fmax(acc[s], v) : acc[s] + v; };
     const int st = D.aff_start[ab], L = D.aff_len[ab], type = D.aff_type[ab];
     const double alpha = D.aff_alpha ? D.aff_alpha[ab] : 0.0;
-    double *psd = D.psd_work ? D.psd_work + D.aff_psd_off[ab] : nullptr;
+    double *psd = type == 4 ? residual_psd_scratch(D.psd_shared) : nullptr;
     double axr[S];
     warp_stream_rows<S>(D.A_rp, D.A_ci, D.A_v, D.xp, st, L, lane, stage, axr, D.A_long);
     WarpSlots<S> pv, mv;
@@ -452,6 +463,8 @@ __global__ void __launch_bounds__(TPB) residual_kernel(ResidualData<VT> D, Resid
             // 3-slot blocks (exponential, power) take the one-slot
             // instantiation, which alone carries their projection
             const int ct = D.cone_type[cb];
+            if (ct == 4 && D.psd_separate)
+                continue;
             if (SECT && D.cone_fixed[cb]) {
                 if (S > 1 && (ct == 2 || ct == 3))
                     residual_cone_block<1, VT, true>(D, P, cb, lane, stage, acc, ops);
@@ -477,6 +490,99 @@ __global__ void __launch_bounds__(TPB) residual_kernel(ResidualData<VT> D, Resid
         }
     }
     block_reduce_store<RS_COUNT>(acc, ops, D.partials);
+}
+
+// The terms of residual_cone_block for PSD blocks, one per thread block: the
+// two projections (dual cone and augmented point, no metric) by the whole
+// block in shared memory, a long chain of small rounds that a warp takes
+// several times as long for.  Partials of block b at row first + b.
+template <typename VT>
+__global__ void __launch_bounds__(TPB) residual_psd_kernel(ResidualData<VT> D, ResidualParams P, const int *ids, int nids,
+                                                           int first)
+{
+    extern __shared__ double psd_dyn[];
+    __shared__ double stage_all[WARPS][STREAM_CHUNK], red[2 * WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double R2 = 1.41421356237309504880, IR2 = 0.70710678118654752440;
+    const int NOP = P.l2 ? RSUM : RMAX;
+    const int ops[RS_COUNT] = {NOP, RSUM, NOP, RSUM, RSUM, RSUM, NOP, NOP, RSUM, RSUM, NOP, NOP, NOP, NOP, NOP};
+    double acc[RS_COUNT];
+#pragma unroll
+    for (int s = 0; s < RS_COUNT; ++s)
+        acc[s] = 0.0;
+    auto fold = [&](int s, double v) { acc[s] = ops[s] == RMAX ? fmax(acc[s], v) : acc[s] + v; };
+    auto qx_of = [&](int j, double x) { return P.qmode == 1 ? D.q[j] * x : (P.qmode == 2 ? D.qx[j] : 0.0); };
+    for (int ib = blockIdx.x; ib < nids; ib += gridDim.x) {
+        const int cb = ids[ib], st = D.cone_start[cb], L = D.cone_len[cb], n = psd_order(L);
+        double *A = psd_dyn, *Vt = A + n * n, *cs = Vt + n * n, *aty = cs + 2 * ((n + 1) / 2), *rcp = aty + L,
+               *augp = rcp + L;
+        __syncthreads(); // the previous block's vectors are read
+        for (int c0 = 32 * warp; c0 < L; c0 += TPB) {
+            const int nr = min(32, L - c0);
+            double a[1];
+            warp_stream_rows<1>(D.At_rp, D.At_ci, D.At_v, D.yp, st + c0, nr, lane, stage_all[warp], a, D.At_long);
+            if (lane < nr) {
+                const int j = st + c0 + lane;
+                const double x = D.xp[j], rc = (P.qmode ? D.c[j] + qx_of(j, x) : D.c[j]) - a[0];
+                aty[c0 + lane] = a[0];
+                rcp[c0 + lane] = rc;
+                augp[c0 + lane] = clampd(D.l[j], x - P.s_aug * rc, D.u[j]);
+            }
+        }
+        for (int which = 0; which < 2; ++which) { // v <- its projection
+            double *v = which ? augp : rcp;
+            int fin = 1;
+            __syncthreads();
+            for (int i = tid; i < L; i += TPB) {
+                int row, col;
+                psd_slot_rc(i, n, row, col);
+                fin &= isfinite(v[i]) != 0;
+                const double e = row == col ? v[i] : v[i] * IR2;
+                A[row * n + col] = e;
+                A[col * n + row] = e;
+            }
+            const bool ok = __syncthreads_and(fin) != 0; // else NaN, as the reference's failed decomposition
+            if (ok && n > 1)
+                cta_jacobi<TPB>(A, Vt, cs, red, n);
+            for (int i = tid; i < L; i += TPB) {
+                if (!ok) {
+                    v[i] = __longlong_as_double(0x7ff8000000000000LL);
+                } else if (n == 1) {
+                    v[i] = fmax(v[i], 0.0);
+                } else {
+                    int row, col;
+                    psd_slot_rc(i, n, row, col);
+                    double p = 0.0;
+                    for (int e = 0; e < n; ++e)
+                        p += fmax(A[e * n + e], 0.0) * Vt[e * n + row] * Vt[e * n + col];
+                    v[i] = row == col ? p : p * R2;
+                }
+            }
+        }
+        __syncthreads();
+        for (int i = tid; i < L; i += TPB) {
+            const int j = st + i;
+            const double x = D.xp[j], qx = qx_of(j, x), vr = D.vr[j];
+            const double rc = (P.qmode ? D.c[j] + qx : D.c[j]) - aty[i];
+            double dr = (rc - rcp[i]) * vr;
+            double rr = (x - augp[i]) / P.s_aug * vr;
+            if (!isfinite(rr))
+                rr = copysign(INFINITY, rr);
+            if (fabs(rr) > fabs(dr))
+                dr = rr;
+            fold(RS_DUAL_RES, norm_term(dr, P.l2));
+            fold(RS_CX, D.c[j] * x);
+            fold(RS_XQX, x * qx);
+            fold(RS_SLACKX, rc * x);
+            fold(RS_QX_NORM, norm_term(qx * vr, P.l2));
+            fold(RS_ATY_NORM, norm_term(aty[i] * vr, P.l2));
+            if (P.want_dist) {
+                const double d = x - (double)D.x0[j];
+                fold(RS_DIST_X, d * d);
+            }
+        }
+    }
+    block_reduce_store<RS_COUNT>(acc, ops, D.partials + (size_t)first * RS_COUNT);
 }
 
 // Fixed-point error pieces (reference compute_fixed_point_error,

@@ -430,7 +430,10 @@ struct DeviceProblem {
     long long *apsd_off_d = nullptr;
     int2 *row_tiles_d = nullptr;
     int n_row_tiles = 0, S_aff = 1;
-    std::vector<long long> psd_off; // per cone block: offset of its PSD scratch (2 n^2 doubles)
+    int *psd_ids = nullptr;     // the variables' PSD blocks
+    int n_psd_blocks = 0;
+    int psd_max = 0, psd_max_short = 0; // largest order of a variable PSD block; of a block held in registers
+    std::vector<long long> psd_off; // per cone block: offset of its PSD scratch
     long long psd_total = 0;
     long long *psd_off_d = nullptr;
     int2 *free_tiles = nullptr; // free variables as tiles of consecutive rows
@@ -630,6 +633,9 @@ std::unique_ptr<DeviceProblem> make_device_problem(const qp_problem_t *p, cudaSt
             // registers of a warp do not hold (any order)
             d.has_psd = true;
             d.var_psd = true;
+            d.psd_max = std::max(d.psd_max, p->cones.v_dim[b]);
+            if (len <= 32 * 8)
+                d.psd_max_short = std::max(d.psd_max_short, p->cones.v_dim[b]);
             d.psd_total += psd_scratch_doubles(p->cones.v_dim[b], len > 32);
         }
         d.cone_alpha.push_back(p->cones.power_alpha ? p->cones.power_alpha[b] : 0.0);
@@ -678,6 +684,15 @@ std::unique_ptr<DeviceProblem> make_device_problem(const qp_problem_t *p, cudaSt
             d.split.place(ar.upload(all.data(), all.size(), s));
             CK(cudaStreamSynchronize(s));
         }
+        if (d.var_psd) { // PSD blocks of the variables (no fixed slots among them)
+            std::vector<int> ids;
+            for (int b = 0; b < nc; ++b)
+                if (d.cone_type[b] == CONE_PSD)
+                    ids.push_back(b);
+            d.n_psd_blocks = (int)ids.size();
+            d.psd_ids = ar.upload(ids.data(), ids.size(), s);
+            CK(cudaStreamSynchronize(s));
+        }
         if (d.has_psd) {
             d.psd_off_d = ar.upload(d.psd_off.data(), nc, s);
             CK(cudaStreamSynchronize(s));
@@ -709,6 +724,7 @@ std::unique_ptr<DeviceProblem> make_device_problem(const qp_problem_t *p, cudaSt
                 if (vd > PSD_MAX_ORDER)
                     d.unsupported = "affine PSD blocks of order above 22 are not supported yet";
                 d.has_psd = true;
+                d.psd_max_short = std::max(d.psd_max_short, std::min(vd, PSD_MAX_ORDER));
                 d.psd_total += psd_work_doubles(vd);
             }
             amax = std::max(amax, len);
@@ -843,7 +859,7 @@ private:
            *g_d_ = nullptr, *cr_d_ = nullptr, *vr_d_ = nullptr;
     int *free_d_ = nullptr, *cst_d_ = nullptr, *clen_d_ = nullptr, *ctype_d_ = nullptr, *cvdim_d_ = nullptr;
     double *cone_warm_ = nullptr, *warm_dual_ = nullptr, *warm_aug_ = nullptr; // per-cone multipliers
-    double *psd_work_ = nullptr; // PSD blocks' eigen-decomposition scratch (2 n^2 doubles each)
+    double *psd_work_ = nullptr; // PSD blocks' eigen-decomposition scratch
     double *x0_, *x_, *xp_, *xr_, *dx_, *dslack_, *y0_, *y_, *yp_, *dy_;
     // FP32 mirrors of the matrices, problem vectors and iterates (mixed precision)
     struct {
@@ -863,7 +879,7 @@ private:
     // infeasibility certificates of the last computation (zero until then)
     double p_ray_obj_ = 0.0, d_ray_obj_ = 0.0, max_p_ray_ = 0.0, max_d_ray_ = 0.0;
     void compute_infeasibility();
-    int res_rows_blocks_ = 0, res_free_blocks_ = 0, res_cone_blocks_ = 0, res_aff_blocks_ = 0;
+    int res_rows_blocks_ = 0, res_free_blocks_ = 0, res_cone_blocks_ = 0, res_aff_blocks_ = 0, res_psd_blocks_ = 0;
     int fpe_col_blocks_ = 0, fpe_row_blocks_ = 0;
 
     // scaling
@@ -1488,6 +1504,7 @@ StepData<T> Solve::step_data()
     D.cone_alpha = dp_.calpha;
     D.psd_work = psd_work_;
     D.psd_off = dp_.psd_off_d;
+    D.psd_max = dp_.psd_max;
     D.n_cones = (int)cone_start_.size();
     if constexpr (std::is_same<T, double>::value) {
         D.A_v = A_.v;
@@ -1665,14 +1682,17 @@ void Solve::enqueue_step_t(bool store_primal, bool store_dual, bool want_fpe, do
     long_pass(At_, D.At_v, D.y); // A^T y of both primal kernels
     bool hasq = qtype_ == PDHCG_DIAG_Q;
     int nfree = D.n_cones > 0 ? D.n_free : n_;
-    if (nfree > 0) {
+    const bool mixed = D.n_cones > 0 && launch_primal_mixed(D, P, dp_.split, S_, hasq, s);
+    if (mixed)
+        stats_.kernel_launches++;
+    if (nfree > 0 && !mixed) {
         int ntiles = D.free_tiles ? D.n_free_tiles : (n_ + 31) / 32;
         int grid = grid_for(ntiles, WARPS);
         launch_primal_free(D, P, hasq, box_free_, grid, s);
         stats_.kernel_launches++;
     }
     if (D.n_cones > 0)
-        stats_.kernel_launches += launch_primal_cones(D, P, dp_.split, S_, hasq, s);
+        stats_.kernel_launches += launch_primal_cones(D, P, dp_.split, S_, hasq, mixed, s);
     launch_dual<T>(D, P);
     stats_.step_kernel_launches++;
     step_bytes_sum_ += step_bytes(sizeof(T), store_primal || !cone_start_.empty(), store_dual);
@@ -1791,6 +1811,7 @@ void Solve::enqueue_residual_t(bool want_dist)
     D.cone_alpha = dp_.calpha;
     D.psd_work = psd_work_;
     D.psd_off = dp_.psd_off_d;
+    D.psd_shared = dp_.psd_max_short > 0 ? (int)psd_work_doubles(dp_.psd_max_short) : 0;
     D.n_cones = (int)cone_start_.size();
     D.partials = partials_;
     D.rows_blocks = res_rows_blocks_;
@@ -1828,7 +1849,14 @@ void Solve::enqueue_residual_t(bool want_dist)
     P.s_aug = sa;
     P.sb = sb_;
     int nb = D.rows_blocks + D.free_blocks + D.cone_blocks + D.aff_blocks;
+    const int psd_blocks = res_psd_blocks_;
+    if (psd_blocks > 0) { // partials behind the others'
+        launch_residual_psd(D, P, dp_.psd_ids, dp_.n_psd_blocks, dp_.psd_max, nb, psd_blocks, s);
+        stats_.kernel_launches++;
+        D.psd_separate = 1;
+    }
     launch_residual(D, P, std::max(S_, dp_.S_aff), dp_.has_fixed, nb, s);
+    nb += psd_blocks;
     fold_partials_kernel<<<RS_COUNT, TPB, 0, s>>>(partials_, nb, RS_COUNT, res_ops_d_, scal_d_);
     stats_.kernel_launches += 2;
     stats_.evaluations++;
@@ -2323,9 +2351,10 @@ void Solve::setup_scratch()
     if (!cone_start_.empty() && free_idx_.empty())
         res_free_blocks_ = 0;
     res_cone_blocks_ = cone_start_.empty() ? 0 : grid_for((long long)cone_start_.size(), WARPS, 148 * 8);
+    res_psd_blocks_ = dp_.n_psd_blocks > 0 && residual_psd_fits(dp_.psd_max) ? grid_for(dp_.n_psd_blocks, 1) : 0;
     fpe_col_blocks_ = grid_for(((long long)n_ + 31) / 32, WARPS, 148 * 8);
     fpe_row_blocks_ = grid_for(m_, TPB, 148 * 4);
-    int maxb = std::max({res_rows_blocks_ + res_free_blocks_ + res_cone_blocks_ + res_aff_blocks_,
+    int maxb = std::max({res_rows_blocks_ + res_free_blocks_ + res_cone_blocks_ + res_aff_blocks_ + res_psd_blocks_,
                          fpe_col_blocks_ + fpe_row_blocks_,
                          res_rows_blocks_ + fpe_col_blocks_, 148 * 4});
     partials_ = ar_.alloc<double>((size_t)maxb * RS_COUNT);
@@ -2538,7 +2567,7 @@ int step_impl(StepData<double> D, StepParams P, const pdhcg_b200_step_t *t, cuda
         launch_primal_free(D, P, hasq, false, grid, s);
     }
     if (nc > 0)
-        launch_primal_cones(D, P, split, S, hasq, s);
+        launch_primal_cones(D, P, split, S, hasq, false, s);
     int dgrid = grid_for(((long long)t->m + 31) / 32, WARPS);
     launch_dual_rows(D, P, false, t->affine_offset != nullptr, dgrid, s);
     CK(cudaGetLastError());

@@ -3,6 +3,8 @@
 
 namespace pdhcg {
 
+constexpr size_t PSD_STEP_SMEM = 200 * 1024;
+
 template <typename T>
 void launch_primal_free(const StepData<T> &D, const StepParams &P, bool hasq, bool box_free, int grid, cudaStream_t s)
 {
@@ -20,13 +22,14 @@ void launch_primal_free(const StepData<T> &D, const StepParams &P, bool hasq, bo
 }
 
 // Primal step over the cone blocks: the SOC / RSOC blocks with S slots per
-// lane, the 3-slot blocks with one; returns the number of launches.
+// lane, the 3-slot blocks with one (mixed: both are done already); returns the
+// number of launches.
 template <typename T>
-int launch_primal_cones(const StepData<T> &D, const StepParams &P, const ConeSplit &sp, int S, bool hasq,
+int launch_primal_cones(const StepData<T> &D, const StepParams &P, const ConeSplit &sp, int S, bool hasq, bool mixed,
                         cudaStream_t s)
 {
     int launches = 0;
-    if (sp.n_wide > 0) {
+    if (sp.n_wide > 0 && !mixed) {
         // no more blocks than are resident at once: each warp then walks
         // several cone blocks and the warps drift apart, so one warp's
         // projection arithmetic overlaps other warps' loads (a full grid
@@ -45,7 +48,7 @@ int launch_primal_cones(const StepData<T> &D, const StepParams &P, const ConeSpl
         });
         ++launches;
     }
-    if (sp.n_three > 0) {
+    if (sp.n_three > 0 && !mixed) {
         int grid = grid_for(sp.n_three, WARPS);
         if (hasq)
             primal_cone_kernel<1, T, true, CONES_THREE><<<grid, TPB, 0, s>>>(D, P, sp.three_d, sp.n_three);
@@ -54,13 +57,34 @@ int launch_primal_cones(const StepData<T> &D, const StepParams &P, const ConeSpl
         ++launches;
     }
     if (sp.n_psd > 0) { // LP path only: diagonal Q with PSD blocks takes the inner BB solve
-        dispatch_s(S, [&](auto SC) {
-            int grid = grid_for(sp.n_psd, WARPS);
-            if (hasq)
-                primal_cone_kernel<SC.value, T, true, CONES_PSD><<<grid, TPB, 0, s>>>(D, P, sp.psd_d, sp.n_psd);
-            else
-                primal_cone_kernel<SC.value, T, false, CONES_PSD><<<grid, TPB, 0, s>>>(D, P, sp.psd_d, sp.n_psd);
-        });
+        // a thread block per PSD block while the matrices fit in its shared
+        // memory (order 112); a warp per block on global scratch beyond
+        const size_t dyn = psd_work_doubles(D.psd_max) * sizeof(double);
+        auto go = [&](auto kernel, int threads) {
+            CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+            kernel<<<grid_for(sp.n_psd, 1), threads, dyn, s>>>(D, P, sp.psd_d, sp.n_psd);
+        };
+        if (D.psd_max > 0 && dyn <= PSD_STEP_SMEM) {
+            if (D.psd_max <= 32) {
+                if (hasq)
+                    go(psd_step_kernel<T, true, 128>, 128);
+                else
+                    go(psd_step_kernel<T, false, 128>, 128);
+            } else {
+                if (hasq)
+                    go(psd_step_kernel<T, true, 256>, 256);
+                else
+                    go(psd_step_kernel<T, false, 256>, 256);
+            }
+        } else {
+            dispatch_s(S, [&](auto SC) {
+                int grid = grid_for(sp.n_psd, WARPS);
+                if (hasq)
+                    primal_cone_kernel<SC.value, T, true, CONES_PSD><<<grid, TPB, 0, s>>>(D, P, sp.psd_d, sp.n_psd);
+                else
+                    primal_cone_kernel<SC.value, T, false, CONES_PSD><<<grid, TPB, 0, s>>>(D, P, sp.psd_d, sp.n_psd);
+            });
+        }
         ++launches;
     }
     if (sp.n_sect > 0) { // blocks with fixed slots: section projectors, one slot class (any block length)
@@ -72,6 +96,33 @@ int launch_primal_cones(const StepData<T> &D, const StepParams &P, const ConeSpl
         ++launches;
     }
     return launches;
+}
+
+// Free variables and cone blocks in one launch where their blocks are resident
+// at once with room to spare (two per SM; more would queue behind one
+// another, and the kernels of one kind are leaner).  PSD and section blocks
+// have launches of their own.  False: not for this problem, nothing launched.
+template <typename T>
+bool launch_primal_mixed(const StepData<T> &D, const StepParams &P, const ConeSplit &sp, int S, bool hasq,
+                         cudaStream_t s)
+{
+    const int kinds = (D.n_free_tiles > 0) + (sp.n_wide > 0) + (sp.n_three > 0);
+    if (kinds < 2 || !D.free_tiles && D.n_free > 0)
+        return false;
+    // a warp of its own block for every 3-slot block up to 64: their chains are the longest
+    const int fb = D.n_free > 0 ? grid_for(D.n_free_tiles, WARPS) : 0, wb = sp.n_wide > 0 ? grid_for(sp.n_wide, WARPS) : 0,
+              tb = sp.n_three > 0 ? grid_for(sp.n_three, WARPS) : 0;
+    if (fb + wb + tb > 2 * 148)
+        return false;
+    dispatch_s(sp.n_wide > 0 ? S : 1, [&](auto SC) {
+        if (hasq)
+            primal_mixed_kernel<SC.value, T, true><<<fb + wb + tb, TPB, 0, s>>>(D, P, fb, sp.wide_d, sp.n_wide, wb,
+                                                                                 sp.three_d, sp.n_three);
+        else
+            primal_mixed_kernel<SC.value, T, false><<<fb + wb + tb, TPB, 0, s>>>(D, P, fb, sp.wide_d, sp.n_wide, wb,
+                                                                                  sp.three_d, sp.n_three);
+    });
+    return true;
 }
 
 template <typename T>
@@ -100,8 +151,10 @@ void launch_dual_rows(const StepData<T> &D, const StepParams &P, bool eq_rows, b
 
 #define PDHCG_STEP(T)                                                                                                  \
     template void launch_primal_free<T>(const StepData<T> &, const StepParams &, bool, bool, int, cudaStream_t);       \
-    template int launch_primal_cones<T>(const StepData<T> &, const StepParams &, const ConeSplit &, int, bool,         \
+    template int launch_primal_cones<T>(const StepData<T> &, const StepParams &, const ConeSplit &, int, bool, bool,   \
                                         cudaStream_t);                                                                 \
+    template bool launch_primal_mixed<T>(const StepData<T> &, const StepParams &, const ConeSplit &, int, bool,        \
+                                         cudaStream_t);                                                                \
     template void launch_dual_cones<T>(const StepData<T> &, const StepParams &, int, cudaStream_t);                    \
     template void launch_dual_rows<T>(const StepData<T> &, const StepParams &, bool, bool, int, cudaStream_t);
 PDHCG_STEP(double)
