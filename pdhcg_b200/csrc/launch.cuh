@@ -13,7 +13,9 @@
 #include <vector>
 
 #include "bb.cuh"
+#include "gridsum.cuh"
 #include "internal.h"
+#include "resident.cuh"
 #include "residual.cuh"
 
 namespace pdhcg {
@@ -169,6 +171,16 @@ void launch_residual_psd(const ResidualData<VT> &D, const ResidualParams &P, con
 int bb_blocks_per_sm(int G, int S, bool fixed); // resident blocks of both kernels
 void launch_bb(int G, int S, bool fixed, int grid, const BBData &D, const BBParams &P, cudaStream_t s);
 void launch_q_apply(int G, int grid, const BBData &D, const double *v, double *qx, cudaStream_t s);
+
+// resident.cu: persistent iterations of a problem without cones
+struct ResidentPlan {
+    int blocks; // 0: not for this shape
+    int cap_a, cap_at, rows, vars; // per block: staged entries of A and A^T, rows, variables
+    size_t smem;
+};
+ResidentPlan resident_plan(int n, int m, long long nnz, int sms);
+void launch_resident(const ResidentPlan &p, const ResidentData &D, const ResidentParams &P, const GridSlots &S,
+                     cudaStream_t s);
 
 // project.cu
 struct ProjectArgs {

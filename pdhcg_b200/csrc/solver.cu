@@ -798,6 +798,14 @@ private:
     GridSlots make_slots(int blocks, int values);
     void check_slots(const GridSlots &S, const char *what);
     void loop();
+    // iterations of a problem without cones in one persistent launch (resident.cuh)
+    bool resident_ = false;
+    ResidentPlan res_plan_{};
+    ResidentState *res_state_ = nullptr, *h_res_ = nullptr;
+    GridSlots res_slots_{};
+    void setup_resident();
+    void run_resident(double elapsed);
+    void resolve_fpe(const double *r);
     void enqueue_step(bool store_primal, bool store_dual, bool want_fpe, double w);
     void enqueue_step_bb(bool store_dual, bool want_fpe, double w);
     template <typename T>
@@ -2072,17 +2080,9 @@ void Solve::leave_fp32()
     fp32_ = false;
 }
 
-// ---- main loop (reference optimize, src/solver.cu:121-170) ---------------
-void Solve::read_residual()
+// pending fixed-point errors computed since the previous read of the scalars r
+void Solve::resolve_fpe(const double *r)
 {
-    cudaStream_t s = st_;
-    CK(cudaMemcpyAsync(h_scal_, scal_d_, (RS_COUNT + 2 * FP_COUNT) * sizeof(double), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    harvest_step_events();
-    const double *r = h_scal_;
-    bool l2 = prm_.optimality_norm == NORM_TYPE_L2;
-    auto nrm = [&](double v) { return l2 ? std::sqrt(v) : v; };
-    // pending fixed-point errors computed since the previous read
     auto fpe_of = [&](const double *f) {
         double pn2 = f[FP_DX2], dn2 = f[FP_DY2], cross = f[FP_CROSS];
         double movement = pn2 * omega_ + dn2 / omega_;
@@ -2096,6 +2096,156 @@ void Solve::read_residual()
         fpe_ = fpe_of(r + RS_COUNT + pending_fpe_slot_ * FP_COUNT);
         pending_fpe_slot_ = -1;
     }
+}
+
+// ---- persistent iterations (resident.cuh) ---------------------------------
+// Problems without cones, long rows or an inner solve whose matrices fit in
+// the blocks' shared memory, in FP64.
+void Solve::setup_resident()
+{
+    resident_ = false;
+    if (bb_ || !cone_start_.empty() || !dp_.aff_start.empty() || A_.lr.n > 0 || At_.lr.n > 0 || opt_.time_steps)
+        return;
+    int dev = 0, nsm = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    res_plan_ = resident_plan(n_, m_, A_.nnz, nsm);
+    if (res_plan_.blocks == 0)
+        return;
+    cudaStream_t s = st_;
+    res_state_ = ar_.alloc<ResidentState>(1);
+    res_slots_ = make_slots(res_plan_.blocks, RESIDENT_SLOTS);
+    static_assert(sizeof(ResidentState) <= 64 * sizeof(double), "the pinned scalar block holds the state");
+    resident_ = true;
+}
+
+void Solve::run_resident(double elapsed)
+{
+    if (elapsed >= prm_.termination_criteria.time_sec_limit) // the host's next evaluation ends the solve
+        return;
+    cudaStream_t s = st_;
+    const restart_parameters_t &rp = prm_.restart_params;
+    const termination_criteria_t &tc = prm_.termination_criteria;
+    if (pending_fpe0_ || pending_fpe_slot_ >= 0) {
+        CK(cudaMemcpyAsync(h_scal_, scal_d_, (RS_COUNT + 2 * FP_COUNT) * sizeof(double), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        resolve_fpe(h_scal_);
+    }
+    ResidentData D{};
+    D.n = n_;
+    D.m = m_;
+    D.A_rp = A_.rp;
+    D.A_ci = A_.ci;
+    D.A_v = A_.v;
+    D.At_rp = At_.rp;
+    D.At_ci = At_.ci;
+    D.At_v = At_.v;
+    D.c = c_d_;
+    D.l = l_d_;
+    D.u = u_d_;
+    D.q = qtype_ == PDHCG_DIAG_Q ? q_d_ : nullptr;
+    D.lc = lc_d_;
+    D.uc = uc_d_;
+    D.g = g_d_;
+    D.vr = vr_d_;
+    D.cr = cr_d_;
+    D.x0 = x0_;
+    D.x = x_;
+    D.xp = xp_;
+    D.xr = xr_;
+    D.dx = dx_;
+    D.ds = dslack_;
+    D.y0 = y0_;
+    D.y = y_;
+    D.yp = yp_;
+    D.dy = dy_;
+    D.state = res_state_;
+    ResidentParams P{};
+    P.l2 = prm_.optimality_norm == NORM_TYPE_L2;
+    P.freq = prm_.termination_evaluation_frequency;
+    P.iteration_limit = tc.iteration_limit;
+    // hand back in time for the host to see the clock and the cancel flag
+    P.budget = RESIDENT_BUDGET;
+    P.eps_opt = tc.eps_optimal_relative;
+    P.eps_feas = tc.eps_feasible_relative;
+    P.step = step_;
+    P.nonconvexity = nonconvexity_;
+    P.rho = prm_.reflection_coefficient;
+    P.sb = sb_;
+    P.sc = sc_;
+    P.cnorm = cnorm_;
+    P.bnorm = bnorm_;
+    P.obj_const = dp_.obj_const;
+    P.artificial = rp.artificial_restart_threshold;
+    P.sufficient = rp.sufficient_reduction_for_restart;
+    P.necessary = rp.necessary_reduction_for_restart;
+    P.k_p = rp.k_p;
+    P.k_i = rp.k_i;
+    P.k_d = rp.k_d;
+    P.i_smooth = rp.i_smooth;
+    ResidentState h{};
+    h.k = k_;
+    h.inner = inner_count_;
+    h.major = is_major_;
+    h.omega = omega_;
+    h.best_omega = best_omega_;
+    h.best_gap = best_gap_;
+    h.err_sum = pw_err_sum_;
+    h.last_err = pw_last_err_;
+    h.fpe = fpe_;
+    h.fpe0 = fpe0_;
+    h.fpe_last = fpe_last_;
+    std::memcpy(h_scal_, &h, sizeof(h));
+    CK(cudaMemcpyAsync(res_state_, h_scal_, sizeof(h), cudaMemcpyHostToDevice, s));
+    launch_resident(res_plan_, D, P, res_slots_, s);
+    stats_.kernel_launches++;
+    CK(cudaMemcpyAsync(h_scal_, res_state_, sizeof(h), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    std::memcpy(&h, h_scal_, sizeof(h));
+    if (h.wait_failed)
+        check_slots(res_slots_, "persistent iteration");
+    const int steps = h.k - k_;
+    stats_.step_kernel_launches += steps;
+    stats_.restarts += h.restarts;
+    stats_.evaluations += h.evaluations;
+    step_bytes_sum_ += steps * step_bytes(sizeof(double), false, false);
+    inner_total_ += steps;
+    k_ = h.k;
+    inner_count_ = h.inner;
+    is_major_ = h.major != 0;
+    omega_ = h.omega;
+    best_omega_ = h.best_omega;
+    best_gap_ = h.best_gap;
+    pw_err_sum_ = h.err_sum;
+    pw_last_err_ = h.last_err;
+    fpe_ = h.fpe;
+    fpe0_ = h.fpe0;
+    fpe_last_ = h.fpe_last;
+    if (h.evaluations > 0) {
+        abs_p_ = h.abs_p;
+        rel_p_ = h.rel_p;
+        abs_d_ = h.abs_d;
+        rel_d_ = h.rel_d;
+        pobj_ = h.pobj;
+        dobj_ = h.dobj;
+        gap_ = h.gap;
+        rel_gap_ = h.rel_gap;
+    }
+    if (h.optimal)
+        reason_ = TERMINATION_REASON_OPTIMAL;
+}
+
+// ---- main loop (reference optimize, src/solver.cu:121-170) ---------------
+void Solve::read_residual()
+{
+    cudaStream_t s = st_;
+    CK(cudaMemcpyAsync(h_scal_, scal_d_, (RS_COUNT + 2 * FP_COUNT) * sizeof(double), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    harvest_step_events();
+    const double *r = h_scal_;
+    bool l2 = prm_.optimality_norm == NORM_TYPE_L2;
+    auto nrm = [&](double v) { return l2 ? std::sqrt(v) : v; };
+    resolve_fpe(r);
     // compute_residual scalars (reference src/pdhg_core_op.cu:1169-1293)
     abs_p_ = nrm(r[RS_PRIMAL_RES]) / sb_;
     double lin_abs_p = abs_p_;
@@ -2144,6 +2294,15 @@ void Solve::loop()
     CK(cudaEventRecord(e0, st_));
     auto t0 = std::chrono::steady_clock::now();
     while (k_ < tc.iteration_limit) {
+        // persistent iterations up to an evaluation that is the host's; a
+        // cancelled solve ends at the host's next one
+        if (resident_ && !fp32_ && !pdhcg_b200_cancel_requested() &&
+            !(is_major_ && k_ < 3 * freq)) {
+            run_resident(std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count());
+            cum_time_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+            if (reason_ != TERMINATION_REASON_UNSPECIFIED || k_ >= tc.iteration_limit)
+                break;
+        }
         if (is_major_ || k_ == 0 || (k_ % print_frequency(k_)) == 0) {
             bool restart_check = is_major_ || k_ == 0;
             enqueue_residual(restart_check);
@@ -2466,6 +2625,7 @@ pdhcg_result_t *Solve::run()
     bb_ = qtype_ != PDHCG_NON_Q && (qtype_ != PDHCG_DIAG_Q || dp_.var_psd);
     if (bb_)
         setup_bb();
+    setup_resident();
     if (opt_.precision == PDHCG_B200_MIXED) {
         if (bb_)
             enter_bb_fp32();
