@@ -25,7 +25,8 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libpdhcg_b200.so")
 SOURCES = ["solver.cu", "steps.cu", "residual.cu", "residual_f32.cu", "inner.cu", "inner_g1.cu", "inner_g4.cu",
-           "inner_g32.cu", "resident.cu", "project.cu", "batch.cu", "mlp.cu", "api.cpp", "mps.cpp", "qcqp.cpp"]
+           "inner_g32.cu", "inner_small.cu", "inner_dense.cu", "resident.cu", "project.cu",
+           "batch.cu", "mlp.cu", "api.cpp", "mps.cpp", "qcqp.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -75,6 +75,18 @@ struct BBData {
 struct BBParams {
     double tau, w, rho;
     int want_fpe;
+    int refresh; // dense path: 0: R x follows from the last solve, 1: form it anew (x = x_init), 2: and R x_init
+};
+
+// A dense low-rank term for inner_dense.cu: R's leading `width` columns in
+// tiles of 32 columns (k x 32 values each, back to back)
+constexpr int DENSE_MAX_K = 256;
+
+struct DenseR {
+    const void *tile;
+    int tiles, width;
+    const double *qd; // diagonal of Q (NULL: no Q)
+    double *rx_state; // [2][k]: R x_init, R x between solves
 };
 
 namespace cgb = cooperative_groups;

@@ -608,6 +608,82 @@ static __global__ void __launch_bounds__(TPB) spmv_kernel(int rows, const int *r
     }
 }
 
+// y = M x for a matrix whose rows are mostly of 64 to MID_ROW_MAX entries,
+// one warp per tile of 32 rows, four rows at a time: the loads of all four
+// (128 entries of each per round) are in flight together, and one exchange
+// network of six shuffles adds the four lane sums.  Taking such rows as long
+// rows instead costs a segment pass with 20 shuffles and two dependent table
+// loads per row, the partials' trip through memory and a folding kernel:
+// 57 + 16 us against 53 us here for 2e5 rows of 102 entries (246 MB).  Rows of
+// at most LONG_ROW entries read v, the longer ones vl (FP32 copies in the
+// mixed bulk phase).
+constexpr int MID_ROW_MAX = 1024;
+
+template <typename VL>
+__global__ void __launch_bounds__(TPB) spmv_mid_kernel(int rows, const int *__restrict__ rp,
+                                                       const int *__restrict__ ci, const double *__restrict__ v,
+                                                       const VL *__restrict__ vl, const double *__restrict__ x,
+                                                       double *y)
+{
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int ntiles = (rows + 31) / 32;
+    for (int tile = blockIdx.x * WARPS + wib; tile < ntiles; tile += gridDim.x * WARPS) {
+        const int r0 = 32 * tile, nr = min(32, rows - r0);
+        const int rb = __ldg(rp + r0 + min(lane, nr)), re = __ldg(rp + r0 + min(lane + 1, nr));
+        double out = 0.0;
+        for (int i = 0; i < nr; i += 4) {
+            int b[4], e[4], longest = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) { // rows past the end are empty
+                b[u] = __shfl_sync(FULL, rb, (i + u) & 31);
+                e[u] = __shfl_sync(FULL, re, (i + u) & 31);
+                longest = max(longest, e[u] - b[u]);
+            }
+            double s[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int k0 = 0; k0 < longest; k0 += 128) {
+                int c[4][4];
+                double a[4][4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const bool lg = e[u] - b[u] > LONG_ROW;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int k = b[u] + k0 + 32 * q + lane;
+                        c[u][q] = -1;
+                        a[u][q] = 0.0;
+                        if (k < e[u]) {
+                            c[u][q] = __ldg(ci + k);
+                            a[u][q] = lg ? (double)__ldg(vl + k) : __ldg(v + k);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (c[u][q] >= 0)
+                            s[u] += a[u][q] * __ldg(x + c[u][q]);
+            }
+            // row i + u ends in the lanes with (lane >> 3) & 3 = u
+            const bool h16 = lane & 16, h8 = lane & 8;
+            double p = h16 ? s[2] : s[0], po = h16 ? s[0] : s[2];
+            double q = h16 ? s[3] : s[1], qo = h16 ? s[1] : s[3];
+            p += __shfl_xor_sync(FULL, po, 16);
+            q += __shfl_xor_sync(FULL, qo, 16);
+            double t = h8 ? q : p, to = h8 ? p : q;
+            t += __shfl_xor_sync(FULL, to, 8);
+            t += __shfl_xor_sync(FULL, t, 4);
+            t += __shfl_xor_sync(FULL, t, 2);
+            t += __shfl_xor_sync(FULL, t, 1);
+            const double mine = __shfl_sync(FULL, t, (lane & 3) << 3);
+            if ((lane >> 2) == (i >> 2))
+                out = mine;
+        }
+        if (lane < nr)
+            y[r0 + lane] = out;
+    }
+}
+
 static __global__ void cone_len_kernel(int nc, const int *vdim, const int *type, int *len)
 {
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nc; b += gridDim.x * blockDim.x) {

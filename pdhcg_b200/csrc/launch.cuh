@@ -172,6 +172,20 @@ int bb_blocks_per_sm(int G, int S, bool fixed); // resident blocks of both kerne
 void launch_bb(int G, int S, bool fixed, int grid, const BBData &D, const BBParams &P, cudaStream_t s);
 void launch_q_apply(int G, int grid, const BBData &D, const double *v, double *qx, cudaStream_t s);
 
+// inner_small.cu: sparse Q with short rows, no cones; blocks: 0 when n does
+// not fit one block per SM
+int bb_small_blocks(int n, long long nnz, int sms);
+void launch_bb_small(int n, long long nnz, int sms, int blocks, const BBData &D, const BBParams &P, const GridSlots &S,
+                     cudaStream_t s);
+
+// inner_dense.cu: dense R, diagonal Q; blocks: 0 when the shape does not fit
+int dense_tile_count(int width);
+int dense_blocks(int k, int tiles, int S, int sms);
+void dense_tiles(int k, int width, const int *rp, const double *v, int tiles, double *d, float *f, cudaStream_t s);
+void dense_qdiag(int n, const int *rp, const int *ci, const double *v, double *qd, int *bad, cudaStream_t s);
+void launch_bb_dense(int S, bool fp32, int blocks, const BBData &D, const BBParams &P, const DenseR &R,
+                     const GridSlots &G, cudaStream_t s);
+
 // resident.cu: persistent iterations of a problem without cones
 struct ResidentPlan {
     int blocks; // 0: not for this shape

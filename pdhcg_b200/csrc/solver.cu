@@ -860,8 +860,17 @@ private:
     float *Qf_ = nullptr, *Rf_ = nullptr, *Rtf_ = nullptr;
     float *Af_ = nullptr, *Atf_ = nullptr; // and of A's, A^T's values, read by the long-row passes
     long long bb_inner_fp32_ = 0;          // inner iterations taken with the FP32 values
+    // the special inner solves: sparse Q of short rows without cones
+    // (inner_small.cu), dense R with a diagonal Q (inner_dense.cu)
+    int bb_small_blocks_ = 0, bb_dense_blocks_ = 0, sms_ = 0;
+    int bb_refresh_ = 1; // BBParams.refresh of the next dense solve
+    GridSlots bb_slots_{};
+    DenseR bb_dense_{};
+    double *Rtile_ = nullptr;
+    float *Rtilef_ = nullptr;
     BBData bb_data() const;
     void setup_bb();
+    void setup_bb_special(int nsm);
     void enqueue_q_apply(const double *v, double *qx);
     double *c_d_ = nullptr, *l_d_ = nullptr, *u_d_ = nullptr, *q_d_ = nullptr, *lc_d_ = nullptr, *uc_d_ = nullptr,
            *g_d_ = nullptr, *cr_d_ = nullptr, *vr_d_ = nullptr;
@@ -1267,6 +1276,7 @@ void Solve::setup_bb()
     bb_tscale_ = bb_tol_ + 1;
     bb_inner_ = ar_.alloc<int>(1);
     CK(cudaMemsetAsync(bb_inner_, 0, sizeof(int), s));
+    setup_bb_special(nsm);
     int lim = prm_.inner_solver_parameters.iteration_limit;
     double it0 = prm_.inner_solver_parameters.initial_tolerance;
     double mt = prm_.inner_solver_parameters.min_tolerance;
@@ -1318,6 +1328,62 @@ void Solve::setup_bb()
     if (nonconvexity_ < 0)
         bb_limit_ = 1; // reference optimize, src/solver.cu:109-112
     CK(cudaGetLastError());
+}
+
+// Which problems leave the general inner kernel: see inner_small.cu and
+// inner_dense.cu for why.  Both take one block per SM.
+void Solve::setup_bb_special(int nsm)
+{
+    cudaStream_t s = st_;
+    sms_ = nsm;
+    const int k = R_.nnz > 0 ? R_.rows : 0, nc = (int)cone_start_.size();
+    if (dp_.has_fixed || dp_.var_psd)
+        return;
+    if (k == 0 && nc == 0 && Q_.nnz > 0 && (long long)Q_.nnz <= 16LL * n_) {
+        // a thread per row: no row of Q may be long
+        int *cnt = ar_.alloc<int>(1);
+        int h = 1;
+        CK(cudaMemsetAsync(cnt, 0, sizeof(int), s));
+        long_count_kernel<<<grid_for(n_, TPB), TPB, 0, s>>>(n_, Q_.rp, cnt);
+        CK(cudaMemcpyAsync(&h, cnt, sizeof(int), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        if (h == 0)
+            bb_small_blocks_ = bb_small_blocks(n_, Q_.nnz, nsm);
+    } else if (r_width_ > 0 && (dp_.dkind != 2 || k <= 64)) {
+        // R must not touch a cone slot, Q must be diagonal; a dense middle
+        // matrix is applied by every block in every pass, so only a small one
+        for (int st : cone_start_)
+            if (st < r_width_)
+                return;
+        const int tiles = dense_tile_count(r_width_);
+        const int blocks = dense_blocks(k, tiles, S_, nsm);
+        if (blocks == 0)
+            return;
+        if (Q_.nnz > 0) {
+            double *qd = ar_.alloc<double>(n_);
+            int *bad = ar_.alloc<int>(1);
+            int h = 1;
+            CK(cudaMemsetAsync(bad, 0, sizeof(int), s));
+            dense_qdiag(n_, Q_.rp, Q_.ci, Q_.v, qd, bad, s);
+            CK(cudaMemcpyAsync(&h, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
+            CK(cudaStreamSynchronize(s));
+            if (h)
+                return;
+            bb_dense_.qd = qd;
+        }
+        const size_t vals = (size_t)tiles * k * 32;
+        Rtile_ = ar_.alloc<double>(vals);
+        if (opt_.precision == PDHCG_B200_MIXED)
+            Rtilef_ = ar_.alloc<float>(vals);
+        dense_tiles(k, r_width_, R_.rp, R_.v, tiles, Rtile_, Rtilef_, s);
+        bb_dense_.tiles = tiles;
+        bb_dense_.width = r_width_;
+        bb_dense_.rx_state = ar_.alloc<double>(2 * (size_t)k);
+        bb_dense_blocks_ = blocks;
+    }
+    if (bb_small_blocks_ > 0 || bb_dense_blocks_ > 0) {
+        bb_slots_ = bb_small_blocks_ > 0 ? make_slots(bb_small_blocks_, 2) : make_slots(bb_dense_blocks_, k + 2);
+    }
 }
 
 void Solve::enqueue_q_apply(const double *v, double *qx)
@@ -1603,12 +1669,20 @@ void Solve::enqueue_step_bb(bool store_dual, bool want_fpe, double w)
         tau = std::fmax(tau, -1.01 * std::fmin(0.0, nonconvexity_));
         tau /= 100;
     }
-    if (bb_fp32_ && Atf_)
-        long_pass(At_, (const float *)Atf_, y_);
-    else
-        long_pass(At_, At_.v, y_);
-    spmv_kernel<<<grid_for(((long long)n_ + 31) / 32, WARPS), TPB, 0, s>>>(n_, At_.rp, At_.ci, At_.v, y_, bb_aty_,
-                                                                          At_.lr);
+    const bool at_f32 = bb_fp32_ && Atf_;
+    const int at_grid = grid_for(((long long)n_ + 31) / 32, WARPS);
+    if (2 * At_.long_nnz >= At_.nnz && At_.max_row <= MID_ROW_MAX) { // mostly rows of a middle length
+        if (at_f32)
+            spmv_mid_kernel<float><<<at_grid, TPB, 0, s>>>(n_, At_.rp, At_.ci, At_.v, Atf_, y_, bb_aty_);
+        else
+            spmv_mid_kernel<double><<<at_grid, TPB, 0, s>>>(n_, At_.rp, At_.ci, At_.v, At_.v, y_, bb_aty_);
+    } else {
+        if (at_f32)
+            long_pass(At_, (const float *)Atf_, y_);
+        else
+            long_pass(At_, At_.v, y_);
+        spmv_kernel<<<at_grid, TPB, 0, s>>>(n_, At_.rp, At_.ci, At_.v, y_, bb_aty_, At_.lr);
+    }
     double inv_tau = 1.0 / tau;
     if (bb_m_ && inv_tau != bb_cached_inv_tau_) {
         int nb = grid_for(n_, TPB, 148 * 4);
@@ -1619,8 +1693,16 @@ void Solve::enqueue_step_bb(bool store_dual, bool want_fpe, double w)
         stats_.kernel_launches += 3;
     }
     BBData D = bb_data();
-    BBParams BP{tau, w, prm_.reflection_coefficient, want_fpe ? 1 : 0};
-    launch_bb(GQ_, S_, dp_.has_fixed, bb_grid_, D, BP, s);
+    BBParams BP{tau, w, prm_.reflection_coefficient, want_fpe ? 1 : 0, bb_refresh_};
+    if (bb_small_blocks_ > 0) {
+        launch_bb_small(n_, Q_.nnz, sms_, bb_small_blocks_, D, BP, bb_slots_, s);
+    } else if (bb_dense_blocks_ > 0) {
+        bb_dense_.tile = bb_fp32_ ? (const void *)Rtilef_ : (const void *)Rtile_;
+        launch_bb_dense(S_, bb_fp32_, bb_dense_blocks_, D, BP, bb_dense_, bb_slots_, s);
+        bb_refresh_ = 0;
+    } else {
+        launch_bb(GQ_, S_, dp_.has_fixed, bb_grid_, D, BP, s);
+    }
     StepParams P{};
     P.tau = tau;
     P.sigma = step_ * omega_;
@@ -1743,6 +1825,7 @@ double Solve::bb_inner_bytes(bool fp32) const
     const double vb = fp32 ? 4.0 : 8.0; // bytes of a value of Q, R, R^T
     double q = Q_.nnz > 0 ? Q_.nnz * (4.0 + vb) + (n + 1) * 4 + n * 8 : 0.0;
     double r = R_.nnz == 0 ? 0.0
+               : bb_dense_blocks_ > 0 ? R_.nnz * vb              // one pass over the tiles
                : r_width_ ? 2.0 * R_.nnz * vb + r_width_ * 8.0 // values only, x_p read contiguously
                           : 2.0 * R_.nnz * (4.0 + vb) + (R_.rows + 1) * 4.0 + (n + 1) * 4 + n * 8;
     return q + r + 15.0 * n * 8;
@@ -2058,6 +2141,7 @@ void Solve::leave_bb_fp32()
     CK(cudaStreamSynchronize(st_));
     bb_inner_fp32_ = inner_total_ + inner; // first passes counted here, further ones on the device
     bb_fp32_ = false;
+    bb_refresh_ = 2; // R x and R x_init with the FP64 values
 }
 
 void Solve::leave_fp32()
@@ -2385,6 +2469,7 @@ void Solve::loop()
                 else
                     restart_copy_kernel<double><<<grid_for((long long)n_ + m_, TPB), TPB, 0, st_>>>(
                         n_, m_, xp_, x0_, x_, yp_, y0_, y_);
+                bb_refresh_ = 1; // x = x_init
                 stats_.kernel_launches++;
                 stats_.restarts++;
                 inner_count_ = 0;
@@ -2638,6 +2723,8 @@ pdhcg_result_t *Solve::run()
         int inner = 0;
         CK(cudaMemcpyAsync(&inner, bb_inner_, sizeof(int), cudaMemcpyDeviceToHost, st_));
         CK(cudaStreamSynchronize(st_));
+        if (bb_slots_.err)
+            check_slots(bb_slots_, "inner solve");
         inner_total_ += inner;
     }
     auto t_res = std::chrono::steady_clock::now();

@@ -1,0 +1,61 @@
+"""The inner solves with their own kernels, sparse Q of short rows and dense
+low-rank terms, against the oracle at the sizes where their launch shape, tile
+grouping or dispatch changes."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from pdhcg_b200 import instances
+from pdhcg_b200.capi import CsrMatrix
+from test_gpu_resident import _problem
+from test_gpu_solver import _solve_gpu, _solve_oracle
+
+pytestmark = pytest.mark.gpu
+
+# An inner solve ends by a test on its step (relative 1e-3 of the start's and
+# tighter as the outer solve goes on), which rounding may pass one inner
+# iteration apart; such a step is below the outer error of 45 iterations by
+# far more than the 1e-6 asked for here.
+PRM = {"termination_criteria.iteration_limit": 45, "termination_criteria.eps_optimal_relative": 1e-15,
+       "termination_criteria.eps_feasible_relative": 1e-15}
+
+
+def _compare(lib, oracle, p):
+    a, b = _solve_gpu(lib, p, PRM), _solve_oracle(oracle, lib, p, PRM)
+    assert a["termination_reason"] == b["termination_reason"]
+    for key in ("x", "y"):
+        np.testing.assert_allclose(a[key], b[key], rtol=0, atol=1e-6 * max(1.0, np.abs(b[key]).max()))
+
+
+# n and half bandwidth of Q.  Cluster form (up to 64 K entries off the
+# diagonal): 128, 512, 1024 variables a block; grid form beyond, 128, 256 a
+# block; past the register forms the general kernel
+@pytest.mark.parametrize("n,band", [(2, 1), (127, 1), (128, 2), (129, 3), (2048, 1), (2049, 2), (8192, 2), (8193, 2),
+                                    (16384, 1), (16385, 1), (8193, 3), (8193, 4), (18944, 2), (18945, 2), (20000, 7),
+                                    (40000, 8)])
+def test_sparse_q(lib, oracle, n, band):
+    rng = np.random.default_rng(n + band)
+    p = _problem(n, n, max(1, n // 2), False)
+    diags = [np.full(n, 2.0 * band)] + [rng.uniform(-0.9, 0.9, n - d) for d in range(1, band + 1) if d < n]
+    Q = sp.diags(diags, range(len(diags)), format="csr")
+    p.Q = CsrMatrix.from_scipy(sp.csr_matrix(Q + sp.triu(Q, 1).T))
+    _compare(lib, oracle, p)
+
+
+# rows of R around the 16 warps, 4, 8 and 16 rows a warp and the limit of 256
+# (FP64 groups of 4 tiles to 64 rows, 2 to 108); widths around the 32 columns
+# of a tile and the groups of tiles a block takes
+@pytest.mark.parametrize("k,n", [(1, 31), (1, 33), (15, 32), (16, 64), (17, 300), (64, 5000), (65, 5000), (108, 9500),
+                                 (109, 4737), (128, 3000), (129, 3000), (256, 700), (257, 700)])
+@pytest.mark.parametrize("with_q", [False, True])
+def test_dense_low_rank(lib, oracle, k, n, with_q):
+    rng = np.random.default_rng(k * 10000 + n)
+    p = _problem(n, n, max(1, n // 4), with_q)
+    p.R_dense = rng.standard_normal((k, n)) / np.sqrt(n)
+    _compare(lib, oracle, p)
+
+
+def test_portfolio_with_columns_of_middle_length(lib, oracle):
+    """The exposure rows make every column of A 70 entries long (the product
+    with A^T by a warp a column); cone slots follow the columns of R."""
+    _compare(lib, oracle, instances.portfolio(seed=11, scale=0.05, rank=70, sectors=40))
