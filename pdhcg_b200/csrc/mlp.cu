@@ -281,7 +281,7 @@ __global__ void mse_kernel(long long n, const float *o, const float *t, float sc
 }
 
 // acc += (sum of the nb block partials, in order) / tot + the head's loss
-__global__ void loss_fold_kernel(const double *part, int nb, double tot, const double *hloss, int nhloss, double *acc)
+__global__ void loss_fold_kernel(const double *part, int nb, double tot, const double *hloss, double *acc)
 {
     __shared__ double sh[256];
     double a = 0.0;
@@ -294,12 +294,8 @@ __global__ void loss_fold_kernel(const double *part, int nb, double tot, const d
             sh[threadIdx.x] += sh[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        double v = sh[0] / tot;
-        for (int b = 0; b < nhloss; ++b)
-            v += hloss[b];
-        acc[0] += v;
-    }
+    if (threadIdx.x == 0)
+        acc[0] += sh[0] / tot + hloss[0];
 }
 
 // log-weight head: lw[b] = wp . h2[b] + bp; dlw = 2 (lw - tl) / B; loss partial
@@ -359,32 +355,33 @@ __global__ void to_bf16_kernel(long long n, const float *src, bf16 *dst)
 int blocks_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 148 * 8); }
 
 // ---------------------------------------------------------------------------
-// The trunk's products for one minibatch (at most SMALL_B rows).  They are
+// The trunk's products of one prediction (at most SMALL_B rows).  They are
 // latency bound, not throughput bound (64 x 512 x 512 is 34 MFLOP), so a CTA
 // owns only a 32 x 16 tile and its 8 warps split K, loading their fragments
 // straight from L2 (no staging: each element is used by one warp) with every
 // load of a warp in flight at once; the 8 partial tiles are added in warp
-// order in shared memory and the epilogue (bias, ReLU, the ReLU mask of the
-// backward pass, the log-weight head's outer product) runs on the sum.  FP32
+// order in shared memory and the epilogue (bias, ReLU) runs on the sum.  FP32
 // sums; an FP32 operand enters a product with BF16 weights as three BF16
-// parts (exact; the third product costs nothing here), one with another FP32
-// operand as a pair, as in mma_gemm_kernel.
+// parts (exact; the third product costs nothing here).
+//
+// Training keeps the tiled products.  On these kernels, with the head's
+// products, loss and Adam update in one pass, a step took 0.12 ms instead of
+// 0.55, but a run of 160 steps carries another order of the sums on to
+// parameters 1e-3 to 5e-3 apart (and, where the loss spikes, further).
 // ---------------------------------------------------------------------------
 constexpr int SMALL_B = 128;           // rows up to which the minibatch kernels are used
 constexpr int SM_M = 32, SM_N = 16;    // tile
 constexpr int SM_W = 8;                // warps, K split over them
 
-enum SmallEpi { EPI_PLAIN, EPI_BIAS, EPI_BIAS_RELU, EPI_MASK, EPI_MASK_OUTER };
+enum SmallEpi { EPI_BIAS, EPI_BIAS_RELU };
 
 struct SmallGemm {
     int M, N, K;
-    const void *A, *B;
-    int lda, ldb;
-    float *C; // ldc = N
-    const float *bias;        // EPI_BIAS*: [N]
-    const float *mask;        // EPI_MASK*: C is kept where mask > 0, 0 elsewhere ([M x N])
-    const float *col, *row;   // EPI_MASK_OUTER: + col[i] * row[j] before the mask
-    int vec;                  // word loads of pairs along K (see small_gemm_tile)
+    const float *A; // [M][K]
+    const bf16 *B;  // [N][K]
+    float *C;       // [M][N]
+    const float *bias;
+    int vec; // word loads of pairs along K (see small_gemm_tile)
     __host__ __device__ int tiles() const { return ((M + SM_M - 1) / SM_M) * ((N + SM_N - 1) / SM_N); }
 };
 
@@ -421,25 +418,22 @@ __device__ __forceinline__ float2 pair_at(const T *p, int ld, int i, int k, int 
     return v;
 }
 
-// the same as a BF16 pair (hi) of a BF16 matrix, VEC: one 4-byte load
-template <bool KFAST, bool VEC>
+// the same as a BF16 pair of a BF16 matrix, VEC: one 4-byte load
+template <bool VEC>
 __device__ __forceinline__ unsigned bf16_pair_at(const bf16 *p, int ld, int i, int k, int I, int K)
 {
-    if (VEC && KFAST)
+    if (VEC)
         return i < I && k < K ? *reinterpret_cast<const unsigned *>(p + (size_t)i * ld + k) : 0u;
-    const float2 v = pair_at<KFAST>(p, ld, i, k, I, K);
+    const float2 v = pair_at<true>(p, ld, i, k, I, K);
     const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
     return *reinterpret_cast<const unsigned *>(&h);
 }
 
 // VEC: pairs along K that are contiguous are loaded as one word (even K and
 // leading dimension, 8-byte aligned FP32, 4-byte aligned BF16)
-template <bool TA, bool TB, bool VEC, typename AT, typename BT, int EPI>
+template <bool VEC, int EPI>
 __device__ __forceinline__ void small_gemm_tile(const SmallGemm &G, int tile, float (*red)[SM_M * SM_N])
 {
-    constexpr bool SA = !std::is_same<AT, bf16>::value, SB = !std::is_same<BT, bf16>::value;
-    const AT *A = (const AT *)G.A;
-    const BT *B = (const BT *)G.B;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int nt_n = (G.N + SM_N - 1) / SM_N;
     const int i0 = (tile / nt_n) * SM_M, j0 = (tile % nt_n) * SM_N;
@@ -449,46 +443,34 @@ __device__ __forceinline__ void small_gemm_tile(const SmallGemm &G, int tile, fl
 #pragma unroll 4
     for (int st = s0; st < s1; ++st) {
         const int k0 = 16 * st + 2 * t;
-        unsigned a[3][2][4], b[2][2][2];
+        unsigned a[3][2][4], b[2][2];
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int i = i0 + 16 * mt + g + 8 * (q & 1), k = k0 + 8 * (q >> 1);
                 float2 v = make_float2(0.0f, 0.0f);
-                if (VEC && !TA) {
+                if (VEC) {
                     if (i < G.M && k < G.K)
-                        v = *reinterpret_cast<const float2 *>(A + (size_t)i * G.lda + k);
+                        v = *reinterpret_cast<const float2 *>(G.A + (size_t)i * G.K + k);
                 } else {
-                    v = pair_at<!TA>(A, G.lda, i, k, G.M, G.K);
+                    v = pair_at<true>(G.A, G.K, i, k, G.M, G.K);
                 }
-                if (SB)
-                    split2(v.x, v.y, a[0][mt][q], a[1][mt][q]);
-                else
-                    split3(v.x, v.y, a[0][mt][q], a[1][mt][q], a[2][mt][q]);
+                split3(v.x, v.y, a[0][mt][q], a[1][mt][q], a[2][mt][q]);
             }
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
-                if constexpr (SB) {
-                    const float2 v = pair_at<TB>(B, G.ldb, j0 + 8 * nt + g, k0 + 8 * q, G.N, G.K);
-                    split2(v.x, v.y, b[0][nt][q], b[1][nt][q]);
-                } else {
-                    b[0][nt][q] = bf16_pair_at<TB, VEC>(B, G.ldb, j0 + 8 * nt + g, k0 + 8 * q, G.N, G.K);
-                }
+                b[nt][q] = bf16_pair_at<VEC>(G.B, G.K, j0 + 8 * nt + g, k0 + 8 * q, G.N, G.K);
             }
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
-                static_assert(SA, "the left operand is FP32");
-                if (!SB)
-                    mma_bf16(acc[mt][nt], a[2][mt], b[0][nt]);
-                mma_bf16(acc[mt][nt], a[1][mt], b[0][nt]);
-                if (SB)
-                    mma_bf16(acc[mt][nt], a[0][mt], b[1][nt]);
-                mma_bf16(acc[mt][nt], a[0][mt], b[0][nt]);
+                mma_bf16(acc[mt][nt], a[2][mt], b[nt]);
+                mma_bf16(acc[mt][nt], a[1][mt], b[nt]);
+                mma_bf16(acc[mt][nt], a[0][mt], b[nt]);
             }
     }
 #pragma unroll
@@ -506,14 +488,9 @@ __device__ __forceinline__ void small_gemm_tile(const SmallGemm &G, int tile, fl
             v += red[w][e];
         const int i = i0 + e / SM_N, j = j0 + e % SM_N;
         if (i < G.M && j < G.N) {
-            if (EPI == EPI_BIAS || EPI == EPI_BIAS_RELU)
-                v += G.bias[j];
+            v += G.bias[j];
             if (EPI == EPI_BIAS_RELU)
                 v = fmaxf(v, 0.0f);
-            if (EPI == EPI_MASK_OUTER)
-                v += G.col[i] * G.row[j];
-            if ((EPI == EPI_MASK || EPI == EPI_MASK_OUTER) && !(G.mask[(size_t)i * G.N + j] > 0.0f))
-                v = 0.0f;
             G.C[(size_t)i * G.N + j] = v;
         }
     }
@@ -524,9 +501,8 @@ __device__ __forceinline__ void small_gemm_tile(const SmallGemm &G, int tile, fl
 // lanes over the hidden units (one thread per row took 512 dependent loads).
 struct HeadArgs {
     int B, H;
-    const float *h2, *wp, *bp, *tl; // tl NULL: prediction only
-    float *lw, *dlw;
-    double *loss; // per block of SM_W rows
+    const float *h2, *wp, *bp;
+    float *lw;
 };
 
 template <int EPI, bool LAST>
@@ -534,10 +510,8 @@ __global__ void __launch_bounds__(32 * SM_W) small_layer_kernel(SmallGemm G, Hea
 {
     __shared__ float red[SM_W][SM_M * SM_N];
     if (LAST && (int)blockIdx.x >= G.tiles()) {
-        __shared__ double sq[SM_W];
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int blk = (int)blockIdx.x - G.tiles(), b = blk * SM_W + warp;
-        double a = 0.0;
+        const int b = ((int)blockIdx.x - G.tiles()) * SM_W + warp;
         if (b < h.B) {
             float s = 0.0f;
 #pragma unroll 8
@@ -546,185 +520,58 @@ __global__ void __launch_bounds__(32 * SM_W) small_layer_kernel(SmallGemm G, Hea
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1)
                 s += __shfl_xor_sync(0xffffffffu, s, o);
-            s += h.bp[0];
-            if (lane == 0) {
-                h.lw[b] = s;
-                if (h.tl) {
-                    const float r = s - h.tl[b];
-                    h.dlw[b] = 2.0f * r / (float)h.B;
-                    a = (double)r * (double)r;
-                }
-            }
-        }
-        if (lane == 0)
-            sq[warp] = a;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int w = 1; w < SM_W; ++w)
-                a += sq[w];
-            h.loss[blk] = a / (double)h.B;
+            if (lane == 0)
+                h.lw[b] = s + h.bp[0];
         }
         return;
     }
     if (G.vec)
-        small_gemm_tile<false, true, true, float, bf16, EPI>(G, blockIdx.x, red);
+        small_gemm_tile<true, EPI>(G, blockIdx.x, red);
     else
-        small_gemm_tile<false, true, false, float, bf16, EPI>(G, blockIdx.x, red);
-}
-
-// One layer of the backward pass: the tiles of dX = dY W (masked by the ReLU
-// of the layer below), then the tiles of dW = dY^T X, whose first column of
-// tiles also sums db over the rows; OUTER: then the log-weight head's
-// gradients.  dY: [B x out], X: [B x in].
-struct BackArgs {
-    SmallGemm dx, dw;
-    float *db;
-    const float *dlw, *h2;
-    float *gwp, *gbp;
-    int B, H;
-};
-
-template <bool OUTER, bool DX>
-__global__ void __launch_bounds__(32 * SM_W) small_back_kernel(BackArgs P)
-{
-    __shared__ float red[SM_W][SM_M * SM_N];
-    int tile = blockIdx.x;
-    if (DX) {
-        if (tile < P.dx.tiles()) {
-            constexpr int EPI = OUTER ? EPI_MASK_OUTER : EPI_MASK;
-            if (P.dx.vec)
-                small_gemm_tile<false, false, true, float, bf16, EPI>(P.dx, tile, red);
-            else
-                small_gemm_tile<false, false, false, float, bf16, EPI>(P.dx, tile, red);
-            return;
-        }
-        tile -= P.dx.tiles();
-    }
-    if (tile < P.dw.tiles()) {
-        small_gemm_tile<true, false, false, float, float, EPI_PLAIN>(P.dw, tile, red);
-        const int nt_n = (P.dw.N + SM_N - 1) / SM_N;
-        const int i = (tile / nt_n) * SM_M + (int)threadIdx.x;
-        if (tile % nt_n == 0 && threadIdx.x < SM_M && i < P.dw.M) { // rows summed in order
-            const float *dy = (const float *)P.dw.A;
-            float s = 0.0f;
-#pragma unroll 8
-            for (int b = 0; b < P.B; ++b)
-                s += dy[(size_t)b * P.dw.lda + i];
-            P.db[i] = s;
-        }
-        return;
-    }
-    tile -= P.dw.tiles();
-    if (OUTER) {
-        const int k = tile * 32 * SM_W + threadIdx.x;
-        if (k < P.H) {
-            float s = 0.0f;
-#pragma unroll 8
-            for (int b = 0; b < P.B; ++b)
-                s += P.dlw[b] * P.h2[(size_t)b * P.H + k];
-            P.gwp[k] = s;
-        }
-        if (k == 0) {
-            float s = 0.0f;
-            for (int b = 0; b < P.B; ++b)
-                s += P.dlw[b];
-            P.gbp[0] = s;
-        }
-    }
+        small_gemm_tile<false, EPI>(G, blockIdx.x, red);
 }
 
 // ---------------------------------------------------------------------------
-// The output head of a training step in one pass over its tiles of 64
-// outputs (B <= 64 rows, rank <= 64).  It is the step's memory traffic: per
-// output 64 weights with their two moments.  Taken apart into products and
-// element-wise kernels it moved O, T, dO and the gradient through HBM about
-// ten times (0.55 ms a step at 75000 outputs); here a tile is
-//   O = Z U^T + bu, dO = 2 (O - T) / (B out), dbu = column sums,
-//   dU = dO^T Z, dZ += dO U
-// on the tensor cores from shared memory, and with ADAM the tile's weights,
-// moments and BF16 copy are updated in the same pass from the gradient in
-// registers, so a step reads T and reads and writes U's state once.
-// GRAD writes the gradient instead.  PREDICT writes O and stops.
-// Every operand is staged once and read by ldmatrix, transposed where a
-// product needs it, and U's state moves as pairs: 53 us at 75000 outputs (97
-// with transposed copies stored 2 bytes at a time and scalar accesses of the
-// state; its 125 MB take 19 us at HBM's rate).
-// Each CTA walks tiles grid-stride and keeps its share of dZ in registers;
-// the shares are written to part and added in CTA order by head_fold_kernel.
+// The output head of a prediction (B <= 64 rows, rank <= 64), O = Z U^T + bu, a
+// CTA per tile of 64 outputs: Z as three BF16 parts and the tile of U staged in
+// shared memory, read by ldmatrix.  It writes O, 64 rows by 4 bytes for every
+// 128 bytes of U, and reads nothing twice: for one row of 75000 outputs the
+// whole prediction took 208 us with the tiled products and now takes 87.
 // ---------------------------------------------------------------------------
 constexpr int HB = 64, HR = 64, HJ = 64; // rows, rank, outputs of a tile
 constexpr int HP = 72;                   // pitch of the staged operands (144 bytes: conflict-free ldmatrix rows)
-enum HeadMode { HEAD_PREDICT, HEAD_GRAD, HEAD_ADAM };
 
 struct AdamArgs {
     float lr, b1, b2, c1, c2, eps;
 };
 
-__device__ __forceinline__ float adam_update(float w, float g, float &m, float &v, const AdamArgs &a)
-{
-    m = a.b1 * m + (1.0f - a.b1) * g;
-    v = a.b2 * v + (1.0f - a.b2) * g * g;
-    return w - a.lr * (m / a.c1) / (sqrtf(v / a.c2) + a.eps);
-}
-
 struct HeadTile {
     int B, rank, out;
-    const float *Z, *T;      // [B x rank], [B x out]
-    float *w, *m, *v, *g;    // U: [out x rank]
-    bf16 *wb;
-    float *bw, *bm, *bv, *bg; // bu: [out]
-    float *O;                // HEAD_PREDICT
-    float scale;             // 1 / (B out)
-    float *part;             // [grid][B x rank] shares of dZ
-    double *loss;            // [grid] sums of (o - t)^2
-    AdamArgs a;
-};
-
-// shared memory: Z as three BF16 parts, U, and dO as a BF16 pair, each once,
-// row-major; the products read them as they are or transposed by ldmatrix
-struct HeadSmem {
-    bf16 z[3][HB][HP], u[HJ][HP]; // all that a prediction stages
-    bf16 d[2][HB][HP];
-    float db[4][HJ];
-    double sq[8];
+    const float *Z;  // [B x rank]
+    const bf16 *wb;  // U: [out x rank]
+    const float *bw; // bu: [out]
+    float *O;        // [B x out]
 };
 
 // four 8 x 8 matrices; lane l passes the address of row l & 7 of matrix l >> 3
-template <bool TRANS>
 __device__ __forceinline__ void ldsm4(unsigned (&r)[4], const bf16 *p)
 {
     const unsigned a = (unsigned)__cvta_generic_to_shared(p);
-    if (TRANS)
-        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                     : "r"(a));
-    else
-        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                     : "r"(a));
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a));
 }
 
 // left operand rows i.., columns k.. of s[i][k]
 __device__ __forceinline__ void frag_a(unsigned (&a)[4], const bf16 (*s)[HP], int i, int k, int lane)
 {
-    ldsm4<false>(a, &s[i + (lane & 15)][k + (lane >> 4) * 8]);
-}
-// the same of s[k][i]
-__device__ __forceinline__ void frag_at(unsigned (&a)[4], const bf16 (*s)[HP], int i, int k, int lane)
-{
-    ldsm4<true>(a, &s[k + (lane >> 4) * 8 + (lane & 7)][i + ((lane >> 3) & 1) * 8]);
+    ldsm4(a, &s[i + (lane & 15)][k + (lane >> 4) * 8]);
 }
 // right operands of two 8-column tiles n.., n + 8.. (registers 0, 1 and 2, 3) of s[n][k]
 __device__ __forceinline__ void frag_b2(unsigned (&b)[4], const bf16 (*s)[HP], int n, int k, int lane)
 {
-    ldsm4<false>(b, &s[n + (lane >> 4) * 8 + (lane & 7)][k + ((lane >> 3) & 1) * 8]);
+    ldsm4(b, &s[n + (lane >> 4) * 8 + (lane & 7)][k + ((lane >> 3) & 1) * 8]);
 }
-// the same of s[k][n]
-__device__ __forceinline__ void frag_bt2(unsigned (&b)[4], const bf16 (*s)[HP], int n, int k, int lane)
-{
-    ldsm4<true>(b, &s[k + (lane & 15)][n + (lane >> 4) * 8]);
-}
-
 __device__ __forceinline__ void mma_pair(float (&c0)[4], float (&c1)[4], const unsigned (&a)[4], const unsigned (&b)[4])
 {
     const unsigned b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
@@ -732,13 +579,14 @@ __device__ __forceinline__ void mma_pair(float (&c0)[4], float (&c1)[4], const u
     mma_bf16(c1, a, b1);
 }
 
-// VEC: rank 64, even out, U's arrays and T on word boundaries: 16-byte loads
-// of U, pairs of everything else
-template <int MODE, bool VEC>
+// VEC: rank 64, even out, U and O on word boundaries: 16-byte loads of U, pairs
+// of O
+template <bool VEC>
 __global__ void __launch_bounds__(256, 2) head_tile_kernel(HeadTile P)
 {
-    extern __shared__ __align__(16) char smem_raw[];
-    HeadSmem &S = *reinterpret_cast<HeadSmem *>(smem_raw);
+    __shared__ __align__(16) struct {
+        bf16 z[3][HB][HP], u[HJ][HP];
+    } S;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int m0 = 16 * (warp & 3), n0 = 32 * (warp >> 2); // this warp's 16 x 32 of every 64 x 64 product
     for (int e = threadIdx.x; e < HB * HR; e += 256) {
@@ -750,8 +598,6 @@ __global__ void __launch_bounds__(256, 2) head_tile_kernel(HeadTile P)
         S.z[1][b][r] = lo;
         S.z[2][b][r] = __float2bfloat16_rn((zv - __bfloat162float(hi)) - __bfloat162float(lo));
     }
-    float dz[4][4] = {};
-    double sq = 0.0;
     const int ntiles = (P.out + HJ - 1) / HJ;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int j0 = tile * HJ;
@@ -772,32 +618,14 @@ __global__ void __launch_bounds__(256, 2) head_tile_kernel(HeadTile P)
                                                          : __float2bfloat16_rn(0.0f);
             }
         }
-        // this thread's targets and biases, in flight while U is staged
-        float tv[4][4], bu[4][2];
+        float bu[4][2]; // this thread's biases, in flight while U is staged
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            const int j = j0 + n0 + 8 * nt + 2 * t;
+        for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-            for (int q = 0; q < 2; ++q)
-                bu[nt][q] = j + q < P.out ? P.bw[j + q] : 0.0f;
-            if (MODE != HEAD_PREDICT) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int b = m0 + g + 8 * h;
-                    if (VEC) { // even out: a pair is in or out
-                        float2 v = make_float2(0.0f, 0.0f);
-                        if (b < P.B && j < P.out)
-                            v = *reinterpret_cast<const float2 *>(P.T + (size_t)b * P.out + j);
-                        tv[nt][2 * h] = v.x;
-                        tv[nt][2 * h + 1] = v.y;
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 2; ++q)
-                            tv[nt][2 * h + q] = b < P.B && j + q < P.out ? P.T[(size_t)b * P.out + j + q] : 0.0f;
-                    }
-                }
+            for (int q = 0; q < 2; ++q) {
+                const int j = j0 + n0 + 8 * nt + 2 * t + q;
+                bu[nt][q] = j < P.out ? P.bw[j] : 0.0f;
             }
-        }
         __syncthreads();
         float o[4][4] = {};
 #pragma unroll
@@ -814,258 +642,42 @@ __global__ void __launch_bounds__(256, 2) head_tile_kernel(HeadTile P)
                 mma_pair(o[nt], o[nt + 1], ah, b);
             }
         }
-        if (MODE == HEAD_PREDICT) {
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int b = m0 + g + 8 * h, j = j0 + n0 + 8 * nt + 2 * t;
-                    if (b >= P.B || j >= P.out)
-                        continue;
-                    const float v0 = o[nt][2 * h] + bu[nt][0], v1 = o[nt][2 * h + 1] + bu[nt][1];
-                    float *dst = P.O + (size_t)b * P.out + j;
-                    if (VEC) {
-                        *reinterpret_cast<float2 *>(dst) = make_float2(v0, v1);
-                    } else {
-                        dst[0] = v0;
-                        if (j + 1 < P.out)
-                            dst[1] = v1;
-                    }
-                }
-            continue;
-        }
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            float cs[2] = {0.0f, 0.0f};
-            const int jj = n0 + 8 * nt + 2 * t;
+        for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int b = m0 + g + 8 * h;
-                float d[2];
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    d[q] = 0.0f;
-                    if (b < P.B && j0 + jj + q < P.out) {
-                        const float r = o[nt][2 * h + q] + bu[nt][q] - tv[nt][2 * h + q];
-                        d[q] = 2.0f * r * P.scale;
-                        sq += (double)r * (double)r;
-                    }
-                    cs[q] += d[q];
-                }
-                unsigned hi, lo;
-                split2(d[0], d[1], hi, lo);
-                *reinterpret_cast<unsigned *>(&S.d[0][b][jj]) = hi;
-                *reinterpret_cast<unsigned *>(&S.d[1][b][jj]) = lo;
-            }
-#pragma unroll
-            for (int q = 0; q < 2; ++q) { // column sums over the warp's 16 rows
-#pragma unroll
-                for (int s = 4; s < 32; s <<= 1)
-                    cs[q] += __shfl_xor_sync(0xffffffffu, cs[q], s);
-                if (g == 0)
-                    S.db[warp & 3][jj + q] = cs[q];
-            }
-        }
-        __syncthreads();
-        float du[4][4] = {};
-#pragma unroll
-        for (int k = 0; k < HB; k += 16) {
-            unsigned ah[4], al[4], bh[4], bl[4];
-            frag_at(ah, S.d[0], m0, k, lane);
-            frag_at(al, S.d[1], m0, k, lane);
-#pragma unroll
-            for (int nt = 0; nt < 4; nt += 2) { // dU = dO^T Z
-                frag_bt2(bh, S.z[0], n0 + 8 * nt, k, lane);
-                frag_bt2(bl, S.z[1], n0 + 8 * nt, k, lane);
-                mma_pair(du[nt], du[nt + 1], al, bh);
-                mma_pair(du[nt], du[nt + 1], ah, bl);
-                mma_pair(du[nt], du[nt + 1], ah, bh);
-            }
-            frag_a(ah, S.d[0], m0, k, lane);
-            frag_a(al, S.d[1], m0, k, lane);
-#pragma unroll
-            for (int nt = 0; nt < 4; nt += 2) { // dZ += dO U
-                frag_bt2(bh, S.u, n0 + 8 * nt, k, lane);
-                mma_pair(dz[nt], dz[nt + 1], al, bh);
-                mma_pair(dz[nt], dz[nt + 1], ah, bh);
-            }
-        }
-        // U's state, half of this thread's entries loaded before any is stored
-        // (with a load behind each store a tile took 28 us)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            float2 w[4], m[4], v[4]; // entry pairs (row j, ranks r, r + 1) of the four column tiles
-            const int j = j0 + m0 + g + 8 * h;
-#pragma unroll
-            for (int nt = 0; nt < 4 && MODE == HEAD_ADAM; ++nt) {
-                const int r = n0 + 8 * nt + 2 * t;
-                w[nt] = m[nt] = v[nt] = make_float2(0.0f, 0.0f);
-                const size_t e = (size_t)j * P.rank + r;
-                if (VEC) {
-                    if (j < P.out) {
-                        w[nt] = *reinterpret_cast<const float2 *>(P.w + e);
-                        m[nt] = *reinterpret_cast<const float2 *>(P.m + e);
-                        v[nt] = *reinterpret_cast<const float2 *>(P.v + e);
-                    }
-                } else if (j < P.out && r < P.rank) {
-                    w[nt].x = P.w[e];
-                    m[nt].x = P.m[e];
-                    v[nt].x = P.v[e];
-                    if (r + 1 < P.rank) {
-                        w[nt].y = P.w[e + 1];
-                        m[nt].y = P.m[e + 1];
-                        v[nt].y = P.v[e + 1];
-                    }
-                }
-            }
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                const int r = n0 + 8 * nt + 2 * t;
-                if (j >= P.out || r >= P.rank)
+                const int b = m0 + g + 8 * h, j = j0 + n0 + 8 * nt + 2 * t;
+                if (b >= P.B || j >= P.out)
                     continue;
-                const size_t e = (size_t)j * P.rank + r;
-                const float g0 = du[nt][2 * h], g1 = du[nt][2 * h + 1];
-                const bool two = VEC || r + 1 < P.rank;
-                if (MODE == HEAD_GRAD) {
-                    P.g[e] = g0;
-                    if (two)
-                        P.g[e + 1] = g1;
-                    continue;
-                }
-                float2 x;
-                x.x = adam_update(w[nt].x, g0, m[nt].x, v[nt].x, P.a);
-                x.y = adam_update(w[nt].y, g1, m[nt].y, v[nt].y, P.a);
+                const float v0 = o[nt][2 * h] + bu[nt][0], v1 = o[nt][2 * h + 1] + bu[nt][1];
+                float *dst = P.O + (size_t)b * P.out + j;
                 if (VEC) {
-                    *reinterpret_cast<float2 *>(P.m + e) = m[nt];
-                    *reinterpret_cast<float2 *>(P.v + e) = v[nt];
-                    *reinterpret_cast<float2 *>(P.w + e) = x;
-                    *reinterpret_cast<__nv_bfloat162 *>(P.wb + e) = __floats2bfloat162_rn(x.x, x.y);
+                    *reinterpret_cast<float2 *>(dst) = make_float2(v0, v1);
                 } else {
-                    P.m[e] = m[nt].x;
-                    P.v[e] = v[nt].x;
-                    P.w[e] = x.x;
-                    P.wb[e] = __float2bfloat16_rn(x.x);
-                    if (two) {
-                        P.m[e + 1] = m[nt].y;
-                        P.v[e + 1] = v[nt].y;
-                        P.w[e + 1] = x.y;
-                        P.wb[e + 1] = __float2bfloat16_rn(x.y);
-                    }
+                    dst[0] = v0;
+                    if (j + 1 < P.out)
+                        dst[1] = v1;
                 }
             }
-        }
-        if (threadIdx.x < HJ && j0 + (int)threadIdx.x < P.out) {
-            const int j = j0 + threadIdx.x;
-            const float gb = ((S.db[0][threadIdx.x] + S.db[1][threadIdx.x]) + S.db[2][threadIdx.x]) +
-                             S.db[3][threadIdx.x];
-            if (MODE == HEAD_GRAD) {
-                P.bg[j] = gb;
-            } else {
-                float m = P.bm[j], v = P.bv[j];
-                P.bw[j] = adam_update(P.bw[j], gb, m, v, P.a);
-                P.bm[j] = m;
-                P.bv[j] = v;
-            }
-        }
-    }
-    if (MODE == HEAD_PREDICT)
-        return;
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int b = m0 + g + 8 * (q >> 1), r = n0 + 8 * nt + 2 * t + (q & 1);
-            if (b < P.B && r < P.rank)
-                P.part[(size_t)blockIdx.x * P.B * P.rank + b * P.rank + r] = dz[nt][q];
-        }
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1)
-        sq += __shfl_xor_sync(0xffffffffu, sq, s);
-    if (lane == 0)
-        S.sq[warp] = sq;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w)
-            sq += S.sq[w];
-        P.loss[blockIdx.x] = sq;
     }
 }
 
-// word boundaries of the head's arrays (and of T's rows, where there are any)
+// word boundaries of the head's arrays
 bool head_vec(const HeadTile &P)
 {
-    return P.rank == HR && P.out % 2 == 0 && (size_t)P.wb % 16 == 0 &&
-           ((size_t)P.w | (size_t)P.m | (size_t)P.v | (size_t)P.T | (size_t)P.O) % 8 == 0;
+    return P.rank == HR && P.out % 2 == 0 && (size_t)P.wb % 16 == 0 && (size_t)P.O % 8 == 0;
 }
 
-template <int MODE>
-void launch_head(const HeadTile &P, int grid, size_t smem, cudaStream_t s)
+__global__ void adam_kernel(long long n, float *w, const float *g, float *mom, float *vel, float lr, float b1, float b2,
+                            float c1, float c2, float eps)
 {
-    if (head_vec(P))
-        head_tile_kernel<MODE, true><<<grid, 256, smem, s>>>(P);
-    else
-        head_tile_kernel<MODE, false><<<grid, 256, smem, s>>>(P);
-}
-
-// dZ = the CTAs' shares in CTA order (8 runs of CTAs, then the runs); the
-// last block adds the loss
-__global__ void __launch_bounds__(256) head_fold_kernel(int n, int shares, const float *part, float *dZ,
-                                                        const double *loss, double tot, const double *hloss,
-                                                        int nhloss, double *acc)
-{
-    if (blockIdx.x == gridDim.x - 1) {
-        __shared__ double sh[256];
-        double a = 0.0;
-        for (int b = threadIdx.x; b < shares; b += 256)
-            a += loss[b];
-        sh[threadIdx.x] = a;
-        __syncthreads();
-        for (int w = 128; w > 0; w >>= 1) {
-            if ((int)threadIdx.x < w)
-                sh[threadIdx.x] += sh[threadIdx.x + w];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) {
-            double v = sh[0] / tot;
-            for (int b = 0; b < nhloss; ++b)
-                v += hloss[b];
-            acc[0] += v;
-        }
-        return;
-    }
-    __shared__ float run[8][32];
-    const int e = blockIdx.x * 32 + (threadIdx.x & 31), k = threadIdx.x >> 5;
-    float s = 0.0f;
-    if (e < n) {
-        const int z1 = shares * (k + 1) / 8;
-#pragma unroll 8
-        for (int z = shares * k / 8; z < z1; ++z)
-            s += part[(size_t)z * n + e];
-    }
-    run[k][threadIdx.x & 31] = s;
-    __syncthreads();
-    if (k == 0 && e < n) {
-        for (int q = 1; q < 8; ++q)
-            s += run[q][threadIdx.x];
-        dZ[e] = s;
-    }
-}
-
-// Adam and the BF16 copy for the parameters outside [skip0, skip1) (the
-// output head's, updated in head_tile_kernel)
-__global__ void adam_outer_kernel(long long n, long long skip0, long long skip1, float *w, const float *g, float *mom,
-                                  float *vel, bf16 *wb, AdamArgs a)
-{
-    const long long cnt = n - (skip1 - skip0);
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < cnt;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long e = i < skip0 ? i : i + (skip1 - skip0);
-        float m = mom[e], v = vel[e];
-        const float x = adam_update(w[e], g[e], m, v, a);
-        mom[e] = m;
-        vel[e] = v;
-        w[e] = x;
-        wb[e] = __float2bfloat16_rn(x);
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+        float gg = g[e];
+        float mm = b1 * mom[e] + (1.0f - b1) * gg;
+        float vv = b2 * vel[e] + (1.0f - b2) * gg * gg;
+        mom[e] = mm;
+        vel[e] = vv;
+        w[e] -= lr * (mm / c1) / (sqrtf(vv / c2) + eps);
     }
 }
 
@@ -1119,7 +731,7 @@ int ensure_acts(pdhcg_b200_mlp_s *n, int B)
         al(&n->T, (long long)B * n->out) || al(&n->TL, B) || al(&n->dO, (long long)B * n->out) ||
         al(&n->dZ, (long long)B * n->rank) || al(&n->dH2, (long long)B * n->hid) ||
         al(&n->dH1, (long long)B * n->hid) || al(&n->dLW, B) ||
-        cudaMalloc((void **)&n->part, 148 * 8 * sizeof(double)) || cudaMalloc((void **)&n->hloss, (SMALL_B / SM_W) * sizeof(double)) ||
+        cudaMalloc((void **)&n->part, 148 * 8 * sizeof(double)) || cudaMalloc((void **)&n->hloss, sizeof(double)) ||
         cudaMalloc((void **)&n->acc, sizeof(double))) {
         std::fprintf(stderr, "[pdhcg_b200_mlp] activation allocation failed.\n");
         return -1;
@@ -1128,10 +740,8 @@ int ensure_acts(pdhcg_b200_mlp_s *n, int B)
     return 0;
 }
 
-// The minibatch kernels take up to SMALL_B rows (a 64-row step of the
-// default network: 0.55 ms with the tiled products and element-wise passes
-// below); larger batches keep the tiled products, whose operands are staged
-// once per 64 x 64 tile.
+// A prediction's kernels take up to SMALL_B rows; larger batches, and training,
+// take the tiled products, whose operands are staged once per 64 x 64 tile.
 bool small_trunk(int B) { return B <= SMALL_B; }
 // one 64 x 64 tile of Z in a CTA's shared memory
 bool fused_head(const pdhcg_b200_mlp_s *n, int B) { return B <= HB && n->rank <= HR; }
@@ -1149,9 +759,7 @@ SmallGemm layer(int B, int N, int K, const float *X, const bf16 *W, const float 
     G.N = N;
     G.K = K;
     G.A = X;
-    G.lda = K;
     G.B = W;
-    G.ldb = K;
     G.C = Y;
     G.bias = b;
     G.vec = word_pairs(K, X, W);
@@ -1159,15 +767,15 @@ SmallGemm layer(int B, int N, int K, const float *X, const bf16 *W, const float 
 }
 
 // hidden layers, low-rank layer and log-weight head of B rows X; with TL
-// also the head's loss and dLW
+// (training) also the head's loss and dLW
 int trunk_forward(pdhcg_b200_mlp_s *n, int B, const float *X, const float *TL)
 {
     cudaStream_t s = n->s;
     const bf16 *W1 = n->wb + n->off[P_W1], *W2 = n->wb + n->off[P_W2], *W3 = n->wb + n->off[P_W3];
     const float *b1 = n->w + n->off[P_B1], *b2 = n->w + n->off[P_B2], *b3 = n->w + n->off[P_B3],
                 *wp = n->w + n->off[P_WP], *bp = n->w + n->off[P_BP];
-    if (small_trunk(B)) {
-        const HeadArgs h{B, n->hid, n->H2, wp, bp, TL, n->LW, n->dLW, n->hloss};
+    if (!TL && small_trunk(B)) {
+        const HeadArgs h{B, n->hid, n->H2, wp, bp, n->LW};
         const SmallGemm g1 = layer(B, n->hid, n->in, X, W1, b1, n->H1),
                         g2 = layer(B, n->hid, n->hid, n->H1, W2, b2, n->H2),
                         g3 = layer(B, n->rank, n->hid, n->H2, W3, b3, n->Z);
@@ -1191,53 +799,31 @@ int trunk_forward(pdhcg_b200_mlp_s *n, int B, const float *X, const float *TL)
     return 0;
 }
 
-HeadTile head_tile(const pdhcg_b200_mlp_s *n, int B, const float *T)
-{
-    HeadTile P{};
-    P.B = B;
-    P.rank = n->rank;
-    P.out = n->out;
-    P.Z = n->Z;
-    P.T = T;
-    P.w = n->w + n->off[P_U];
-    P.m = n->mom + n->off[P_U];
-    P.v = n->vel + n->off[P_U];
-    P.g = n->g + n->off[P_U];
-    P.wb = n->wb + n->off[P_U];
-    P.bw = n->w + n->off[P_BU];
-    P.bm = n->mom + n->off[P_BU];
-    P.bv = n->vel + n->off[P_BU];
-    P.bg = n->g + n->off[P_BU];
-    P.O = n->O;
-    P.scale = 1.0f / (float)((long long)B * n->out);
-    P.loss = n->part;
-    return P;
-}
-
-int head_grid(const pdhcg_b200_mlp_s *n) { return std::min((n->out + HJ - 1) / HJ, 2 * 148); }
-constexpr size_t HEAD_SMEM_PREDICT = offsetof(HeadSmem, d), HEAD_SMEM = sizeof(HeadSmem);
-
 // o of the rows that trunk_forward took, into n->O
-int head_forward(pdhcg_b200_mlp_s *n, int B)
+int head_forward(pdhcg_b200_mlp_s *n, int B, bool training)
 {
     cudaStream_t s = n->s;
-    if (fused_head(n, B)) {
+    const bf16 *U = n->wb + n->off[P_U];
+    const float *bu = n->w + n->off[P_BU];
+    if (!training && fused_head(n, B)) {
         const int grid = std::min((n->out + HJ - 1) / HJ, 8 * 148);
-        launch_head<HEAD_PREDICT>(head_tile(n, B, nullptr), grid, HEAD_SMEM_PREDICT, s);
+        const HeadTile P{B, n->rank, n->out, n->Z, U, bu, n->O};
+        if (head_vec(P))
+            head_tile_kernel<true><<<grid, 256, 0, s>>>(P);
+        else
+            head_tile_kernel<false><<<grid, 256, 0, s>>>(P);
     } else {
-        if (gemm<false, true>(B, n->out, n->rank, n->Z, n->rank, n->wb + n->off[P_U], n->rank, n->O, n->out, 1.0f, 0.0f,
-                              s, n->ws))
+        if (gemm<false, true>(B, n->out, n->rank, n->Z, n->rank, U, n->rank, n->O, n->out, 1.0f, 0.0f, s, n->ws))
             return -1;
-        bias_act_kernel<<<blocks_for((long long)B * n->out), 256, 0, s>>>(B, n->out, n->O, n->w + n->off[P_BU], 0);
+        bias_act_kernel<<<blocks_for((long long)B * n->out), 256, 0, s>>>(B, n->out, n->O, bu, 0);
     }
     MCK(cudaGetLastError());
     return 0;
 }
 
 // Forward and backward of one minibatch: the loss is added to n->acc on the
-// device (no host wait); the gradient goes to n->g, except that with adam
-// the parameters are updated (the fused output head's from registers, the
-// others after the whole gradient is there).
+// device (no host wait), the gradient goes to n->g, and with adam the
+// parameters are updated.
 int step(pdhcg_b200_mlp_s *n, int B, const float *X, const float *T, const float *TL, const AdamArgs *adam)
 {
     cudaStream_t s = n->s;
@@ -1247,106 +833,45 @@ int step(pdhcg_b200_mlp_s *n, int B, const float *X, const float *T, const float
     const float *wp = n->w + n->off[P_WP];
     float *g = n->g;
     const long long tot = (long long)B * n->out;
-    const bool fused = fused_head(n, B);
-    if (fused) {
-        const int grid = head_grid(n);
-        const size_t need = (size_t)grid * B * n->rank;
-        if (grow_ws(n->ws, need))
-            return -1;
-        HeadTile P = head_tile(n, B, T);
-        P.part = n->ws.p;
-        if (adam) {
-            P.a = *adam;
-            launch_head<HEAD_ADAM>(P, grid, HEAD_SMEM, s);
-        } else {
-            launch_head<HEAD_GRAD>(P, grid, HEAD_SMEM, s);
-        }
-        head_fold_kernel<<<(B * n->rank + 31) / 32 + 1, 256, 0, s>>>(B * n->rank, grid, n->ws.p, n->dZ, n->part,
-                                                                    (double)tot, n->hloss, (B + SM_W - 1) / SM_W,
-                                                                    n->acc);
-    } else {
-        if (head_forward(n, B))
-            return -1;
-        int nb = blocks_for(tot);
-        mse_kernel<<<nb, 256, 0, s>>>(tot, n->O, T, 1.0f / (float)tot, n->dO, n->part);
-        loss_fold_kernel<<<1, 256, 0, s>>>(n->part, nb, (double)tot, n->hloss,
-                                           small_trunk(B) ? (B + SM_W - 1) / SM_W : 1, n->acc);
-        // dU = dO^T Z, dbu = colsum dO, dZ = dO U
-        if (gemm<true, false>(n->out, n->rank, B, n->dO, n->out, n->Z, n->rank, g + n->off[P_U], n->rank, 1.0f, 0.0f, s,
-                              n->ws))
-            return -1;
-        colsum_kernel<<<blocks_for(n->out), 256, 0, s>>>(B, n->out, n->dO, g + n->off[P_BU]);
-        if (gemm<false, false>(B, n->rank, n->out, n->dO, n->out, U, n->rank, n->dZ, n->rank, 1.0f, 0.0f, s, n->ws))
-            return -1;
-    }
-    if (small_trunk(B)) {
-        BackArgs b3{}, b2{}, b1{};
-        auto back = [&](BackArgs &b, int out, int in, const float *dY, const bf16 *W, const float *Xin, float *dX,
-                        const float *mask, int pw, int pb) {
-            b.dx.M = B;
-            b.dx.N = in;
-            b.dx.K = out;
-            b.dx.A = dY;
-            b.dx.lda = out;
-            b.dx.B = W;
-            b.dx.ldb = in;
-            b.dx.C = dX;
-            b.dx.mask = mask;
-            b.dx.vec = word_pairs(out, dY, nullptr);
-            b.dw.M = out;
-            b.dw.N = in;
-            b.dw.K = B;
-            b.dw.A = dY;
-            b.dw.lda = out;
-            b.dw.B = Xin;
-            b.dw.ldb = in;
-            b.dw.C = g + n->off[pw];
-            b.db = g + n->off[pb];
-            b.B = B;
-            b.H = n->hid;
-        };
-        back(b3, n->rank, n->hid, n->dZ, W3, n->H2, n->dH2, n->H2, P_W3, P_B3);
-        b3.dx.col = n->dLW;
-        b3.dx.row = wp;
-        b3.dlw = n->dLW;
-        b3.h2 = n->H2;
-        b3.gwp = g + n->off[P_WP];
-        b3.gbp = g + n->off[P_BP];
-        back(b2, n->hid, n->hid, n->dH2, W2, n->H1, n->dH1, n->H1, P_W2, P_B2);
-        back(b1, n->hid, n->in, n->dH1, nullptr, X, nullptr, nullptr, P_W1, P_B1);
-        const int hb = (n->hid + 32 * SM_W - 1) / (32 * SM_W);
-        small_back_kernel<true, true><<<b3.dx.tiles() + b3.dw.tiles() + hb, 32 * SM_W, 0, s>>>(b3);
-        small_back_kernel<false, true><<<b2.dx.tiles() + b2.dw.tiles(), 32 * SM_W, 0, s>>>(b2);
-        small_back_kernel<false, false><<<b1.dw.tiles(), 32 * SM_W, 0, s>>>(b1);
-    } else {
-        // z = W3 h2 + b3
-        if (gemm<true, false>(n->rank, n->hid, B, n->dZ, n->rank, n->H2, n->hid, g + n->off[P_W3], n->hid, 1.0f, 0.0f, s,
-                              n->ws))
-            return -1;
-        colsum_kernel<<<blocks_for(n->rank), 256, 0, s>>>(B, n->rank, n->dZ, g + n->off[P_B3]);
-        if (gemm<false, false>(B, n->hid, n->rank, n->dZ, n->rank, W3, n->hid, n->dH2, n->hid, 1.0f, 0.0f, s, n->ws))
-            return -1;
-        // log-weight head
-        head_back_kernel<<<blocks_for(n->hid), 256, 0, s>>>(B, n->hid, n->H2, wp, n->dLW, n->dH2, g + n->off[P_WP],
-                                                             g + n->off[P_BP]);
-        relu_back_kernel<<<blocks_for((long long)B * n->hid), 256, 0, s>>>((long long)B * n->hid, n->dH2, n->H2);
-        // h2 = relu(W2 h1 + b2)
-        if (gemm<true, false>(n->hid, n->hid, B, n->dH2, n->hid, n->H1, n->hid, g + n->off[P_W2], n->hid, 1.0f, 0.0f, s,
-                              n->ws))
-            return -1;
-        colsum_kernel<<<blocks_for(n->hid), 256, 0, s>>>(B, n->hid, n->dH2, g + n->off[P_B2]);
-        if (gemm<false, false>(B, n->hid, n->hid, n->dH2, n->hid, W2, n->hid, n->dH1, n->hid, 1.0f, 0.0f, s, n->ws))
-            return -1;
-        relu_back_kernel<<<blocks_for((long long)B * n->hid), 256, 0, s>>>((long long)B * n->hid, n->dH1, n->H1);
-        // h1 = relu(W1 x + b1)
-        if (gemm<true, false>(n->hid, n->in, B, n->dH1, n->hid, X, n->in, g + n->off[P_W1], n->in, 1.0f, 0.0f, s, n->ws))
-            return -1;
-        colsum_kernel<<<blocks_for(n->hid), 256, 0, s>>>(B, n->hid, n->dH1, g + n->off[P_B1]);
-    }
+    if (head_forward(n, B, true))
+        return -1;
+    int nb = blocks_for(tot);
+    mse_kernel<<<nb, 256, 0, s>>>(tot, n->O, T, 1.0f / (float)tot, n->dO, n->part);
+    loss_fold_kernel<<<1, 256, 0, s>>>(n->part, nb, (double)tot, n->hloss, n->acc);
+    // dU = dO^T Z, dbu = colsum dO, dZ = dO U
+    if (gemm<true, false>(n->out, n->rank, B, n->dO, n->out, n->Z, n->rank, g + n->off[P_U], n->rank, 1.0f, 0.0f, s,
+                          n->ws))
+        return -1;
+    colsum_kernel<<<blocks_for(n->out), 256, 0, s>>>(B, n->out, n->dO, g + n->off[P_BU]);
+    if (gemm<false, false>(B, n->rank, n->out, n->dO, n->out, U, n->rank, n->dZ, n->rank, 1.0f, 0.0f, s, n->ws))
+        return -1;
+    // z = W3 h2 + b3
+    if (gemm<true, false>(n->rank, n->hid, B, n->dZ, n->rank, n->H2, n->hid, g + n->off[P_W3], n->hid, 1.0f, 0.0f, s,
+                          n->ws))
+        return -1;
+    colsum_kernel<<<blocks_for(n->rank), 256, 0, s>>>(B, n->rank, n->dZ, g + n->off[P_B3]);
+    if (gemm<false, false>(B, n->hid, n->rank, n->dZ, n->rank, W3, n->hid, n->dH2, n->hid, 1.0f, 0.0f, s, n->ws))
+        return -1;
+    // log-weight head
+    head_back_kernel<<<blocks_for(n->hid), 256, 0, s>>>(B, n->hid, n->H2, wp, n->dLW, n->dH2, g + n->off[P_WP],
+                                                         g + n->off[P_BP]);
+    relu_back_kernel<<<blocks_for((long long)B * n->hid), 256, 0, s>>>((long long)B * n->hid, n->dH2, n->H2);
+    // h2 = relu(W2 h1 + b2)
+    if (gemm<true, false>(n->hid, n->hid, B, n->dH2, n->hid, n->H1, n->hid, g + n->off[P_W2], n->hid, 1.0f, 0.0f, s,
+                          n->ws))
+        return -1;
+    colsum_kernel<<<blocks_for(n->hid), 256, 0, s>>>(B, n->hid, n->dH2, g + n->off[P_B2]);
+    if (gemm<false, false>(B, n->hid, n->hid, n->dH2, n->hid, W2, n->hid, n->dH1, n->hid, 1.0f, 0.0f, s, n->ws))
+        return -1;
+    relu_back_kernel<<<blocks_for((long long)B * n->hid), 256, 0, s>>>((long long)B * n->hid, n->dH1, n->H1);
+    // h1 = relu(W1 x + b1)
+    if (gemm<true, false>(n->hid, n->in, B, n->dH1, n->hid, X, n->in, g + n->off[P_W1], n->in, 1.0f, 0.0f, s, n->ws))
+        return -1;
+    colsum_kernel<<<blocks_for(n->hid), 256, 0, s>>>(B, n->hid, n->dH1, g + n->off[P_B1]);
     if (adam) {
-        const long long skip0 = fused ? n->off[P_U] : n->total, skip1 = fused ? n->off[P_WP] : n->total;
-        adam_outer_kernel<<<blocks_for(n->total - (skip1 - skip0)), 256, 0, s>>>(n->total, skip0, skip1, n->w, n->g,
-                                                                                n->mom, n->vel, n->wb, *adam);
+        adam_kernel<<<blocks_for(n->total), 256, 0, s>>>(n->total, n->w, n->g, n->mom, n->vel, adam->lr, adam->b1,
+                                                         adam->b2, adam->c1, adam->c2, adam->eps);
+        to_bf16_kernel<<<blocks_for(n->total), 256, 0, s>>>(n->total, n->w, n->wb);
     }
     MCK(cudaGetLastError());
     return 0;
@@ -1357,17 +882,6 @@ int refresh_bf16(pdhcg_b200_mlp_s *n)
     to_bf16_kernel<<<blocks_for(n->total), 256, 0, n->s>>>(n->total, n->w, n->wb);
     MCK(cudaGetLastError());
     return 0;
-}
-
-cudaError_t head_attributes()
-{
-    for (auto k : {head_tile_kernel<HEAD_GRAD, false>, head_tile_kernel<HEAD_GRAD, true>,
-                   head_tile_kernel<HEAD_ADAM, false>, head_tile_kernel<HEAD_ADAM, true>}) {
-        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HEAD_SMEM);
-        if (e != cudaSuccess)
-            return e;
-    }
-    return cudaSuccess;
 }
 
 // splitmix64 -> uniform in [-1, 1)
@@ -1426,7 +940,6 @@ pdhcg_b200_mlp_t *pdhcg_b200_mlp_create(int in_dim, int hidden, int rank, int ou
         cudaMemcpyAsync(n->w, h.data(), o * sizeof(float), cudaMemcpyHostToDevice, n->s) != cudaSuccess ||
         cudaMemsetAsync(n->mom, 0, o * sizeof(float), n->s) != cudaSuccess ||
         cudaMemsetAsync(n->vel, 0, o * sizeof(float), n->s) != cudaSuccess ||
-        head_attributes() != cudaSuccess ||
         refresh_bf16(n) != 0 || cudaStreamSynchronize(n->s) != cudaSuccess) {
         std::fprintf(stderr, "[pdhcg_b200_mlp_create] device allocation failed.\n");
         pdhcg_b200_mlp_free(n);
@@ -1484,7 +997,7 @@ int pdhcg_b200_mlp_predict(pdhcg_b200_mlp_t *n, int batch, const float *theta, f
     if (ensure_acts(n, batch))
         return -1;
     MCK(cudaMemcpyAsync(n->X, theta, (size_t)batch * n->in * sizeof(float), cudaMemcpyHostToDevice, n->s));
-    if (trunk_forward(n, batch, n->X, nullptr) || head_forward(n, batch))
+    if (trunk_forward(n, batch, n->X, nullptr) || head_forward(n, batch, false))
         return -1;
     MCK(cudaMemcpyAsync(out, n->O, (size_t)batch * n->out * sizeof(float), cudaMemcpyDeviceToHost, n->s));
     if (logw)

@@ -1,6 +1,6 @@
-"""The warm-start network's minibatch kernels against the CPU oracle where
-their tiles end: 64 rows and 64 outputs a head tile, rank 64, 32 x 16 hidden
-tiles, word loads only for even sizes."""
+"""The warm-start network against the CPU oracle where the tiles of its
+predictions and of its training products end: 64 rows and 64 outputs a head
+tile, rank 64, 32 x 16 hidden tiles, word loads only for even sizes."""
 import ctypes as C
 
 import numpy as np
@@ -44,7 +44,7 @@ def test_loss_gradient_and_prediction(lib, dims, batch):
         np.testing.assert_allclose(out, oo, rtol=0, atol=1e-4 * np.abs(oo).max())
         np.testing.assert_allclose(lw, lwo, rtol=0, atol=1e-4 * np.abs(lwo).max())
         # one training step moves every parameter against its gradient by lr m / (sqrt(v) + eps)
-        # = lr g / (|g| + eps): the head's update is in its own kernel
+        # = lr g / (|g| + eps)
         la = C.c_double()
         assert lib.pdhcg_b200_mlp_train(net, batch, _fp(x), _fp(t), _fp(tl), 1, batch, 1e-3, C.byref(la)) == 0
         w1 = np.zeros_like(w)
