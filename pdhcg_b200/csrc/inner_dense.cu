@@ -641,7 +641,7 @@ int dense_blocks(int k, int tiles, int S, int sms)
     if (k < 1 || k > DENSE_MAX_K || tiles < 1)
         return 0;
     for (const DenseForm &f : {dense_form<double>(k, S), dense_form<float>(k, S)}) {
-        CK(cudaFuncSetAttribute(f.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem));
+        allow_shared(f.kernel, DENSE_SMEM);
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f.kernel, f.threads, f.smem));
         if (per_sm < 1)

@@ -300,7 +300,7 @@ int bb_small_blocks(int n, long long nnz, int sms)
     if (!sh.kernel)
         return 0;
     const size_t smem = (size_t)sh.cap * 12;
-    CK(cudaFuncSetAttribute(sh.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared(sh.kernel, smem); // (one cap per kernel)
     if (sh.cluster) {
         CK(cudaFuncSetAttribute(sh.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         cudaLaunchAttribute at;

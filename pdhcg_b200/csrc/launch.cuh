@@ -42,6 +42,16 @@ inline int grid_for(long long work, int per_block, int cap = 148 * 16)
     return (int)g;
 }
 
+// Lets `kernel` be launched with up to `bytes` of dynamic shared memory.  The
+// limit is state of the kernel on the device, shared by every thread that
+// solves: all callers pass one constant per kernel, the most that any of its
+// launches takes, so that no caller lowers it under another's launch.
+template <typename K>
+void allow_shared(K kernel, size_t bytes)
+{
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
 // Blocks of `kernel` (TPB threads, static shared memory) resident at once
 // on the current device; cached per kernel and device.
 inline int resident_blocks(const void *kernel)

@@ -372,7 +372,7 @@ ResidentPlan resident_plan(int n, int m, long long nnz, int sms)
             return ResidentPlan{};
     }
     const void *f = p.blocks == 1 ? (const void *)resident_kernel<true> : (const void *)resident_kernel<false>;
-    CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RESIDENT_SMEM));
+    allow_shared(f, RESIDENT_SMEM);
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, RT, p.smem));
     return per_sm >= 1 ? p : ResidentPlan{};

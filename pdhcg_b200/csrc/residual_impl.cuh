@@ -6,13 +6,18 @@
 
 namespace pdhcg {
 
+// most dynamic shared memory of the two kernels: the scratch of the largest
+// block held in registers for every warp; a thread block's for one PSD block
+constexpr size_t RESIDUAL_SMEM = WARPS * psd_work_doubles(PSD_MAX_ORDER) * sizeof(double);
+constexpr size_t RESIDUAL_PSD_SMEM = 190 * 1024;
+
 template <typename VT>
 void launch_residual(const ResidualData<VT> &D, const ResidualParams &P, int S, bool fixed, int blocks, cudaStream_t s)
 {
     const size_t dyn = (size_t)D.psd_shared * WARPS * sizeof(double);
     auto go = [&](auto kernel) {
         if (dyn > 0)
-            CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+            allow_shared(kernel, RESIDUAL_SMEM);
         kernel<<<blocks, TPB, dyn, s>>>(D, P);
     };
     if (fixed) // one slot class for problems with fixed cone slots
@@ -31,7 +36,7 @@ void launch_residual_psd(const ResidualData<VT> &D, const ResidualParams &P, con
                          int first, int blocks, cudaStream_t s)
 {
     const size_t dyn = residual_psd_smem(max_order);
-    CK(cudaFuncSetAttribute(residual_psd_kernel<VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    allow_shared(residual_psd_kernel<VT>, RESIDUAL_PSD_SMEM);
     residual_psd_kernel<VT><<<blocks, TPB, dyn, s>>>(D, P, ids, nids, first);
 }
 

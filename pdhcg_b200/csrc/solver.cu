@@ -1463,7 +1463,7 @@ double Solve::power_sigma2(double *v0)
     const int m = m_, n = n_, max_iter = prm_.sv_max_iter;
     if (max_iter < 1)
         return 1.0;
-    CK(cudaFuncSetAttribute((const void *)lanczos_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LANCZOS_SMEM));
+    allow_shared(lanczos_kernel, LANCZOS_SMEM);
     const int limit = std::min(LANCZOS_MAX, std::min(m, 2 * max_iter) + 1); // steps at which T is exact or given up
     int dev = 0, nsm = 0;
     CK(cudaGetDevice(&dev));

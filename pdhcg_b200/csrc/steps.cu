@@ -61,7 +61,7 @@ int launch_primal_cones(const StepData<T> &D, const StepParams &P, const ConeSpl
         // memory (order 112); a warp per block on global scratch beyond
         const size_t dyn = psd_work_doubles(D.psd_max) * sizeof(double);
         auto go = [&](auto kernel, int threads) {
-            CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+            allow_shared(kernel, PSD_STEP_SMEM);
             kernel<<<grid_for(sp.n_psd, 1), threads, dyn, s>>>(D, P, sp.psd_d, sp.n_psd);
         };
         if (D.psd_max > 0 && dyn <= PSD_STEP_SMEM) {
