@@ -890,6 +890,9 @@ private:
     double best_fp32_kkt_ = INFINITY;
     int fp32_stall_ = 0;
     double *partials_ = nullptr, *scal_d_ = nullptr, *h_scal_ = nullptr;
+    // scal_d_ and its host mirror: the residual's sums, two fixed-point errors,
+    // and (as an int) the flag of an inner solve whose wait ran out
+    static constexpr int SC_FLAG = RS_COUNT + 2 * FP_COUNT, SC_COUNT = SC_FLAG + 1;
     int *res_ops_d_ = nullptr, *fpe_ops_d_ = nullptr, *norm_ops_d_ = nullptr;
     int *rayn_ops_d_ = nullptr, *ray_ops_d_ = nullptr;
     double *ray_d_ = nullptr; // [RN_COUNT + RY_COUNT] folded certificate scalars
@@ -1383,6 +1386,7 @@ void Solve::setup_bb_special(int nsm)
     }
     if (bb_small_blocks_ > 0 || bb_dense_blocks_ > 0) {
         bb_slots_ = bb_small_blocks_ > 0 ? make_slots(bb_small_blocks_, 2) : make_slots(bb_dense_blocks_, k + 2);
+        bb_slots_.err = (int *)(scal_d_ + SC_FLAG); // read with every evaluation's scalars
     }
 }
 
@@ -2323,10 +2327,12 @@ void Solve::run_resident(double elapsed)
 void Solve::read_residual()
 {
     cudaStream_t s = st_;
-    CK(cudaMemcpyAsync(h_scal_, scal_d_, (RS_COUNT + 2 * FP_COUNT) * sizeof(double), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(h_scal_, scal_d_, SC_COUNT * sizeof(double), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     harvest_step_events();
     const double *r = h_scal_;
+    if (*(const int *)(r + SC_FLAG)) // the iterates since are not those of the method
+        throw CudaError("a wait of the blocks for one another ran out (inner solve)");
     bool l2 = prm_.optimality_norm == NORM_TYPE_L2;
     auto nrm = [&](double v) { return l2 ? std::sqrt(v) : v; };
     resolve_fpe(r);
@@ -2602,8 +2608,8 @@ void Solve::setup_scratch()
                          fpe_col_blocks_ + fpe_row_blocks_,
                          res_rows_blocks_ + fpe_col_blocks_, 148 * 4});
     partials_ = ar_.alloc<double>((size_t)maxb * RS_COUNT);
-    scal_d_ = ar_.alloc<double>(RS_COUNT + 2 * FP_COUNT);
-    CK(cudaMemsetAsync(scal_d_, 0, (RS_COUNT + 2 * FP_COUNT) * sizeof(double), st_));
+    scal_d_ = ar_.alloc<double>(SC_COUNT);
+    CK(cudaMemsetAsync(scal_d_, 0, SC_COUNT * sizeof(double), st_));
     h_scal_ = pinned_scalars();
     {
         int nop = prm_.optimality_norm == NORM_TYPE_L2 ? RSUM : RMAX;
@@ -2723,8 +2729,6 @@ pdhcg_result_t *Solve::run()
         int inner = 0;
         CK(cudaMemcpyAsync(&inner, bb_inner_, sizeof(int), cudaMemcpyDeviceToHost, st_));
         CK(cudaStreamSynchronize(st_));
-        if (bb_slots_.err)
-            check_slots(bb_slots_, "inner solve");
         inner_total_ += inner;
     }
     auto t_res = std::chrono::steady_clock::now();
