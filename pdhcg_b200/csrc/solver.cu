@@ -1468,7 +1468,8 @@ double Solve::power_sigma2(double *v0)
     if (max_iter < 1)
         return 1.0;
     allow_shared(lanczos_kernel, LANCZOS_SMEM);
-    const int limit = std::min(LANCZOS_MAX, std::min(m, 2 * max_iter) + 1); // steps at which T is exact or given up
+    // steps at which T is exact or given up (max_iter may be INT_MAX: no limit)
+    const int limit = (int)std::min<long long>(LANCZOS_MAX, std::min<long long>(m, 2LL * max_iter) + 1);
     int dev = 0, nsm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -1506,7 +1507,7 @@ double Solve::power_sigma2(double *v0)
         al.assign(h.begin() + 4, h.begin() + 4 + have);
         be.assign(h.begin() + 4 + LANCZOS_MAX, h.begin() + 4 + LANCZOS_MAX + have);
         s2 = power_on_tridiagonal(al, be, max_iter, prm_.sv_tol, its);
-        if (have < j || 2 * its + 1 < have || (its == last_its && std::fabs(s2 - last) <= 1e-13 * s2))
+        if (have < j || 2LL * its + 1 < have || (its == last_its && std::fabs(s2 - last) <= 1e-13 * s2))
             break;
         last = s2;
         last_its = its;
