@@ -202,7 +202,8 @@ struct ResidentPlan {
     int cap_a, cap_at, rows, vars; // per block: staged entries of A and A^T, rows, variables
     size_t smem;
 };
-ResidentPlan resident_plan(int n, int m, long long nnz, int sms);
+ResidentPlan resident_plan(int n, int m, long long nnz, const int *A_rp, const int *At_rp, int sms, int *shares,
+                           cudaStream_t s);
 void launch_resident(const ResidentPlan &p, const ResidentData &D, const ResidentParams &P, const GridSlots &S,
                      cudaStream_t s);
 

@@ -57,17 +57,14 @@ __global__ void __launch_bounds__(RT, 1) resident_kernel(ResidentData D, Residen
     double *xrs = take(ONE ? L.vars : 0);
     int *trp = (int *)p, *arp = trp + L.vars + 1, *tci = arp + L.rows + 1, *aci = tci + L.cap_at;
     const int tb = D.At_rp[c0], te = D.At_rp[c1], ab = D.A_rp[w0], ae = D.A_rp[w1];
-    const bool st_t = te - tb <= L.cap_at, st_a = ae - ab <= L.cap_a;
-    if (st_t)
-        for (int k = tid; k < te - tb; k += RT) {
-            tv[k] = D.At_v[tb + k];
-            tci[k] = D.At_ci[tb + k];
-        }
-    if (st_a)
-        for (int k = tid; k < ae - ab; k += RT) {
-            av[k] = D.A_v[ab + k];
-            aci[k] = D.A_ci[ab + k];
-        }
+    for (int k = tid; k < te - tb; k += RT) {
+        tv[k] = D.At_v[tb + k];
+        tci[k] = D.At_ci[tb + k];
+    }
+    for (int k = tid; k < ae - ab; k += RT) {
+        av[k] = D.A_v[ab + k];
+        aci[k] = D.A_ci[ab + k];
+    }
     for (int j = tid; j <= nv; j += RT)
         trp[j] = D.At_rp[c0 + j] - tb;
     for (int i = tid; i <= nr; i += RT)
@@ -87,42 +84,42 @@ __global__ void __launch_bounds__(RT, 1) resident_kernel(ResidentData D, Residen
         y0[i] = D.y0[w0 + i];
         y[i] = D.y[w0 + i];
     }
-    // row r's product with v, the entries in order, four gathers in flight
-    auto dot = [](bool staged, const double *sv, const int *sc, const double *gv, const int *gc, int b, int e,
-                  const double *v, bool shared) {
+    // row r's product with v, the entries in order, eight gathers in flight
+    auto dot = [](const double *sv, const int *sc, int b, int e, const double *v, bool shared) {
         double s = 0.0;
         auto ldv = [&](const double *a) { return shared ? *a : __ldcg(a); };
-        if (staged) {
-            int k = b;
-            for (; k + 4 <= e; k += 4) {
-                const double a0 = ldv(v + sc[k]), a1 = ldv(v + sc[k + 1]), a2 = ldv(v + sc[k + 2]),
-                             a3 = ldv(v + sc[k + 3]);
-                s += sv[k] * a0;
-                s += sv[k + 1] * a1;
-                s += sv[k + 2] * a2;
-                s += sv[k + 3] * a3;
-            }
-            const bool p0 = k < e, p1 = k + 1 < e, p2 = k + 2 < e;
-            const double a0 = p0 ? ldv(v + sc[k]) : 0.0, a1 = p1 ? ldv(v + sc[k + 1]) : 0.0,
-                         a2 = p2 ? ldv(v + sc[k + 2]) : 0.0;
-            if (p0)
-                s += sv[k] * a0;
-            if (p1)
-                s += sv[k + 1] * a1;
-            if (p2)
-                s += sv[k + 2] * a2;
-        } else {
-            for (int k = b; k < e; ++k)
-                s += gv[k] * ldv(v + gc[k]);
+        int k = b;
+        for (; k + 8 <= e; k += 8) {
+            double a[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                a[u] = ldv(v + sc[k + u]);
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                s += sv[k + u] * a[u];
         }
+        if (k + 4 <= e) {
+            const double a0 = ldv(v + sc[k]), a1 = ldv(v + sc[k + 1]), a2 = ldv(v + sc[k + 2]),
+                         a3 = ldv(v + sc[k + 3]);
+            s += sv[k] * a0;
+            s += sv[k + 1] * a1;
+            s += sv[k + 2] * a2;
+            s += sv[k + 3] * a3;
+            k += 4;
+        }
+        const bool p0 = k < e, p1 = k + 1 < e, p2 = k + 2 < e;
+        const double a0 = p0 ? ldv(v + sc[k]) : 0.0, a1 = p1 ? ldv(v + sc[k + 1]) : 0.0,
+                     a2 = p2 ? ldv(v + sc[k + 2]) : 0.0;
+        if (p0)
+            s += sv[k] * a0;
+        if (p1)
+            s += sv[k + 1] * a1;
+        if (p2)
+            s += sv[k + 2] * a2;
         return s;
     };
-    auto col_dot = [&](int j, const double *v, bool shared) {
-        return dot(st_t, tv, tci, D.At_v + tb, D.At_ci + tb, trp[j], trp[j + 1], v, shared);
-    };
-    auto row_dot_ = [&](int i, const double *v, bool shared) {
-        return dot(st_a, av, aci, D.A_v + ab, D.A_ci + ab, arp[i], arp[i + 1], v, shared);
-    };
+    auto col_dot = [&](int j, const double *v, bool shared) { return dot(tv, tci, trp[j], trp[j + 1], v, shared); };
+    auto row_dot_ = [&](int i, const double *v, bool shared) { return dot(av, aci, arp[i], arp[i + 1], v, shared); };
     const bool hasq = D.q != nullptr;
     ResidentState s = *D.state;
     s.optimal = s.restarts = s.evaluations = 0;
@@ -338,37 +335,82 @@ static size_t resident_smem(const ResidentPlan &p)
 
 constexpr size_t RESIDENT_SMEM = 216 * 1024;
 
+// Most entries of a block's rows of M when its rows are dealt to `blocks` (by
+// count, as the kernel deals them).
+__device__ int most_entries(const int *rp, int rows, int blocks)
+{
+    int most = 0;
+    for (int b = threadIdx.x; b < blocks; b += blockDim.x)
+        most = max(most, rp[(long long)rows * (b + 1) / blocks] - rp[(long long)rows * b / blocks]);
+    return most;
+}
+
+// out[0..3]: A's and A^T's most entries of a block at b0 blocks, then at b1
+__global__ void resident_share_kernel(int n, int m, const int *A_rp, const int *At_rp, int b0, int b1, int *out)
+{
+    __shared__ int most[4];
+    if (threadIdx.x < 4)
+        most[threadIdx.x] = 0;
+    __syncthreads();
+    atomicMax(&most[0], most_entries(A_rp, m, b0));
+    atomicMax(&most[1], most_entries(At_rp, n, b0));
+    atomicMax(&most[2], most_entries(A_rp, m, b1));
+    atomicMax(&most[3], most_entries(At_rp, n, b1));
+    __syncthreads();
+    if (threadIdx.x < 4)
+        out[threadIdx.x] = most[threadIdx.x];
+}
+
 // One block when everything fits in it with at most RESIDENT_ONE variables or
 // rows (measured against a grid: one block's barrier is 50 cycles, the grid's
 // 1700, and a block's FP64 units take 4 cycles per variable); otherwise about
-// a thread per variable, at most one block per SM.  The entries of a block's
-// rows may be a quarter over the mean; a block over that reads its matrix
-// from L2.
+// a thread per variable, at most one block per SM.  Every block stages its
+// rows of A and A^T, so the fullest block decides whether the problem fits: a
+// block that reads a matrix from L2 instead, a row per thread, is waited for
+// by all others at both barriers (columns of 64 entries side by side in
+// 150000 variables: 102 us per iteration, 37 by the kernels of one launch per
+// step; 60 entries in 100000: 50 against 35).
 constexpr int RESIDENT_ONE = 2048;
 
-ResidentPlan resident_plan(int n, int m, long long nnz, int sms)
+// shares: 4 ints of device scratch
+ResidentPlan resident_plan(int n, int m, long long nnz, const int *A_rp, const int *At_rp, int sms, int *shares,
+                           cudaStream_t s)
 {
-    auto plan = [&](int blocks) {
+    auto plan = [&](int blocks, long long a, long long at) {
         ResidentPlan p{};
         p.blocks = blocks;
         p.vars = (n + blocks - 1) / blocks;
         p.rows = (m + blocks - 1) / blocks;
-        const long long per = (nnz + blocks - 1) / blocks;
-        p.cap_a = p.cap_at = (int)std::min<long long>(nnz, blocks == 1 ? nnz : per + per / 4 + 64);
+        p.cap_a = (int)a;
+        p.cap_at = (int)at;
         p.smem = resident_smem(p);
         return p;
     };
-    ResidentPlan p{};
+    auto fits = [](const ResidentPlan &p) { return p.smem <= RESIDENT_SMEM && p.vars <= 2 * RT && p.rows <= 2 * RT; };
     if (nnz > (1 << 24))
-        return p;
-    if (std::max(n, m) <= RESIDENT_ONE && (p = plan(1)).smem <= RESIDENT_SMEM)
-        ;
-    else {
-        const int blocks = std::min(sms, std::max(2, (std::max(n, m) + RT - 1) / RT * 2));
-        p = plan(blocks);
-        if (p.smem > RESIDENT_SMEM)
-            p = plan(sms);
-        if (p.smem > RESIDENT_SMEM || p.vars > 2 * RT || p.rows > 2 * RT)
+        return ResidentPlan{};
+    ResidentPlan p{};
+    if (std::max(n, m) <= RESIDENT_ONE)
+        p = plan(1, nnz, nnz);
+    if (p.blocks == 0 || p.smem > RESIDENT_SMEM) {
+        const long long mean = (nnz + sms - 1) / sms;
+        if (!fits(plan(sms, mean, mean)))
+            return ResidentPlan{};
+        int blocks = std::min(sms, std::max(2, (std::max(n, m) + RT - 1) / RT * 2));
+        // with so many entries that a quarter over the mean would not fit, a
+        // block per SM: their gathers are what an iteration waits for (rows of
+        // 60 entries, 5000 variables: 19.0 us on 20 blocks, 12.1 on 148)
+        const long long quarter = (nnz + blocks - 1) / blocks * 5 / 4 + 64;
+        if (!fits(plan(blocks, quarter, quarter)))
+            blocks = sms;
+        int h[4];
+        resident_share_kernel<<<1, TPB, 0, s>>>(n, m, A_rp, At_rp, blocks, sms, shares);
+        CK(cudaMemcpyAsync(h, shares, sizeof(h), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        p = plan(blocks, h[0], h[1]);
+        if (!fits(p))
+            p = plan(sms, h[2], h[3]);
+        if (!fits(p))
             return ResidentPlan{};
     }
     const void *f = p.blocks == 1 ? (const void *)resident_kernel<true> : (const void *)resident_kernel<false>;

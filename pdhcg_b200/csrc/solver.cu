@@ -2198,10 +2198,9 @@ void Solve::setup_resident()
     int dev = 0, nsm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    res_plan_ = resident_plan(n_, m_, A_.nnz, nsm);
+    res_plan_ = resident_plan(n_, m_, A_.nnz, A_.rp, At_.rp, nsm, ar_.alloc<int>(4), st_);
     if (res_plan_.blocks == 0)
         return;
-    cudaStream_t s = st_;
     res_state_ = ar_.alloc<ResidentState>(1);
     res_slots_ = make_slots(res_plan_.blocks, RESIDENT_SLOTS);
     static_assert(sizeof(ResidentState) <= 64 * sizeof(double), "the pinned scalar block holds the state");
