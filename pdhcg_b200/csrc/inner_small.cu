@@ -34,6 +34,13 @@ constexpr int SMALL_CLUSTER_NNZ = 64 * 1024;
 
 namespace cgc = cooperative_groups;
 
+// Gathers of one row in flight: an inner iteration waits for its longest row's
+// rounds.  Two rows a thread, Q = B'B with rows to about 20 entries, 1e4
+// variables, us per inner iteration at 8 / 12 / 16: 7.6 / 5.2 / 5.8; tridiagonal,
+// one row a thread, 2000 variables: 4.5 / 4.5 / 5.0.
+template <int V>
+constexpr int ROW_WIDTH = V == 1 ? 8 : 12;
+
 // Barriers and sums of the two forms.  fold: both values summed over the
 // launch's blocks, in block order, the same in every thread; also a barrier.
 // barrier: what any thread wrote to global memory is visible after it.
@@ -109,12 +116,10 @@ __global__ void __launch_bounds__(NT) bb_small_kernel(BBData D, BBParams P, Grid
     const int nb = gridDim.x, tid = threadIdx.x;
     const int r0 = (int)((long long)D.n * blockIdx.x / nb), r1 = (int)((long long)D.n * (blockIdx.x + 1) / nb);
     const int q0 = D.Q_rp[r0], q1 = D.Q_rp[r1];
-    const bool staged = q1 - q0 <= cap;
-    if (staged)
-        for (int e = tid; e < q1 - q0; e += NT) {
-            sc[e] = D.Q_ci[q0 + e];
-            sv[e] = D.Q_vf ? (double)D.Q_vf[q0 + e] : D.Q_v[q0 + e];
-        }
+    for (int e = tid; e < q1 - q0; e += NT) {
+        sc[e] = D.Q_ci[q0 + e];
+        sv[e] = D.Q_vf ? (double)D.Q_vf[q0 + e] : D.Q_v[q0 + e];
+    }
     if (!CLUSTER)
         grid_begin(S);
     const double inv_tau = 1.0 / P.tau;
@@ -143,42 +148,47 @@ __global__ void __launch_bounds__(NT) bb_small_kernel(BBData D, BBParams P, Grid
     __syncthreads();
     // the diagonal entries, whose operand the thread holds, leave the staged
     // rows (the later entries move up)
-    if (staged) {
 #pragma unroll
-        for (int v = 0; v < V; ++v) {
-            const int j = r0 + tid + NT * v;
-            int w = b[v];
-            for (int k = b[v]; k < e[v]; ++k) {
-                if (sc[k] == j) {
-                    dq[v] += sv[k];
-                } else {
-                    sc[w] = sc[k];
-                    sv[w] = sv[k];
-                    ++w;
-                }
+    for (int v = 0; v < V; ++v) {
+        const int j = r0 + tid + NT * v;
+        int w = b[v];
+        for (int k = b[v]; k < e[v]; ++k) {
+            if (sc[k] == j) {
+                dq[v] += sv[k];
+            } else {
+                sc[w] = sc[k];
+                sv[w] = sv[k];
+                ++w;
             }
-            e[v] = w;
         }
+        e[v] = w;
     }
-    // Q row . v (the diagonal's operand is own), eight gathers in flight
-    auto row = [&](const double *v, int k, int end, double diag, double own) {
-        double s = diag * own;
-        if (staged) {
-            for (; k < end; k += 8) {
-                double a[8];
+    // s = (Q w) of the thread's rows (the diagonal's operands are `own`), the rows
+    // side by side with ROW_W gathers of each in flight, entries in order
+    int longest = 0;
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    a[u] = k + u < end ? __ldcg(v + sc[k + u]) : 0.0;
+    for (int v = 0; v < V; ++v)
+        longest = max(longest, e[v] - b[v]);
+    constexpr int ROW_W = ROW_WIDTH<V>;
+    auto rows = [&](const double *w, const double (&own)[V], double (&s)[V]) {
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (k + u < end)
-                        s += sv[k + u] * a[u];
-            }
-        } else {
-            for (; k < end; ++k)
-                s += (D.Q_vf ? (double)D.Q_vf[q0 + k] : D.Q_v[q0 + k]) * __ldcg(v + D.Q_ci[q0 + k]);
+        for (int v = 0; v < V; ++v)
+            s[v] = dq[v] * own[v];
+#pragma unroll 1
+        for (int k = 0; k < longest; k += ROW_W) {
+            double a[V][ROW_W];
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+#pragma unroll
+                for (int u = 0; u < ROW_W; ++u)
+                    a[v][u] = b[v] + k + u < e[v] ? __ldcg(w + sc[b[v] + k + u]) : 0.0;
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+#pragma unroll
+                for (int u = 0; u < ROW_W; ++u)
+                    if (b[v] + k + u < e[v])
+                        s[v] += sv[b[v] + k + u] * a[v][u];
         }
-        return s;
     };
     // the projected step from `from` along M^-1 g; the partial of dir' M dir
     auto var_step = [&](double alpha, const double (&from)[V]) {
@@ -196,10 +206,12 @@ __global__ void __launch_bounds__(NT) bb_small_kernel(BBData D, BBParams P, Grid
         }
         return part;
     };
+    double qv[V];
+    rows(D.x, x, qv);
 #pragma unroll
     for (int v = 0; v < V; ++v) {
         dir[v] = xp[v] = 0.0;
-        g[v] = row(D.x, b[v], e[v], dq[v], x[v]) + cb[v];
+        g[v] = qv[v] + cb[v];
     }
     // A step's dir' M dir is wanted for the convergence test and the next step
     // length, both after the gradient at x_p is there; so the step only passes
@@ -211,9 +223,10 @@ __global__ void __launch_bounds__(NT) bb_small_kernel(BBData D, BBParams P, Grid
     for (;;) {
         double t = 0.0;
         if (it < D.limit) {
+            rows(D.xp, xp, qv);
 #pragma unroll
             for (int v = 0; v < V; ++v) {
-                const double gn = row(D.xp, b[v], e[v], dq[v], xp[v]) + cb[v] + inv_tau * (xp[v] - x[v]);
+                const double gn = qv[v] + cb[v] + inv_tau * (xp[v] - x[v]);
                 t += dir[v] * (gn - g[v]);
                 g[v] = gn;
             }
@@ -245,43 +258,45 @@ __global__ void __launch_bounds__(NT) bb_small_kernel(BBData D, BBParams P, Grid
 
 // Launch shapes.  Cluster: 16 blocks, the fewest threads that hold the
 // variables.  Grid: the smallest blocks that fit one per SM (a smaller block
-// reduces and synchronises faster).  cap: entries of Q staged per block.
+// reduces and synchronises faster).  cap: entries of Q that a block has room
+// for at least (the fullest block may raise it).
 struct SmallShape {
     const void *kernel;
     int threads, vars, cap;
-    bool cluster;
 };
 
-static SmallShape small_shape(int n, long long nnz, int sms)
+static SmallShape cluster_shape(int n)
 {
-    if (nnz - n <= SMALL_CLUSTER_NNZ) { // (every row of Q has a diagonal entry in practice)
-        const int cap = 8192;
-        if (n <= SMALL_CLUSTER * 128)
-            return {(const void *)bb_small_kernel<128, 1, true>, 128, 128, cap, true};
-        if (n <= SMALL_CLUSTER * 512)
-            return {(const void *)bb_small_kernel<512, 1, true>, 512, 512, cap, true};
-        if (n <= SMALL_CLUSTER * 1024)
-            return {(const void *)bb_small_kernel<512, 2, true>, 512, 1024, cap, true};
-    }
-    if (n <= sms * 128)
-        return {(const void *)bb_small_kernel<128, 1, false>, 128, 128, 2048, false};
-    if (n <= sms * 256)
-        return {(const void *)bb_small_kernel<256, 1, false>, 256, 256, 4096, false};
-    if (n <= sms * 512)
-        return {(const void *)bb_small_kernel<512, 1, false>, 512, 512, 8192, false};
-    if (n <= sms * 1024)
-        return {(const void *)bb_small_kernel<512, 2, false>, 512, 1024, 16384, false};
-    return {nullptr, 0, 0, 0, false};
+    if (n <= SMALL_CLUSTER * 128)
+        return {(const void *)bb_small_kernel<128, 1, true>, 128, 128, 8192};
+    if (n <= SMALL_CLUSTER * 512)
+        return {(const void *)bb_small_kernel<512, 1, true>, 512, 512, 8192};
+    if (n <= SMALL_CLUSTER * 1024)
+        return {(const void *)bb_small_kernel<512, 2, true>, 512, 1024, 8192};
+    return {nullptr, 0, 0, 0};
 }
 
-static cudaLaunchConfig_t small_config(const SmallShape &sh, int blocks, cudaLaunchAttribute *at, cudaStream_t s)
+static SmallShape grid_shape(int n, int sms)
+{
+    if (n <= sms * 128)
+        return {(const void *)bb_small_kernel<128, 1, false>, 128, 128, 2048};
+    if (n <= sms * 256)
+        return {(const void *)bb_small_kernel<256, 1, false>, 256, 256, 4096};
+    if (n <= sms * 512)
+        return {(const void *)bb_small_kernel<512, 1, false>, 512, 512, 8192};
+    if (n <= sms * 1024)
+        return {(const void *)bb_small_kernel<512, 2, false>, 512, 1024, 16384};
+    return {nullptr, 0, 0, 0};
+}
+
+static cudaLaunchConfig_t small_config(const SmallPlan &p, cudaLaunchAttribute *at, cudaStream_t s)
 {
     cudaLaunchConfig_t c = {};
-    c.gridDim = dim3(blocks);
-    c.blockDim = dim3(sh.threads);
-    c.dynamicSmemBytes = (size_t)sh.cap * 12;
+    c.gridDim = dim3(p.blocks);
+    c.blockDim = dim3(p.threads);
+    c.dynamicSmemBytes = (size_t)p.cap * 12;
     c.stream = s;
-    if (sh.cluster) {
+    if (p.cluster) {
         at->id = cudaLaunchAttributeClusterDimension;
         at->val.clusterDim.x = SMALL_CLUSTER;
         at->val.clusterDim.y = at->val.clusterDim.z = 1;
@@ -294,35 +309,69 @@ static cudaLaunchConfig_t small_config(const SmallShape &sh, int blocks, cudaLau
     return c;
 }
 
-int bb_small_blocks(int n, long long nnz, int sms)
+// most entries of a block's rows at b0 and at b1 blocks (rows dealt by count)
+__global__ void small_share_kernel(int n, const int *rp, int b0, int b1, int *out)
 {
-    const SmallShape sh = small_shape(n, nnz, sms);
-    if (!sh.kernel)
-        return 0;
-    const size_t smem = (size_t)sh.cap * 12;
-    allow_shared(sh.kernel, smem); // (one cap per kernel)
-    if (sh.cluster) {
-        CK(cudaFuncSetAttribute(sh.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        cudaLaunchAttribute at;
-        const cudaLaunchConfig_t c = small_config(sh, SMALL_CLUSTER, &at, nullptr);
-        int clusters = 0;
-        CK(cudaOccupancyMaxActiveClusters(&clusters, sh.kernel, &c));
-        return clusters >= 1 ? SMALL_CLUSTER : 0;
+    __shared__ int most[2];
+    if (threadIdx.x < 2)
+        most[threadIdx.x] = 0;
+    __syncthreads();
+    for (int which = 0; which < 2; ++which) {
+        const int nb = which ? b1 : b0;
+        for (int b = threadIdx.x; b < nb; b += blockDim.x)
+            atomicMax(&most[which], rp[(long long)n * (b + 1) / nb] - rp[(long long)n * b / nb]);
     }
-    int per_sm = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sh.kernel, sh.threads, smem));
-    const int blocks = (n + sh.vars - 1) / sh.vars;
-    return per_sm >= 1 && blocks <= sms ? std::max(blocks, 1) : 0;
+    __syncthreads();
+    if (threadIdx.x < 2)
+        out[threadIdx.x] = most[threadIdx.x];
 }
 
-void launch_bb_small(int n, long long nnz, int sms, int blocks, const BBData &D, const BBParams &P, const GridSlots &S,
-                     cudaStream_t s)
+constexpr int SMALL_CAP = 200 * 1024 / 12; // entries of Q that a block can stage
+
+// The shape for an n x n Q, blocks = 0: none.  Every block stages its rows, so
+// a shape is taken only if its fullest block fits: rows read from L2 by a
+// thread each are what all blocks then wait for (500 rows of 60 entries side
+// by side in 10000: 240 us per outer iteration that way, 113 by the general
+// kernel; 3000 in 60000: 384 against 201).  shares: 2 ints of device scratch.
+SmallPlan bb_small_plan(int n, long long nnz, const int *Q_rp, int sms, int *shares, cudaStream_t s)
 {
-    SmallShape sh = small_shape(n, nnz, sms);
+    // (every row of Q has a diagonal entry in practice)
+    const SmallShape cl = nnz - n <= SMALL_CLUSTER_NNZ ? cluster_shape(n) : SmallShape{}, gr = grid_shape(n, sms);
+    if (!cl.kernel && !gr.kernel)
+        return SmallPlan{};
+    const int grid = gr.kernel ? std::max((n + gr.vars - 1) / gr.vars, 1) : 1;
+    int h[2];
+    small_share_kernel<<<1, TPB, 0, s>>>(n, Q_rp, SMALL_CLUSTER, grid, shares);
+    CK(cudaMemcpyAsync(h, shares, sizeof(h), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    if (cl.kernel && h[0] <= SMALL_CAP) {
+        const SmallPlan p{cl.kernel, SMALL_CLUSTER, cl.threads, std::max(cl.cap, h[0]), true};
+        allow_shared(p.kernel, (size_t)SMALL_CAP * 12);
+        CK(cudaFuncSetAttribute(p.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t c = small_config(p, &at, nullptr);
+        int clusters = 0;
+        CK(cudaOccupancyMaxActiveClusters(&clusters, p.kernel, &c));
+        if (clusters >= 1)
+            return p;
+    }
+    if (gr.kernel && h[1] <= SMALL_CAP) {
+        const SmallPlan p{gr.kernel, grid, gr.threads, std::max(gr.cap, h[1]), false};
+        allow_shared(p.kernel, (size_t)SMALL_CAP * 12);
+        int per_sm = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p.kernel, p.threads, (size_t)p.cap * 12));
+        if (per_sm >= 1 && grid <= sms)
+            return p;
+    }
+    return SmallPlan{};
+}
+
+void launch_bb_small(const SmallPlan &p, const BBData &D, const BBParams &P, const GridSlots &S, cudaStream_t s)
+{
     cudaLaunchAttribute at;
-    const cudaLaunchConfig_t c = small_config(sh, blocks, &at, s);
-    void *args[] = {(void *)&D, (void *)&P, (void *)&S, &sh.cap};
-    CK(cudaLaunchKernelExC(&c, sh.kernel, args));
+    const cudaLaunchConfig_t c = small_config(p, &at, s);
+    void *args[] = {(void *)&D, (void *)&P, (void *)&S, (void *)&p.cap};
+    CK(cudaLaunchKernelExC(&c, p.kernel, args));
 }
 
 } // namespace pdhcg

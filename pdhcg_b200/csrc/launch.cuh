@@ -182,11 +182,15 @@ int bb_blocks_per_sm(int G, int S, bool fixed); // resident blocks of both kerne
 void launch_bb(int G, int S, bool fixed, int grid, const BBData &D, const BBParams &P, cudaStream_t s);
 void launch_q_apply(int G, int grid, const BBData &D, const double *v, double *qx, cudaStream_t s);
 
-// inner_small.cu: sparse Q with short rows, no cones; blocks: 0 when n does
-// not fit one block per SM
-int bb_small_blocks(int n, long long nnz, int sms);
-void launch_bb_small(int n, long long nnz, int sms, int blocks, const BBData &D, const BBParams &P, const GridSlots &S,
-                     cudaStream_t s);
+// inner_small.cu: sparse Q with short rows, no cones; blocks: 0 when Q does
+// not fit the blocks' shared memory
+struct SmallPlan {
+    const void *kernel;
+    int blocks, threads, cap; // cap: entries of Q that a block has room for
+    bool cluster;
+};
+SmallPlan bb_small_plan(int n, long long nnz, const int *Q_rp, int sms, int *shares, cudaStream_t s);
+void launch_bb_small(const SmallPlan &p, const BBData &D, const BBParams &P, const GridSlots &S, cudaStream_t s);
 
 // inner_dense.cu: dense R, diagonal Q; blocks: 0 when the shape does not fit
 int dense_tile_count(int width);

@@ -862,7 +862,8 @@ private:
     long long bb_inner_fp32_ = 0;          // inner iterations taken with the FP32 values
     // the special inner solves: sparse Q of short rows without cones
     // (inner_small.cu), dense R with a diagonal Q (inner_dense.cu)
-    int bb_small_blocks_ = 0, bb_dense_blocks_ = 0, sms_ = 0;
+    SmallPlan bb_small_{};
+    int bb_dense_blocks_ = 0;
     int bb_refresh_ = 1; // BBParams.refresh of the next dense solve
     GridSlots bb_slots_{};
     DenseR bb_dense_{};
@@ -1338,7 +1339,6 @@ void Solve::setup_bb()
 void Solve::setup_bb_special(int nsm)
 {
     cudaStream_t s = st_;
-    sms_ = nsm;
     const int k = R_.nnz > 0 ? R_.rows : 0, nc = (int)cone_start_.size();
     if (dp_.has_fixed || dp_.var_psd)
         return;
@@ -1351,7 +1351,7 @@ void Solve::setup_bb_special(int nsm)
         CK(cudaMemcpyAsync(&h, cnt, sizeof(int), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         if (h == 0)
-            bb_small_blocks_ = bb_small_blocks(n_, Q_.nnz, nsm);
+            bb_small_ = bb_small_plan(n_, Q_.nnz, Q_.rp, nsm, ar_.alloc<int>(2), s);
     } else if (r_width_ > 0 && (dp_.dkind != 2 || k <= 64)) {
         // R must not touch a cone slot, Q must be diagonal; a dense middle
         // matrix is applied by every block in every pass, so only a small one
@@ -1384,8 +1384,8 @@ void Solve::setup_bb_special(int nsm)
         bb_dense_.rx_state = ar_.alloc<double>(2 * (size_t)k);
         bb_dense_blocks_ = blocks;
     }
-    if (bb_small_blocks_ > 0 || bb_dense_blocks_ > 0) {
-        bb_slots_ = bb_small_blocks_ > 0 ? make_slots(bb_small_blocks_, 2) : make_slots(bb_dense_blocks_, k + 2);
+    if (bb_small_.blocks > 0 || bb_dense_blocks_ > 0) {
+        bb_slots_ = bb_small_.blocks > 0 ? make_slots(bb_small_.blocks, 2) : make_slots(bb_dense_blocks_, k + 2);
         bb_slots_.err = (int *)(scal_d_ + SC_FLAG); // read with every evaluation's scalars
     }
 }
@@ -1699,8 +1699,8 @@ void Solve::enqueue_step_bb(bool store_dual, bool want_fpe, double w)
     }
     BBData D = bb_data();
     BBParams BP{tau, w, prm_.reflection_coefficient, want_fpe ? 1 : 0, bb_refresh_};
-    if (bb_small_blocks_ > 0) {
-        launch_bb_small(n_, Q_.nnz, sms_, bb_small_blocks_, D, BP, bb_slots_, s);
+    if (bb_small_.blocks > 0) {
+        launch_bb_small(bb_small_, D, BP, bb_slots_, s);
     } else if (bb_dense_blocks_ > 0) {
         bb_dense_.tile = bb_fp32_ ? (const void *)Rtilef_ : (const void *)Rtile_;
         launch_bb_dense(S_, bb_fp32_, bb_dense_blocks_, D, BP, bb_dense_, bb_slots_, s);

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import scipy.sparse as sp
 
-from pdhcg_b200 import instances
+from pdhcg_b200 import instances, native
 from pdhcg_b200.capi import CsrMatrix
 from test_gpu_resident import _problem
 from test_gpu_solver import _solve_gpu, _solve_oracle
@@ -40,6 +40,51 @@ def test_sparse_q(lib, oracle, n, band):
     Q = sp.diags(diags, range(len(diags)), format="csr")
     p.Q = CsrMatrix.from_scipy(sp.csr_matrix(Q + sp.triu(Q, 1).T))
     _compare(lib, oracle, p)
+
+
+# The first rows of Q are long (half bandwidth `wide`), the others tridiagonal:
+# the fullest block's share fits its shared memory (cluster form, grid form
+# where the cluster's 16 blocks do not) or the general kernel is taken
+@pytest.mark.parametrize("n,stretch,wide", [(3000, 150, 30), (10000, 500, 30), (60000, 3000, 8), (60000, 3000, 30)])
+def test_sparse_q_with_a_dense_stretch(lib, oracle, n, stretch, wide):
+    _compare(lib, oracle, _dense_stretch(n, stretch, wide))
+
+
+def _dense_stretch(n, stretch, wide):
+    rng = np.random.default_rng(n + wide)
+    p = _problem(n, n, max(1, n // 2), False)
+    rows, cols, vals = [np.arange(n)], [np.arange(n)], [np.full(n, 2.0 * wide)]
+    for d in range(1, wide + 1):
+        at = np.arange(n - 1 if d == 1 else stretch - d)
+        v = rng.uniform(-0.9, 0.9, at.size)
+        rows += [at, at + d]
+        cols += [at + d, at]
+        vals += [v, v]
+    p.Q = CsrMatrix.from_scipy(sp.csr_matrix((np.concatenate(vals), (np.concatenate(rows), np.concatenate(cols))),
+                                             shape=(n, n)))
+    return p
+
+
+def test_dense_stretch_keeps_its_time(lib):
+    """An inner iteration on rows of 61 entries side by side takes no more than
+    1.2 times that of the same rows spread over the matrix (the same entries, an
+    even share of them in every block)."""
+    p = _dense_stretch(10000, 500, 30)
+    perm = np.random.default_rng(0).permutation(10000)
+    spread = _dense_stretch(10000, 500, 30)
+    Q = p.Q.to_scipy()[perm][:, perm]
+    Q.sort_indices()
+    spread.Q = CsrMatrix.from_scipy(sp.csr_matrix(Q))
+    prm = dict(PRM, **{"termination_criteria.iteration_limit": 300})
+
+    def per_inner(q):
+        best = np.inf
+        for _ in range(3):
+            d = native.solve(q, prm)
+            best = min(best, native.last_stats()["loop_ms"] / d["total_inner_count"])
+        return best
+
+    assert per_inner(p) <= 1.2 * per_inner(spread)
 
 
 # rows of R around the 16 warps, 4, 8 and 16 rows a warp and the limit of 256
