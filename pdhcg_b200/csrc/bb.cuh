@@ -533,8 +533,13 @@ __device__ double bb_grad_phase(const BBData &D, const double *drx, double inv_t
     return part;
 }
 
-template <int G, int S, bool SECT>
-__global__ void __launch_bounds__(TPB) bb_kernel(BBData D, BBParams P)
+// PER_SM: blocks per SM to leave registers for.  Most instantiations take 220 to
+// 255 registers unbounded, which leaves one; a large problem waits on its
+// gathers and wants two (a Q of 300000 rows of 5 entries: 674 us per outer
+// iteration with one, 497 with two), a small one is taken by one block per SM
+// without the bound's spills.  With the section projectors (SECT) always one.
+template <int G, int S, bool SECT, int PER_SM>
+__global__ void __launch_bounds__(TPB, PER_SM) bb_kernel(BBData D, BBParams P)
 {
     cgb::grid_group grid = cgb::this_grid();
     __shared__ double drx[BB_MAX_RANK];

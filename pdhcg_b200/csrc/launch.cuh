@@ -177,9 +177,10 @@ void launch_residual_psd(const ResidualData<VT> &D, const ResidualParams &P, con
                          int first, int blocks, cudaStream_t s);
 
 // inner.cu: the inner BB solve and the Q apply (G lanes per row of Q, S
-// slots per lane of a cone block)
-int bb_blocks_per_sm(int G, int S, bool fixed); // resident blocks of both kernels
-void launch_bb(int G, int S, bool fixed, int grid, const BBData &D, const BBParams &P, cudaStream_t s);
+// slots per lane of a cone block; one_per_sm: the form for a grid of one block
+// per SM)
+int bb_blocks_per_sm(int G, int S, bool fixed, bool one_per_sm); // resident blocks of both kernels
+void launch_bb(int G, int S, bool fixed, bool one_per_sm, int grid, const BBData &D, const BBParams &P, cudaStream_t s);
 void launch_q_apply(int G, int grid, const BBData &D, const double *v, double *qx, cudaStream_t s);
 
 // inner_small.cu: sparse Q with short rows, no cones; blocks: 0 when Q does

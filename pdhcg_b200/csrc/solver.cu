@@ -849,6 +849,7 @@ private:
     // inner BB solve (non-diagonal Q)
     bool bb_ = false;
     int bb_grid_ = 0, bb_limit_ = 1, GQ_ = 1;
+    bool bb_one_per_sm_ = false;
     double *bb_aty_ = nullptr, *bb_grad_ = nullptr, *bb_dir_ = nullptr, *bb_qx_ = nullptr, *qx_res_ = nullptr;
     double *bb_part_ = nullptr, *bb_rxp_ = nullptr, *bb_rx_ = nullptr, *bb_tol_ = nullptr, *bb_tscale_ = nullptr;
     double *bb_diag_h_ = nullptr, *bb_m_ = nullptr, *bb_minv_ = nullptr;
@@ -1263,10 +1264,16 @@ void Solve::setup_bb()
     int dev = 0, nsm = 0, per_sm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    per_sm = bb_blocks_per_sm(GQ_, S_, dp_.has_fixed);
+    // One block per SM where that is a thread per row lane (and cone slot): the
+    // four barriers of an inner iteration cost more with more blocks (9000
+    // variables in 260 cones, 7 entries a row: 76 us per outer iteration on 148
+    // blocks, 90 on 296; 300000 variables, 5 a row: 674 and 497).
+    const long long lanes = std::max((long long)n * GQ_, 32LL * (long long)cone_start_.size());
+    bb_one_per_sm_ = R_.nnz == 0 && lanes <= (long long)nsm * TPB;
+    per_sm = bb_blocks_per_sm(GQ_, S_, dp_.has_fixed, bb_one_per_sm_);
     if (per_sm < 1)
         throw CudaError("inner BB kernel cannot be made resident");
-    bb_grid_ = nsm * std::min(per_sm, 4);
+    bb_grid_ = nsm * (bb_one_per_sm_ ? 1 : std::min(per_sm, 4));
     int k = R_.nnz > 0 ? R_.rows : 0;
     bb_aty_ = ar_.alloc<double>(n);
     bb_grad_ = ar_.alloc<double>(n);
@@ -1312,7 +1319,9 @@ void Solve::setup_bb()
         double *part = ar_.alloc<double>((size_t)2 * bb_grid_);
         int eper = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&eper, power_eig_kernel, TPB, 0));
-        int eg = std::max(1, std::min(bb_grid_, nsm * std::max(eper, 1)));
+        // (a thread per row: no more blocks than rows fill)
+        const int eneed = std::max(nsm, grid_for(n, TPB, bb_grid_));
+        int eg = std::max(1, std::min({bb_grid_, eneed, nsm * std::max(eper, 1)}));
         double lmax = 0.0;
         for (int shifted = 0; shifted < 2; ++shifted) {
             CK(cudaMemcpyAsync(v, v0.data(), n * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -1706,7 +1715,7 @@ void Solve::enqueue_step_bb(bool store_dual, bool want_fpe, double w)
         launch_bb_dense(S_, bb_fp32_, bb_dense_blocks_, D, BP, bb_dense_, bb_slots_, s);
         bb_refresh_ = 0;
     } else {
-        launch_bb(GQ_, S_, dp_.has_fixed, bb_grid_, D, BP, s);
+        launch_bb(GQ_, S_, dp_.has_fixed, bb_one_per_sm_, bb_grid_, D, BP, s);
     }
     StepParams P{};
     P.tau = tau;

@@ -42,6 +42,13 @@ def test_sparse_q(lib, oracle, n, band):
     _compare(lib, oracle, p)
 
 
+# more than 16 entries a row: the general kernel, 32 lanes a row, on one block per
+# SM up to 148 * 256 / 32 rows and on two beyond
+@pytest.mark.parametrize("n", [1184, 1185])
+def test_general_kernel_on_one_and_two_blocks_per_sm(lib, oracle, n):
+    test_sparse_q(lib, oracle, n, 20)
+
+
 # The first rows of Q are long (half bandwidth `wide`), the others tridiagonal:
 # the fullest block's share fits its shared memory (cluster form, grid form
 # where the cluster's 16 blocks do not) or the general kernel is taken
