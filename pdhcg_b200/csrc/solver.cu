@@ -873,6 +873,7 @@ private:
     BBData bb_data() const;
     void setup_bb();
     void setup_bb_special(int nsm);
+    bool dense_pays(int k, int tiles, int blocks) const;
     void enqueue_q_apply(const double *v, double *qx);
     double *c_d_ = nullptr, *l_d_ = nullptr, *u_d_ = nullptr, *q_d_ = nullptr, *lc_d_ = nullptr, *uc_d_ = nullptr,
            *g_d_ = nullptr, *cr_d_ = nullptr, *vr_d_ = nullptr;
@@ -1343,6 +1344,47 @@ void Solve::setup_bb()
     CK(cudaGetLastError());
 }
 
+// Whether a pass of bb_dense_kernel is shorter than one of bb_kernel, by
+// estimates in microseconds from their timings over ranks 10 to 256, widths 300
+// to 100000 and tails of 0 to 64 strides or 0 to 16 cones per block.  The dense
+// kernel saves two grid barriers and a pass over R, and pays for the fold of k
+// sums over its blocks; above 128 rows its tiles go through the step one at a
+// time.  What lies past R's width (the tail) is stepped by ONE warp per block
+// beside the tiles, where bb_kernel spreads it over all warps of all SMs: R over
+// 1000 of 1000000 columns took 4745 us per outer iteration against 543, over 20000
+// with 20000 cones behind them 701 against 174.  Per block of the dense kernel:
+//   strides of 32 variables 0.65 (bb_kernel: 0.2 on as many blocks as SMs),
+//   a SOC / RSOC block of L slots 1.2 + 0.024 L (0.15 + 0.006 L), an exponential
+//   block 5.7, a power block 9.4 (0.6, and one chain of 6 or 9 in either kernel).
+// The line lies where the two forms are within 10 % of one another (rank 64, width
+// 5000: 16 strides, 5 cones of 12 slots, 2 exponential blocks per block).
+bool Solve::dense_pays(int k, int tiles, int blocks) const
+{
+    const double spread = std::min(1.0, blocks / 148.0), per_block = 1.0 / blocks;
+    const long long past = (cone_start_.empty() ? (long long)n_ : (long long)free_idx_.size()) - r_width_;
+    const double strides = std::max(past, 0LL) * per_block / 32;
+    double tail = 0.65 * strides, other = 0.2 * spread * strides, chain = 0.0;
+    for (size_t b = 0; b < cone_start_.size(); ++b) {
+        const int type = dp_.cone_type[b], len = dp_.cone_len[b];
+        if (type == CONE_EXPONENTIAL || type == CONE_POWER) {
+            tail += (type == CONE_POWER ? 9.4 : 5.7) * per_block;
+            other += 0.6 * spread * per_block;
+            chain = std::max(chain, type == CONE_POWER ? 9.0 : 6.0);
+        } else {
+            tail += (1.2 + 0.024 * len) * per_block;
+            other += (0.15 + 0.006 * len) * spread * per_block;
+        }
+    }
+    const double per = (double)tiles * per_block, bytes = 8.0 * k * r_width_;
+    double gain = 8.5 + 0.04 * k - 5.7e-4 * k * blocks;
+    if (k > 128)
+        gain -= 1.0 + 0.6 * per;
+    if (bytes > 60e6) // the second pass of bb_kernel comes from HBM
+        gain += bytes / 6.5e6;
+    // the tail's own time beside the tiles is free
+    return std::max(0.0, tail - per * (0.4 + 0.0075 * k)) - other - std::min(chain, tail) <= gain;
+}
+
 // Which problems leave the general inner kernel: see inner_small.cu and
 // inner_dense.cu for why.  Both take one block per SM.
 void Solve::setup_bb_special(int nsm)
@@ -1369,7 +1411,7 @@ void Solve::setup_bb_special(int nsm)
                 return;
         const int tiles = dense_tile_count(r_width_);
         const int blocks = dense_blocks(k, tiles, S_, nsm);
-        if (blocks == 0)
+        if (blocks == 0 || !dense_pays(k, tiles, blocks))
             return;
         if (Q_.nnz > 0) {
             double *qd = ar_.alloc<double>(n_);

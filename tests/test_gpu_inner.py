@@ -6,7 +6,7 @@ import pytest
 import scipy.sparse as sp
 
 from pdhcg_b200 import instances, native
-from pdhcg_b200.capi import CsrMatrix
+from pdhcg_b200.capi import CONE_EXPONENTIAL, CONE_STANDARD_SOC, Cone, CsrMatrix
 from test_gpu_resident import _problem
 from test_gpu_solver import _solve_gpu, _solve_oracle
 
@@ -105,6 +105,48 @@ def test_dense_low_rank(lib, oracle, k, n, with_q):
     p = _problem(n, n, max(1, n // 4), with_q)
     p.R_dense = rng.standard_normal((k, n)) / np.sqrt(n)
     _compare(lib, oracle, p)
+
+
+def _with_tail(k, width, n, cones=()):
+    """R over the leading `width` of n variables and of `cones` (type, count,
+    slots) behind them."""
+    rng = np.random.default_rng(k + width + n)
+    p = _problem(k, n + sum(c * w for _, c, w in cones), max(1, n // 8), True, per_row=3)
+    p.R_dense = np.zeros((k, p.n))
+    p.R_dense[:, :width] = rng.standard_normal((k, width)) / np.sqrt(width)
+    at = n
+    for kind, count, slots in cones:
+        for _ in range(count):
+            p.cones.append(Cone(kind, at, 1 if kind == CONE_EXPONENTIAL else slots - 2))
+            at += slots
+    p.var_lb[n:], p.var_ub[n:] = -np.inf, np.inf
+    return p
+
+
+# variables and cones past R's width: few (the dense kernel), many (the general
+# one), and to either side of the line between them
+@pytest.mark.parametrize("k,width,n,cones", [
+    (64, 1000, 1000, ()), (64, 1000, 1001, ()), (64, 1000, 16000, ()), (64, 1000, 21000, ()), (64, 1000, 100000, ()),
+    (64, 20000, 20000, ((CONE_STANDARD_SOC, 500, 12),)), (64, 20000, 20000, ((CONE_STANDARD_SOC, 2000, 12),)),
+    (20, 3000, 5000, ((CONE_STANDARD_SOC, 30, 40), (CONE_EXPONENTIAL, 60, 3))),
+    (20, 3000, 5000, ((CONE_STANDARD_SOC, 30, 40), (CONE_EXPONENTIAL, 900, 3)))])
+def test_dense_low_rank_with_a_tail(lib, oracle, k, width, n, cones):
+    _compare(lib, oracle, _with_tail(k, width, n, cones))
+
+
+def test_a_long_tail_keeps_its_time(lib):
+    """R over 1000 of 200000 columns: an inner iteration at rank 64 takes no more
+    than 1.3 times one at rank 300 (the general kernel at any tail)."""
+    prm = dict(PRM, **{"termination_criteria.iteration_limit": 200})
+
+    def per_inner(q):
+        best = np.inf
+        for _ in range(3):
+            d = native.solve(q, prm)
+            best = min(best, native.last_stats()["loop_ms"] / d["total_inner_count"])
+        return best
+
+    assert per_inner(_with_tail(64, 1000, 200000)) <= 1.3 * per_inner(_with_tail(300, 1000, 200000))
 
 
 def test_portfolio_with_columns_of_middle_length(lib, oracle):
