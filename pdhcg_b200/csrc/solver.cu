@@ -193,6 +193,26 @@ struct Arena {
         ptrs.push_back(p);
         return (T *)p;
     }
+    // the same for memory that can be done without: NULL when the device has none left
+    template <typename T>
+    T *try_alloc(size_t count)
+    {
+        void *p = nullptr;
+        keep_pool_memory();
+        const cudaError_t e = cudaMallocAsync(&p, std::max<size_t>(count, 1) * sizeof(T), s);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        CK(e);
+        ptrs.push_back(p);
+        return (T *)p;
+    }
+    void release_last()
+    {
+        CK(cudaFreeAsync(ptrs.back(), s));
+        ptrs.pop_back();
+    }
     template <typename T>
     T *upload(const T *h, size_t count, cudaStream_t s)
     {
@@ -1425,10 +1445,22 @@ void Solve::setup_bb_special(int nsm)
                 return;
             bb_dense_.qd = qd;
         }
+        // the tiles (FP32 ones behind them), where they leave room for what the
+        // solve still allocates: the general kernel needs no copy of R
         const size_t vals = (size_t)tiles * k * 32;
-        Rtile_ = ar_.alloc<double>(vals);
-        if (opt_.precision == PDHCG_B200_MIXED)
-            Rtilef_ = ar_.alloc<float>(vals);
+        const bool mixed = opt_.precision == PDHCG_B200_MIXED;
+        const size_t rest = 30 * ((size_t)n_ + m_) + (mixed ? ((size_t)R_.nnz + 2 * (size_t)A_.nnz) / 2 : 0);
+        Rtile_ = ar_.try_alloc<double>(mixed ? vals + vals / 2 : vals);
+        if (!Rtile_)
+            return;
+        if (!ar_.try_alloc<double>(rest)) {
+            ar_.release_last();
+            Rtile_ = nullptr;
+            return;
+        }
+        ar_.release_last();
+        if (mixed)
+            Rtilef_ = (float *)(Rtile_ + vals);
         dense_tiles(k, r_width_, R_.rp, R_.v, tiles, Rtile_, Rtilef_, s);
         bb_dense_.tiles = tiles;
         bb_dense_.width = r_width_;
