@@ -107,7 +107,11 @@ int pdhcg_b200_rescaling(const qp_problem_t *prob, const pdhg_parameters_t *para
  * (which declares it extern and sets it from a SIGINT handler, reference
  * python_bindings/_core_bindings.cpp:41-47) links unchanged.  A non-zero
  * value ends the running solve at its next evaluation with
- * TERMINATION_REASON_USER_INTERRUPT. */
+ * TERMINATION_REASON_USER_INTERRUPT.  Where the main loop runs in persistent
+ * launches (LP and diagonal QP without cones that fit on chip) that is the
+ * next evaluation of the host: a launch in flight, 2000 iterations and those
+ * up to its next evaluation at most (6 to 40 ms at the default frequency),
+ * ends first, and its own outcome gives way to the flag. */
 extern volatile sig_atomic_t g_pdhcg_cancel_request;
 void pdhcg_b200_request_cancel(int on);
 

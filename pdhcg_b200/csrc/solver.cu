@@ -2473,8 +2473,17 @@ void Solve::loop()
             !(is_major_ && k_ < 3 * freq)) {
             run_resident(std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count());
             cum_time_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-            if (reason_ != TERMINATION_REASON_UNSPECIFIED || k_ >= tc.iteration_limit)
+            if (reason_ != TERMINATION_REASON_UNSPECIFIED || k_ >= tc.iteration_limit) {
+                // a cancel that came during the launch comes before its outcome
+                if (pdhcg_b200_cancel_requested()) {
+                    if (reason_ == TERMINATION_REASON_UNSPECIFIED) {
+                        enqueue_residual(false);
+                        read_residual();
+                    }
+                    reason_ = TERMINATION_REASON_USER_INTERRUPT;
+                }
                 break;
+            }
         }
         if (is_major_ || k_ == 0 || (k_ % print_frequency(k_)) == 0) {
             bool restart_check = is_major_ || k_ == 0;
