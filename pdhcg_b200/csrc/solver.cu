@@ -823,6 +823,7 @@ private:
     ResidentPlan res_plan_{};
     ResidentState *res_state_ = nullptr, *h_res_ = nullptr;
     GridSlots res_slots_{};
+    double res_pace_ = 0.0; // seconds per iteration of the last launch
     void setup_resident();
     void run_resident(double elapsed);
     void resolve_fpe(const double *r);
@@ -2335,8 +2336,10 @@ void Solve::run_resident(double elapsed)
     P.l2 = prm_.optimality_norm == NORM_TYPE_L2;
     P.freq = prm_.termination_evaluation_frequency;
     P.iteration_limit = tc.iteration_limit;
-    // hand back in time for the host to see the clock and the cancel flag
-    P.budget = RESIDENT_BUDGET;
+    // hand back in time for the host to see the clock and the cancel flag: no
+    // more iterations than the time limit leaves at the last launch's pace
+    const double left = (prm_.termination_criteria.time_sec_limit - elapsed) / (res_pace_ > 0.0 ? res_pace_ : 2e-5);
+    P.budget = (int)std::fmin(RESIDENT_BUDGET, std::fmax(1.0, left));
     P.eps_opt = tc.eps_optimal_relative;
     P.eps_feas = tc.eps_feasible_relative;
     P.step = step_;
@@ -2367,6 +2370,7 @@ void Solve::run_resident(double elapsed)
     h.fpe0 = fpe0_;
     h.fpe_last = fpe_last_;
     std::memcpy(h_scal_, &h, sizeof(h));
+    const auto launched = std::chrono::steady_clock::now();
     CK(cudaMemcpyAsync(res_state_, h_scal_, sizeof(h), cudaMemcpyHostToDevice, s));
     launch_resident(res_plan_, D, P, res_slots_, s);
     stats_.kernel_launches++;
@@ -2376,6 +2380,8 @@ void Solve::run_resident(double elapsed)
     if (h.wait_failed)
         check_slots(res_slots_, "persistent iteration");
     const int steps = h.k - k_;
+    if (steps > 0)
+        res_pace_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - launched).count() / steps;
     stats_.step_kernel_launches += steps;
     stats_.restarts += h.restarts;
     stats_.evaluations += h.evaluations;

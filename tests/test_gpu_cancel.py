@@ -43,3 +43,17 @@ def test_cancel_during_the_last_launch(lib, flag):
             assert np.isfinite(d["x"]).all() and d["total_count"] <= 2300
             break
     assert seen[-1] == "USER_INTERRUPT", seen
+
+
+def test_time_limit_within_a_launch(lib):
+    """A limit that ends half way through a launch of 2000 iterations (20 ms): the
+    solve stops at an evaluation soon after it."""
+    p, prm = _problem(6, 150000, 75000, False), _params(20000)
+    native.solve(p, dict(prm, **{"termination_criteria.iteration_limit": 400}))
+    limit = 0.012
+    over = []
+    for _ in range(5):  # the host may stall
+        d = native.solve(p, dict(prm, **{"termination_criteria.time_sec_limit": limit}))
+        assert d["status"] == "TIME_LIMIT"
+        over.append(d["cumulative_time_sec"] - limit)
+    assert min(over) <= 0.005, over
