@@ -323,6 +323,11 @@ void build_long_rows(DevCsr &M, Arena &ar, cudaStream_t s)
     CK(cudaStreamSynchronize(s));
     std::vector<int> rows, first{0}, index(M.rows, -1);
     std::vector<int2> seg;
+    for (int r = 0; r < M.rows; ++r)
+        if (rp[r + 1] - rp[r] > LONG_ROW) {
+            index[r] = (int)rows.size();
+            rows.push_back(r);
+        }
     M.long_nnz = 0;
     // The segment length that fills whole rounds of the pass's resident warps
     // (a warp takes a segment; 5450 segments of 4096 entries over 3552 warps ran
@@ -331,9 +336,8 @@ void build_long_rows(DevCsr &M, Arena &ar, cudaStream_t s)
     const int warps = WARPS * resident_blocks((const void *)long_partials_kernel<double, double>);
     auto count_segs = [&](int len) {
         long long c = 0;
-        for (int r = 0; r < M.rows; ++r)
-            if (rp[r + 1] - rp[r] > LONG_ROW)
-                c += (rp[r + 1] - rp[r] + len - 1) / len;
+        for (int r : rows)
+            c += (rp[r + 1] - rp[r] + len - 1) / len;
         return c;
     };
     int seg_len = LONG_SEG;
@@ -354,13 +358,9 @@ void build_long_rows(DevCsr &M, Arena &ar, cudaStream_t s)
             seg_len = hi;
         }
     }
-    for (int r = 0; r < M.rows; ++r) {
-        if (rp[r + 1] - rp[r] <= LONG_ROW)
-            continue;
+    for (int r : rows) {
         M.long_nnz += rp[r + 1] - rp[r];
         M.max_row = std::max(M.max_row, rp[r + 1] - rp[r]);
-        index[r] = (int)rows.size();
-        rows.push_back(r);
         for (int b = rp[r]; b < rp[r + 1]; b += seg_len)
             seg.push_back(make_int2(b, std::min(rp[r + 1], b + seg_len)));
         first.push_back((int)seg.size());
