@@ -1099,12 +1099,14 @@ __host__ __device__ constexpr long long psd_work_doubles(long long order)
 // Rotation for a pair: the tangent of the smaller angle that annihilates a_pq
 // is t = a2 / (h + sign(h) sqrt(h^2 + a2^2)), h = a_qq - a_pp, a2 = 2 a_pq.
 // The rounds are chains of these angles, and FP64 square roots and divisions
-// are a few hundred cycles each, so t is formed in FP32 on the pair scaled by
-// its larger magnitude (a power of two), and only the cosine, which makes
-// (c, t c) a rotation to FP64 rounding, in FP64: 1 / sqrt(1 + t^2) by two
-// Newton steps from its FP32 value (errors 1e-7, 1e-14, below rounding).  An
-// angle 1e-7 off leaves 1e-7 of a_pq behind, which is kept, not set to zero;
-// the next sweep takes it.
+// are a few hundred cycles each, so t starts from its FP32 value on the pair
+// scaled by its larger magnitude (a power of two) and takes one Newton step in
+// FP64 on t^2 a2 / 2 + t h - a2 / 2 (error 3e-7, then 1e-13; the slope at the root
+// is that square root, and its reciprocal may be FP32, as it multiplies a
+// correction of 3e-7), and the cosine,
+// which makes (c, t c) a rotation to FP64 rounding, is 1 / sqrt(1 + t^2) by two
+// Newton steps from its FP32 value (errors 1e-7, 1e-14, below rounding).  What
+// the angle leaves of a_pq is kept, not set to zero.
 __device__ __forceinline__ void jacobi_angle(double app, double aqq, double apq, double &c, double &sn)
 {
     c = 1.0;
@@ -1117,9 +1119,12 @@ __device__ __forceinline__ void jacobi_angle(double app, double aqq, double apq,
     if (e < 2 || e > 2045)
         return;
     const double scale = __longlong_as_double((long long)(2046 - e) << 52);
-    const float hf = (float)(h * scale), af = (float)(a2 * scale);
-    const float tf = af / (hf + copysignf(sqrtf(hf * hf + af * af), hf));
-    const double t = (double)tf, r = fma(t, t, 1.0);
+    const double hs = h * scale, as = a2 * scale;
+    const float hf = (float)hs, af = (float)as;
+    const float q = hf * hf + af * af, rq = copysignf(rsqrtf(q), hf); // q in [1, 8)
+    const double t0 = (double)__fdividef(af, hf + q * rq);
+    const double t = fma(-(double)rq, fma(fma(0.5 * as, t0, hs), t0, -0.5 * as), t0);
+    const double r = fma(t, t, 1.0);
     double y = (double)rsqrtf((float)r);
     y = y * fma(-0.5 * r * y, y, 1.5);
     y = y * fma(-0.5 * r * y, y, 1.5);
