@@ -107,6 +107,21 @@ def test_dense_low_rank(lib, oracle, k, n, with_q):
     _compare(lib, oracle, p)
 
 
+# a dense R with a dense middle matrix: up to 64 rows the dense kernel (every block
+# applies D in every pass), beyond it the general one; a diagonal one at any rank
+@pytest.mark.parametrize("k,dense", [(3, True), (64, True), (65, True), (65, False)])
+def test_dense_low_rank_with_a_middle_matrix(lib, oracle, k, dense):
+    rng = np.random.default_rng(k)
+    p = _problem(k, 900, 200, True)
+    p.R_dense = rng.standard_normal((k, 900)) / 30.0
+    if dense:
+        B = rng.standard_normal((k, k)) / np.sqrt(k)
+        p.D = CsrMatrix.from_dense(B @ B.T + 0.1 * np.eye(k))
+    else:
+        p.D = CsrMatrix.from_scipy(sp.diags(rng.uniform(0.5, 2.0, k), format="csr"))
+    _compare(lib, oracle, p)
+
+
 def _with_tail(k, width, n, cones=()):
     """R over the leading `width` of n variables and of `cones` (type, count,
     slots) behind them."""
