@@ -65,7 +65,11 @@ int launch_primal_cones(const StepData<T> &D, const StepParams &P, const ConeSpl
             kernel<<<grid_for(sp.n_psd, 1), threads, dyn, s>>>(D, P, sp.psd_d, sp.n_psd);
         };
         if (D.psd_max > 0 && dyn <= PSD_STEP_SMEM) {
-            if (D.psd_max <= 32) {
+            // 128 threads to order 20, 256 beyond: a round of order 20 is 255
+            // updates and rotations for two barriers (us a step of 38 blocks, 128
+            // and 256 threads: order 8 59 and 61, 16 130 and 131, 24 257 and 229,
+            // 32 548 and 391)
+            if (D.psd_max <= 20) {
                 if (hasq)
                     go(psd_step_kernel<T, true, 128>, 128);
                 else
@@ -98,10 +102,13 @@ int launch_primal_cones(const StepData<T> &D, const StepParams &P, const ConeSpl
     return launches;
 }
 
-// Free variables and cone blocks in one launch where their blocks are resident
-// at once with room to spare (two per SM; more would queue behind one
-// another, and the kernels of one kind are leaner).  PSD and section blocks
-// have launches of their own.  False: not for this problem, nothing launched.
+// Free variables and cone blocks in one launch up to six thread blocks per SM,
+// where the three launches would run one after the other for the length of
+// their longest chains (us an iteration, one launch and three: 108 blocks 42
+// and 59, 216 44 and 57, 324 45 and 61, 432 48 and 63, 863 56 and 68); beyond,
+// where every kind fills the chip by itself, the kernels of one kind are
+// leaner.  PSD and section blocks have launches of their own.  False: not for
+// this problem, nothing launched.
 template <typename T>
 bool launch_primal_mixed(const StepData<T> &D, const StepParams &P, const ConeSplit &sp, int S, bool hasq,
                          cudaStream_t s)
@@ -109,10 +116,10 @@ bool launch_primal_mixed(const StepData<T> &D, const StepParams &P, const ConeSp
     const int kinds = (D.n_free_tiles > 0) + (sp.n_wide > 0) + (sp.n_three > 0);
     if (kinds < 2 || !D.free_tiles && D.n_free > 0)
         return false;
-    // a warp of its own block for every 3-slot block up to 64: their chains are the longest
+    // (a warp per cone block, eight to a thread block, of either kind)
     const int fb = D.n_free > 0 ? grid_for(D.n_free_tiles, WARPS) : 0, wb = sp.n_wide > 0 ? grid_for(sp.n_wide, WARPS) : 0,
               tb = sp.n_three > 0 ? grid_for(sp.n_three, WARPS) : 0;
-    if (fb + wb + tb > 2 * 148)
+    if (fb + wb + tb > 6 * 148)
         return false;
     dispatch_s(sp.n_wide > 0 ? S : 1, [&](auto SC) {
         if (hasq)

@@ -36,6 +36,25 @@ def test_iterates_follow_the_oracle(lib, oracle, make):
         np.testing.assert_allclose(a[key], b[key], rtol=0, atol=1e-7 * max(1.0, np.abs(b[key]).max()))
 
 
+# 402 and 952 thread blocks of free variables and cones (one launch up to 888), PSD
+# blocks on 128 threads (to order 20) and on 256
+@pytest.mark.parametrize("make", [
+    lambda: instances.conic_lp(seed=38, nfree=400, nsoc=1600, soc_len=5, nrsoc=1, nexp=800, npow=800),
+    lambda: instances.conic_lp(seed=39, nfree=400, nsoc=3600, soc_len=5, nrsoc=1, nexp=2000, npow=2000),
+    lambda: instances.psd_lp(seed=40, orders=(20, 20)), lambda: instances.psd_lp(seed=41, orders=(21, 20, 2)),
+    lambda: instances.psd_lp(seed=42, orders=(40,))],
+    ids=["one launch", "a launch per kind", "128 threads", "256 threads", "order 40"])
+def test_iterates_at_the_launch_rules(lib, oracle, make):
+    """As above over 40 iterations: among 2000 random exponential blocks one is so
+    ill-conditioned that its two projections are 3e-9 apart, which the primal weight
+    of a restart after 40 multiplies by a thousand."""
+    p = make()
+    prm = dict(PRM, **{"termination_criteria.iteration_limit": 40})
+    a, b = _solve_gpu(lib, p, prm), _solve_oracle(oracle, lib, p, prm)
+    for key in ("x", "y"):
+        np.testing.assert_allclose(a[key], b[key], rtol=0, atol=1e-7 * max(1.0, np.abs(b[key]).max()))
+
+
 # the largest PSD block that a thread block takes in the residual (83) and in the
 # step (112), and the first that a warp takes on device scratch instead
 @pytest.mark.parametrize("orders", [(83,), (84,), (112,), (113, 4)])
