@@ -72,14 +72,16 @@ void pdhcg_b200_device_problem_free(pdhcg_b200_device_problem_t *handle);
 typedef struct {
     double setup_ms;             /* upload, transpose, rescaling, power method (CUDA events) */
     double loop_ms;              /* main loop on the device, first to last iteration (CUDA events) */
-    double step_kernel_ms;       /* summed duration of the fused primal/dual step kernels */
-    long long step_kernel_launches;
+    double step_kernel_ms;       /* summed duration of the fused primal/dual step kernels: with time_steps,
+                                    which also selects the loop of one launch per step kernel */
+    long long step_kernel_launches; /* steps taken (those of a persistent launch count one by one) */
     long long kernel_launches;   /* all kernels launched by the solve */
     int iterations;
     int fp32_iterations;
     int restarts;
     int evaluations;
-    double step_bytes;           /* algorithmic HBM bytes of one primal + dual step */
+    double step_bytes;           /* algorithmic bytes of one primal + dual step (a persistent launch
+                                    reads the matrices from HBM once, then from shared memory) */
     double spmv_bytes;           /* algorithmic bytes of the two SpMVs inside one step */
     double host_copy_ms;         /* host-side copy / classification of the problem */
     double upload_ms;            /* allocation and host->device copies */
