@@ -40,7 +40,7 @@ WORKLOAD = "soc_qp: n=1e6 (20000 SOC blocks x 50), m=5e5 eq rows, 10 nnz/row, di
 # kernels), from an ncu capture of the two step kernels on it
 STEP_TRAFFIC = {"f64": 202.5e6, "f32": 121.4e6}
 # random 4- / 8-byte gathers per second of one B200 through L1TEX, measured
-# by pdhcg_b200/csrc/probes/gather_ceiling.cu
+# by a stand-alone probe (profiles/spmv_gather_ceiling_b200.md)
 GATHER_RATE = 1.95e11
 
 # Single-instance workloads: the generator, whether the mixed form is timed
