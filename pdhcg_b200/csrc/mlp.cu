@@ -404,16 +404,16 @@ __device__ __forceinline__ void split3(float v0, float v1, unsigned &hi, unsigne
     split2(v0 - hf.x, v1 - hf.y, mid, lo);
 }
 
-// elements (i, k) and (i, k + 1) of a matrix stored [i][k] (KFAST) or [k][i]
-template <bool KFAST, typename T>
+// elements (i, k) and (i, k + 1) of a matrix stored [i][k]
+template <typename T>
 __device__ __forceinline__ float2 pair_at(const T *p, int ld, int i, int k, int I, int K)
 {
     float2 v = make_float2(0.0f, 0.0f);
     if (i < I) {
         if (k < K)
-            v.x = ::ld(KFAST ? p + (size_t)i * ld + k : p + (size_t)k * ld + i);
+            v.x = ::ld(p + (size_t)i * ld + k);
         if (k + 1 < K)
-            v.y = ::ld(KFAST ? p + (size_t)i * ld + k + 1 : p + (size_t)(k + 1) * ld + i);
+            v.y = ::ld(p + (size_t)i * ld + k + 1);
     }
     return v;
 }
@@ -424,7 +424,7 @@ __device__ __forceinline__ unsigned bf16_pair_at(const bf16 *p, int ld, int i, i
 {
     if (VEC)
         return i < I && k < K ? *reinterpret_cast<const unsigned *>(p + (size_t)i * ld + k) : 0u;
-    const float2 v = pair_at<true>(p, ld, i, k, I, K);
+    const float2 v = pair_at(p, ld, i, k, I, K);
     const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
     return *reinterpret_cast<const unsigned *>(&h);
 }
@@ -454,7 +454,7 @@ __device__ __forceinline__ void small_gemm_tile(const SmallGemm &G, int tile, fl
                     if (i < G.M && k < G.K)
                         v = *reinterpret_cast<const float2 *>(G.A + (size_t)i * G.K + k);
                 } else {
-                    v = pair_at<true>(G.A, G.K, i, k, G.M, G.K);
+                    v = pair_at(G.A, G.K, i, k, G.M, G.K);
                 }
                 split3(v.x, v.y, a[0][mt][q], a[1][mt][q], a[2][mt][q]);
             }
