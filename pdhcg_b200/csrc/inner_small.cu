@@ -34,12 +34,15 @@ constexpr int SMALL_CLUSTER_NNZ = 64 * 1024;
 
 namespace cgc = cooperative_groups;
 
-// Gathers of one row in flight: an inner iteration waits for its longest row's
-// rounds.  Two rows a thread, Q = B'B with rows to about 20 entries, 1e4
-// variables, us per inner iteration at 8 / 12 / 16: 7.6 / 5.2 / 5.8; tridiagonal,
-// one row a thread, 2000 variables: 4.5 / 4.5 / 5.0.
+// Gathers of one row in flight: ROW_WIDTH, and as many again where one of the
+// thread's rows is longer.  An inner iteration waits for its longest row's rounds,
+// but every gather that a round has room for costs its issue slots in the short
+// rows too.  Us per inner iteration at a fixed 8 / 12 / 16, and with 8 (one row a
+// thread) or 6 (two) doubled where needed: Q = B'B with rows to about 20 entries,
+// 1000 variables 6.5 / 4.1 / - and 3.9, 10000 7.6 / 5.2 / 5.8 and 5.0;
+// tridiagonal, 2000 4.5 / 4.5 / 5.0 and 4.5, 16000 5.3 / 5.5 / 6.1 and 5.1.
 template <int V>
-constexpr int ROW_WIDTH = V == 1 ? 8 : 12;
+constexpr int ROW_WIDTH = V == 1 ? 8 : 6;
 
 // Barriers and sums of the two forms.  fold: both values summed over the
 // launch's blocks, in block order, the same in every thread; also a barrier.
@@ -164,7 +167,7 @@ __global__ void __launch_bounds__(NT) bb_small_kernel(BBData D, BBParams P, Grid
         e[v] = w;
     }
     // s = (Q w) of the thread's rows (the diagonal's operands are `own`), the rows
-    // side by side with ROW_W gathers of each in flight, entries in order
+    // side by side with up to 2 ROW_W gathers of each in flight, entries in order
     int longest = 0;
 #pragma unroll
     for (int v = 0; v < V; ++v)
@@ -175,19 +178,33 @@ __global__ void __launch_bounds__(NT) bb_small_kernel(BBData D, BBParams P, Grid
         for (int v = 0; v < V; ++v)
             s[v] = dq[v] * own[v];
 #pragma unroll 1
-        for (int k = 0; k < longest; k += ROW_W) {
-            double a[V][ROW_W];
+        for (int k = 0; k < longest; k += 2 * ROW_W) {
+            const bool more = longest > k + ROW_W;
+            double a[V][2 * ROW_W];
 #pragma unroll
             for (int v = 0; v < V; ++v)
 #pragma unroll
                 for (int u = 0; u < ROW_W; ++u)
                     a[v][u] = b[v] + k + u < e[v] ? __ldcg(w + sc[b[v] + k + u]) : 0.0;
+            if (more)
+#pragma unroll
+                for (int v = 0; v < V; ++v)
+#pragma unroll
+                    for (int u = ROW_W; u < 2 * ROW_W; ++u)
+                        a[v][u] = b[v] + k + u < e[v] ? __ldcg(w + sc[b[v] + k + u]) : 0.0;
 #pragma unroll
             for (int v = 0; v < V; ++v)
 #pragma unroll
                 for (int u = 0; u < ROW_W; ++u)
                     if (b[v] + k + u < e[v])
                         s[v] += sv[b[v] + k + u] * a[v][u];
+            if (more)
+#pragma unroll
+                for (int v = 0; v < V; ++v)
+#pragma unroll
+                    for (int u = ROW_W; u < 2 * ROW_W; ++u)
+                        if (b[v] + k + u < e[v])
+                            s[v] += sv[b[v] + k + u] * a[v][u];
         }
     };
     // the projected step from `from` along M^-1 g; the partial of dir' M dir
