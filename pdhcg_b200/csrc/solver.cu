@@ -177,6 +177,23 @@ void keep_pool_memory()
     done[dev] = true;
 }
 
+// Bytes that the default pool can still hand out: what it keeps unused and what
+// the device has left.  (A trial allocation instead grows the pool: 0.2 s of a
+// first solve.)
+size_t device_room()
+{
+    int dev = 0;
+    size_t free_b = 0, total = 0;
+    cudaMemPool_t pool;
+    unsigned long long reserved = 0, used = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaMemGetInfo(&free_b, &total));
+    CK(cudaDeviceGetDefaultMemPool(&pool, dev));
+    CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+    CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+    return free_b + (size_t)(reserved > used ? reserved - used : 0);
+}
+
 // Device allocations owned by one solve or one device problem: stream-ordered
 // from the default pool on the owner's stream s, returned to the pool on the
 // legacy stream when the owner (which has synchronised its streams by then)
@@ -207,11 +224,6 @@ struct Arena {
         CK(e);
         ptrs.push_back(p);
         return (T *)p;
-    }
-    void release_last()
-    {
-        CK(cudaFreeAsync(ptrs.back(), s));
-        ptrs.pop_back();
     }
     template <typename T>
     T *upload(const T *h, size_t count, cudaStream_t s)
@@ -1451,15 +1463,12 @@ void Solve::setup_bb_special(int nsm)
         const size_t vals = (size_t)tiles * k * 32;
         const bool mixed = opt_.precision == PDHCG_B200_MIXED;
         const size_t rest = 30 * ((size_t)n_ + m_) + (mixed ? ((size_t)R_.nnz + 2 * (size_t)A_.nnz) / 2 : 0);
-        Rtile_ = ar_.try_alloc<double>(mixed ? vals + vals / 2 : vals);
+        const size_t copy = mixed ? vals + vals / 2 : vals;
+        if (device_room() < (copy + rest) * sizeof(double))
+            return;
+        Rtile_ = ar_.try_alloc<double>(copy);
         if (!Rtile_)
             return;
-        if (!ar_.try_alloc<double>(rest)) {
-            ar_.release_last();
-            Rtile_ = nullptr;
-            return;
-        }
-        ar_.release_last();
         if (mixed)
             Rtilef_ = (float *)(Rtile_ + vals);
         dense_tiles(k, r_width_, R_.rp, R_.v, tiles, Rtile_, Rtilef_, s);
